@@ -53,8 +53,8 @@ const char* yan_b200_return_code_string(int code);
  * describes: yan/jit_kernels/gemm.py:9-31 (`Gemm<...>::run(out, rhs_scales, nullptr, m, descs..., stream,
  * num_sms, smem_size)`) and the kernel yan/include/gemm/fp8_gemm.cuh:32-197.
  * block_n: 0 = choose; 32, 64, 96, 128, 160, 192, 224 or 256 = tile width of the general kernel; 1 = the weight-streaming kernel
- * for M <= 64 (split-K over a pair of CTAs), 2 = the weight-streaming kernel for M <= 32 that keeps all of K in one
- * CTA (YAN_B200_BAD_ARGUMENT when the problem does not fit the kernel asked for).
+ * for M <= 64 (split-K over a pair of CTAs), 2 = the weight-streaming kernel of 0 for small batches, asked for by
+ * name for M <= 32, N % 32 = 0, K % 512 = 0, K <= 16384 (YAN_B200_BAD_ARGUMENT when the problem does not fit the kernel asked for).
  * num_sms: CTAs of the persistent grid (<= device SMs).
  */
 void yan_b200_gemm_fp8_fp8_bf16_nt(const void* lhs, const void* lhs_scales, const void* rhs, const void* rhs_scales,
@@ -250,8 +250,9 @@ void yan_b200_allreduce_bf16_gather_staged(const void* stage, void* const* data,
  * previous kernel of the stream is still running; activations, scales of the activations and the output are
  * only touched after the previous kernel has completed.  Enable it only when `rhs` / `rhs_scales` are not
  * written by the kernel that precedes the GEMM in its stream (true for inference weights).  Default: off.
- * While enabled, the quantizer inside yan_b200_fp8_linear_bf16(_static) is launched the same way: its launch overlaps
- * the tail of the previous kernel of the stream, and it waits for that kernel before it reads or writes anything.
+ * The quantizer is always launched that way (its launch overlaps the tail of the previous kernel of the stream, and it
+ * waits for that kernel before it reads or writes anything); while this is enabled it also lets the GEMM behind it in
+ * yan_b200_fp8_linear_bf16(_static) start loading weights before that wait instead of after it.
  * No reference counterpart (the reference launches every kernel with plain <<<>>>, e.g.
  * yan/include/gemm/cute_gemm.cuh:373).
  */

@@ -1,0 +1,87 @@
+"""The weight-streaming kernel of the small batches (M <= 64) at the edges of its tiles, k-parts, slots and clusters, against
+the CPU oracle and the general kernel, and its ordering behind kernels that write its weights."""
+import pytest
+import torch
+
+from oracle import ref
+
+pytestmark = pytest.mark.gpu
+
+
+def _device(lhs, rhs):
+    return (lhs[0].cuda(), lhs[1].t().contiguous().cuda().t()), (rhs[0].cuda(), rhs[1].cuda())
+
+
+def _operands(m, n, k, seed):
+    """Both operands (a ragged N is cut out of whole 128-row scale blocks) and the oracle's result."""
+    a, b = ref.make_inputs(m, (n + 127) // 128 * 128, k, seed=seed, outliers=True)
+    lhs, (q, s) = ref.per_token_cast_to_fp8(a), ref.per_block_cast_to_fp8(b)
+    return lhs, (q[:n].contiguous(), s), ref.ref_gemm(lhs, (q, s))[:, :n]
+
+
+# M: both sides of every padding.  N: one CTA, widths no CTA divides (n % 32 == 16), clusters of 2 and 4, more row groups
+# than SMs.  K: one k-block (all k-parts but one empty), short last parts, more steps than slots, the longest declared.
+@pytest.mark.parametrize("m,n,k", [(1, 16, 128), (16, 48, 384), (17, 16, 128), (32, 80, 640), (33, 16, 128), (64, 144, 896),
+                                   (8, 528, 13440), (16, 1040, 7168), (5, 2064, 7168), (16, 4784, 1152), (31, 1008, 7168),
+                                   (32, 9488, 384), (40, 528, 7168), (64, 1040, 4224), (64, 9472, 256), (63, 272, 18432),
+                                   (2, 256, 18432), (24, 272, 18432)])
+def test_edges_match_oracle_and_general_kernel(cuda_lib, m, n, k):
+    import yan_b200
+    lhs, rhs, d_ref = _operands(m, n, k, seed=m + n + k)
+    lhs_d, rhs_d = _device(lhs, rhs)
+    full = torch.full((m, n + 32), 7.0, dtype=torch.bfloat16, device="cuda")
+    yan_b200.gemm_fp8_fp8_bf16_nt(lhs_d, rhs_d, full[:, 16:16 + n])
+    general = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    yan_b200.gemm_fp8_fp8_bf16_nt(lhs_d, rhs_d, general, block_n=32)
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    out = full[:, 16:16 + n].cpu()
+    bound = ref.bf16_ulp_at(float(d_ref.float().abs().max()))
+    assert ref.rel_frobenius(out, d_ref) <= 1e-3 and ref.max_abs_err(out, d_ref) <= bound
+    # both kernels sum in fp32, in another order: bf16 results differ by one rounding of few values
+    assert ref.rel_frobenius(out, general.cpu()) <= 1e-3
+    assert bool((full[:, :16] == 7.0).all()) and bool((full[:, 16 + n:] == 7.0).all()), "stored outside the slice"
+
+
+@pytest.mark.parametrize("m", [16, 64])
+def test_fp8_linear_sees_weights_written_just_before(cuda_lib, m):
+    """The weight quantizer, then fp8_linear on its result, many times over the same buffers: every launch may start
+    early, none may read the weights of the round before."""
+    import yan_b200
+    n, k = 2048, 2048
+    gen = torch.Generator().manual_seed(3)
+    x = torch.randn(m, k, generator=gen).to(torch.bfloat16).cuda()
+    q, s = torch.empty(n, k, dtype=torch.float8_e4m3fn, device="cuda"), torch.empty(n // 128, k // 128, device="cuda")
+    ws = [(torch.randn(n, k, generator=gen) * 0.02 * (i + 1)).to(torch.bfloat16).cuda() for i in range(4)]
+    pairs = [yan_b200.per_block_cast_to_fp8(w) for w in ws]
+    want = [yan_b200.fp8_linear(x, p).clone() for p in pairs]
+    torch.cuda.synchronize()
+    got = []
+    for i in list(range(4)) * 3:
+        q.view(torch.uint8).copy_(pairs[i][0].view(torch.uint8))
+        s.copy_(pairs[i][1])
+        got.append(yan_b200.fp8_linear(x, (q, s)).clone())
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    assert all(torch.equal(g, want[i % 4]) for i, g in enumerate(got))
+
+
+def test_output_that_only_the_streaming_kernels_take(cuda_lib):
+    """An output row stride that is no multiple of 8: still accepted where a weight-streaming kernel serves the shape, still
+    refused where the general kernel does."""
+    import ctypes
+    from yan_b200 import _lib
+    lhs, rhs, d_ref = _operands(16, 256, 512, seed=5)
+    lhs_d, rhs_d = _device(lhs, rhs)
+    out = torch.zeros(16, 257, dtype=torch.bfloat16, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def call(n, k):
+        return _lib.call_rc("yan_b200_gemm_fp8_fp8_bf16_nt", lhs_d[0].data_ptr(), lhs_d[1].data_ptr(), rhs_d[0].data_ptr(),
+                            rhs_d[1].data_ptr(), out.data_ptr(), 16, n, k, 257, stream, sms, 0)
+
+    assert call(256, 512) == 0
+    torch.cuda.synchronize()
+    assert ref.rel_frobenius(out[:, :256].cpu(), d_ref) <= 1e-3
+    assert call(256, 384) == 1 and call(240, 512) == 1

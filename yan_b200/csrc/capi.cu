@@ -128,26 +128,29 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
     a.clock_probe = g_clock_probe;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // M <= 64: the weight-streaming kernels.  block_n 1 asks for the pair-cluster kernel, 2 for the stacked-K kernel
-    // (M <= 32), 0 picks the stacked one where it is the faster (M <= 16, two CTAs per SM), else the pair kernel.
+    // (M <= 32), 0 picks the stacked one where it is the fastest.
     if (type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16 && (want_auto || block_n == 1 || block_n == 2)) {
-        int dev = 0, max_smem = 0;
+        int dev = 0, max_smem = 0, sm_count = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        const bool programmatic = g_programmatic_launch != 0 || after_own_quantizer;
-        if (block_n == 2) {
-            if (!yan::stacked_k_supported(a.m, a.n, a.k, max_smem) && !yan::stacked_k_ring_supported(a.m, a.n, a.k, max_smem))
-                return yan::kBadArgument;
-            return yan::launch_fp8_gemm_stacked_k(a, s, programmatic);
+        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+        const yan::StackedOrder order = g_programmatic_launch != 0 ? yan::kConstantWeights
+                                        : after_own_quantizer     ? yan::kAfterOwnQuantizer
+                                                                  : yan::kAfterAnyKernel;
+        const bool small_m_ok = yan::small_m_supported(a.m, a.n, a.k, max_smem);
+        const bool stacked_ok = yan::stacked_k_supported(a.m, a.n, a.k);
+        if (block_n == 2) return stacked_ok ? yan::launch_fp8_gemm_stacked_k(a, s, order) : yan::kBadArgument;
+        // The general kernel stores 16 bytes at a time and checks num_sms; the weight-streaming kernels do neither.  A shape
+        // that one of them serves whatever the output is keeps that; the others are held to the general kernel's terms.
+        const bool general_ok = yan::is_aligned(a.out, 16) && a.ldd % 8 == 0 && a.num_sms <= sm_count;
+        const bool any_output = small_m_ok || (stacked_ok && (a.m <= 16 || a.n / 32 <= static_cast<uint32_t>(sm_count)));
+        if (want_auto && (general_ok || any_output) &&
+            yan::stacked_k_preferred(a.m, a.n, a.k, static_cast<uint32_t>(sm_count), static_cast<uint32_t>(max_smem)))
+            return yan::launch_fp8_gemm_stacked_k(a, s, order);
+        if (block_n == 1 || (want_auto && !general_ok && small_m_ok)) {
+            if (!small_m_ok) return yan::kBadArgument;
+            return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || after_own_quantizer);
         }
-        if (want_auto) {
-            int max_smem_sm = 0, sm_count = 0;
-            cudaDeviceGetAttribute(&max_smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-            cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-            if (yan::stacked_k_preferred(a.m, a.n, a.k, max_smem, max_smem_sm, sm_count))
-                return yan::launch_fp8_gemm_stacked_k(a, s, programmatic);
-        }
-        if (yan::small_m_supported(a.m, a.n, a.k, max_smem)) return yan::launch_fp8_gemm_small_m(a, s, programmatic);
-        if (block_n == 1) return yan::kBadArgument;
     }
     switch (block_n) {
         case 32: return yan::launch_gemm_bn32(type, out_kind, a, s);

@@ -59,17 +59,18 @@ template <uint32_t kRows>
 __global__ void __launch_bounds__(256) per_token_cast_to_fp8_kernel(const __nv_bfloat16* __restrict__ x,
                                                                     uint8_t* __restrict__ q,
                                                                     float* __restrict__ scales, uint32_t m, uint32_t k,
-                                                                    uint32_t x_ld, uint32_t sa_ld) {
+                                                                    uint32_t x_ld, uint32_t sa_ld,
+                                                                    bool weights_are_constant) {
     constexpr uint32_t kGroups = 4;
     constexpr uint32_t kItems = kRows * kGroups / 16;  // per half-warp
     __shared__ float s_scales[kGroups][kRows];
-    // A GEMM launched behind this kernel with programmatic stream serialization may start its weight loads now;
-    // it waits for this grid to complete before it touches the quantized activations.  No effect otherwise.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // When this kernel itself was launched with programmatic stream serialization its CTAs may be resident before the
-    // kernel that produces x has finished: wait for it (and for the previous readers of q / scales) here.  No effect
-    // for an ordinary launch.
+    // This kernel is launched with programmatic stream serialization: its CTAs may be resident before the kernel in front
+    // of it has finished, and wait for it (the producer of x, the previous readers of q / scales) here.  A GEMM launched
+    // the same way behind this kernel starts loading its weights when every CTA here has let it: after the wait, so that
+    // whatever the earlier kernels wrote to them is there; before it only if the caller has promised that nothing did.
+    if (weights_are_constant) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (!weights_are_constant) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const uint32_t hw = threadIdx.x / 16, l = threadIdx.x % 16;
     const uint32_t row0 = blockIdx.y * kRows, kb0 = blockIdx.x * kGroups;
@@ -139,10 +140,11 @@ __global__ void __launch_bounds__(256) per_block_cast_to_fp8_kernel(const __nv_b
 }
 
 // Host launchers.  Return a ReturnCode.
-// programmatic: launch with programmatic stream serialization, so that the launch latency overlaps the tail of the
-// kernel before it in the stream (the kernel waits for that kernel before it reads or writes anything).
+// Always launched with programmatic stream serialization, so that the launch latency overlaps the tail of the kernel
+// before it in the stream (the kernel waits for that kernel before it reads or writes anything).
+// weights_are_constant: no kernel in front of this one writes the weights of the GEMM behind it (see the kernel).
 inline int launch_per_token_cast_to_fp8(const void* x, void* q, float* scales, uint32_t m, uint32_t k, uint32_t x_ld,
-                                        uint32_t sa_ld, cudaStream_t stream, bool programmatic = false) {
+                                        uint32_t sa_ld, cudaStream_t stream, bool weights_are_constant = false) {
     if (x == nullptr || q == nullptr || scales == nullptr || m == 0 || k == 0 || k % 128 != 0) return kBadArgument;
     if (x_ld < k || x_ld % 8 != 0 || sa_ld < m) return kBadArgument;
     if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(q) % 8 != 0) return kBadArgument;
@@ -156,15 +158,17 @@ inline int launch_per_token_cast_to_fp8(const void* x, void* q, float* scales, u
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = programmatic ? 1 : 0;
+    cfg.numAttrs = 1;
     cudaError_t e;
     if (m >= 1024) {
         cfg.gridDim = dim3(ceil_div(num_kb, 4u), ceil_div(m, 32u));
         if (cfg.gridDim.y > 65535) return kBadArgument;
-        e = cudaLaunchKernelEx(&cfg, per_token_cast_to_fp8_kernel<32>, xp, qp, scales, m, k, x_ld, sa_ld);
+        e = cudaLaunchKernelEx(&cfg, per_token_cast_to_fp8_kernel<32>, xp, qp, scales, m, k, x_ld, sa_ld,
+                               weights_are_constant);
     } else {
         cfg.gridDim = dim3(ceil_div(num_kb, 4u), ceil_div(m, 8u));
-        e = cudaLaunchKernelEx(&cfg, per_token_cast_to_fp8_kernel<8>, xp, qp, scales, m, k, x_ld, sa_ld);
+        e = cudaLaunchKernelEx(&cfg, per_token_cast_to_fp8_kernel<8>, xp, qp, scales, m, k, x_ld, sa_ld,
+                               weights_are_constant);
     }
     if (e != cudaSuccess) {
         cudaGetLastError();
