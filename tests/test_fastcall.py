@@ -1,0 +1,79 @@
+"""The native front of the operators: it takes exactly the ordinary calls, gives them the same result as the Python path,
+and leaves everything else (copies, errors) to that path."""
+import pytest
+import torch
+
+from oracle import ref
+
+
+def test_leaves_unusual_arguments_to_python():
+    from yan_b200 import _lib
+    f = _lib.fast()
+    t = torch.zeros(128, 128)
+    assert f.gemm_bf16(t, t, t, t, t, 0, 148, True) == -1          # not on a CUDA device
+    assert f.gemm_f32(1, None, "x", t, t, 0, 148, False) == -1     # not tensors
+    assert f.gemm_bf16(t, t) == -1 and f.linear() == -1 and f.per_token_cast(t) == -1
+    assert f.linear(t, t, t, t, None, {}, 0, 148) == -1
+    with pytest.raises(TypeError):
+        f.bind(1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 7, 130])
+@pytest.mark.parametrize("k", [128, 512])
+def test_same_results_as_the_python_path(cuda_lib, m, k, monkeypatch):
+    """Every scale layout, an output slice and both output types, with the native front and (where it did take the call)
+    without it."""
+    import yan_b200
+    from yan_b200 import _lib
+    a, b = ref.make_inputs(m, 256, k, seed=m + k)
+    x, rhs = a.cuda(), tuple(t.cuda() for t in ref.per_block_cast_to_fp8(b))
+    yan_b200.get_num_sms()
+
+    class NotTaken:
+        def __getattr__(self, name):
+            return lambda *args: -1
+
+    def run():
+        q, s = yan_b200.per_token_cast_to_fp8(x)
+        s_wide = torch.zeros(k // 128, m + 5, device="cuda").t()[:m]
+        q2 = torch.empty_like(q)
+        yan_b200.per_token_cast_to_fp8(x, out=(q2, s_wide))
+        outs = [q2.view(torch.uint8), s_wide.clone()]
+        for scales in (s, s.contiguous(), s_wide):
+            full = torch.full((m, 512), 7.0, dtype=torch.bfloat16, device="cuda")
+            yan_b200.gemm_fp8_fp8_bf16_nt((q, scales), rhs, full[:, 128:384])
+            f32 = torch.empty(m, 256, device="cuda")
+            yan_b200.gemm_fp8_fp8_f32_nt((q, scales), rhs, f32)
+            outs += [full, f32]
+        out = torch.empty(m, 256, dtype=torch.bfloat16, device="cuda")
+        ws = torch.empty(yan_b200.fp8_linear_workspace_bytes(m, k), dtype=torch.uint8, device="cuda")
+        outs += [yan_b200.fp8_linear(x, rhs), yan_b200.fp8_linear(x, rhs, out).clone(), yan_b200.fp8_linear(x, rhs, out, ws).clone()]
+        torch.cuda.synchronize()
+        return outs
+
+    native = run()
+    monkeypatch.setattr(_lib, "_fast", NotTaken())
+    assert all(torch.equal(n, p) for n, p in zip(native, run()))
+
+
+@pytest.mark.gpu
+def test_errors_are_raised_as_before(cuda_lib):
+    import yan_b200
+    a, b = ref.make_inputs(16, 256, 512, seed=1)
+    lhs = yan_b200.per_token_cast_to_fp8(a.cuda())
+    rhs = tuple(t.cuda() for t in ref.per_block_cast_to_fp8(b))
+    out = torch.empty(16, 256, dtype=torch.bfloat16, device="cuda")
+    yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out)
+    for bad in (out.float(), out[:8], out.t(), out.cpu(), torch.empty(16, 257, dtype=torch.bfloat16, device="cuda")[:, :256]):
+        with pytest.raises(AssertionError):
+            yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, bad)
+    with pytest.raises(AssertionError):
+        yan_b200.gemm_fp8_fp8_f32_nt(lhs, rhs, out)
+    with pytest.raises(AssertionError):
+        yan_b200.per_token_cast_to_fp8(a.cuda(), out=(lhs[0], lhs[1].contiguous()))
+    with pytest.raises(AssertionError):
+        yan_b200.fp8_linear(a.cuda().float(), rhs, out)
+    from yan_b200._lib import YanB200Error
+    with pytest.raises(YanB200Error):
+        yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out, block_n=48)

@@ -59,7 +59,10 @@ SIGNATURES = {
 # YAN_B200_STATIC_SCRATCH_MAX_ELEMENTS of include/yan_b200.h
 STATIC_SCRATCH_MAX_ELEMENTS = 8 << 20
 
+FASTCALL_PATH = os.path.join(_PKG_DIR, "lib", "_fastcall.so")
+
 _lib: Optional[ctypes.CDLL] = None
+_fast = None
 
 
 class YanB200Error(RuntimeError):
@@ -84,12 +87,35 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def fast():
+    """The native front of the hot operators (csrc/fastcall.cpp), bound to the loaded library."""
+    global _fast
+    if _fast is None:
+        if not os.path.exists(FASTCALL_PATH):
+            raise ImportError(f"{FASTCALL_PATH} is missing: build it with `python -m yan_b200.build`")
+        import importlib.util
+        import torch  # noqa: F401  (its libraries have to be loaded first)
+        spec = importlib.util.spec_from_file_location("yan_b200.lib._fastcall", FASTCALL_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.bind(*(ctypes.cast(getattr(lib(), name), _P).value for name in
+                      ("yan_b200_gemm_fp8_fp8_bf16_nt", "yan_b200_gemm_fp8_fp8_f32_nt", "yan_b200_fp8_linear_bf16",
+                       "yan_b200_fp8_linear_workspace_bytes", "yan_b200_per_token_cast_to_fp8")))
+        _fast = module
+    return _fast
+
+
+def check(name: str, rc: int) -> None:
+    """Raises on a non-zero return code."""
+    if rc != 0:
+        raise YanB200Error(name, rc, lib().yan_b200_return_code_string(rc).decode())
+
+
 def call(name: str, *args) -> None:
     """Calls a `void f(..., int* return_code)` entry point and raises on a non-zero code."""
     rc = ctypes.c_int(0)
     getattr(lib(), name)(*args, ctypes.byref(rc))
-    if rc.value != 0:
-        raise YanB200Error(name, rc.value, lib().yan_b200_return_code_string(rc.value).decode())
+    check(name, rc.value)
 
 
 def call_rc(name: str, *args) -> int:

@@ -13,6 +13,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from typing import List
 
@@ -22,6 +23,8 @@ INCLUDE_DIR = os.path.join(PKG_DIR, "include")
 LIB_DIR = os.path.join(PKG_DIR, "lib")
 OBJ_DIR = os.path.join(PKG_DIR, "lib", "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libyan_b200.so")
+FASTCALL_SRC = os.path.join(CSRC_DIR, "fastcall.cpp")
+FASTCALL_PATH = os.path.join(LIB_DIR, "_fastcall.so")
 
 BLOCK_NS = (32, 64, 96, 128, 160, 192, 224, 256)
 
@@ -72,8 +75,38 @@ def _run(cmd: List[str], verbose: bool) -> None:
         raise RuntimeError(f"nvcc failed ({r.returncode}): {' '.join(cmd)}\n{r.stdout}")
 
 
+def build_fastcall(force: bool = False, verbose: bool = False) -> str:
+    """Compiles the native front of the Python operators (a CPython extension against the installed torch)."""
+    import torch
+    torch_dir = os.path.dirname(torch.__file__)
+    if not force and os.path.exists(FASTCALL_PATH) and os.path.getmtime(FASTCALL_PATH) > max(
+            os.path.getmtime(FASTCALL_SRC), os.path.getmtime(os.path.join(torch_dir, "version.py"))):
+        return FASTCALL_PATH
+    cxx = os.environ.get("CXX") or shutil.which("g++")
+    if not cxx:
+        raise RuntimeError("g++ not found: set CXX")
+    os.makedirs(LIB_DIR, exist_ok=True)
+    cuda_home = os.path.dirname(os.path.dirname(find_nvcc()))
+    tmp = FASTCALL_PATH + f".tmp.{os.getpid()}"
+    _run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+          f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{torch_dir}/include",
+          f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda_home}/include",
+          FASTCALL_SRC, "-o", tmp, f"-L{torch_dir}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"], verbose)
+    os.replace(tmp, FASTCALL_PATH)
+    return FASTCALL_PATH
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compiles the library if it is missing or older than any source.  Returns its path."""
+    """Compiles the library and the native front of its operators if they are missing or older than any source.  Returns
+    the library's path."""
+    with ThreadPoolExecutor(max_workers=1) as pool:
+        front = pool.submit(build_fastcall, force, verbose)
+        path = _build_cuda_library(force, verbose)
+        front.result()
+    return path
+
+
+def _build_cuda_library(force: bool, verbose: bool) -> str:
     if not force and not is_stale():
         return LIB_PATH
     nvcc = find_nvcc()

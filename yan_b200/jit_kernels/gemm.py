@@ -18,6 +18,7 @@ import torch
 
 from .. import _lib
 from .quant import per_token_cast_to_fp8
+from . import utils as _utils
 from .utils import ceil_div, get_col_major_tensor, get_m_alignment_for_contiguous_layout, get_num_sms
 
 # C++ code templates (JIT path)
@@ -86,6 +87,9 @@ def _stream_ptr() -> ctypes.c_void_p:
     return _lib.current_stream_ptr()
 
 
+NOT_TAKEN = -1  # the native front leaves this call to the Python path (see csrc/fastcall.cpp)
+
+
 def _check_operands(lhs, lhs_scales, rhs, rhs_scales, out, out_dtype) -> Tuple[int, int, int]:
     m, k = lhs.shape
     n, k_ = rhs.shape
@@ -116,6 +120,10 @@ def gemm_fp8_fp8_bf16_nt(lhs: Tuple[torch.Tensor, torch.Tensor], rhs: Tuple[torc
     """
     lhs_q, lhs_scales = lhs
     rhs_q, rhs_scales = rhs
+    if _utils._num_sms is not None:
+        rc = _lib.fast().gemm_bf16(lhs_q, lhs_scales, rhs_q, rhs_scales, out, block_n, _utils._num_sms, _tail_cut[0])
+        if rc != NOT_TAKEN:
+            return _lib.check("yan_b200_gemm_fp8_fp8_bf16_nt", rc)
     m, n, k = _check_operands(lhs_q, lhs_scales, rhs_q, rhs_scales, out, torch.bfloat16)
     lhs_scales = get_col_major_tensor(lhs_scales)
     if m == 1 or lhs_scales.stride(1) != m:
@@ -184,6 +192,10 @@ def gemm_fp8_fp8_f32_nt(lhs, rhs, out: torch.Tensor, block_n: int = 0) -> None:
     """Same GEMM with an fp32 output (partial sums of the K-split path keep full precision)."""
     lhs_q, lhs_scales = lhs
     rhs_q, rhs_scales = rhs
+    if _utils._num_sms is not None:
+        rc = _lib.fast().gemm_f32(lhs_q, lhs_scales, rhs_q, rhs_scales, out, block_n, _utils._num_sms, False)
+        if rc != NOT_TAKEN:
+            return _lib.check("yan_b200_gemm_fp8_fp8_f32_nt", rc)
     m, n, k = _check_operands(lhs_q, lhs_scales, rhs_q, rhs_scales, out, torch.float32)
     lhs_scales = get_col_major_tensor(lhs_scales)
     if m == 1 or lhs_scales.stride(1) != m:
@@ -278,6 +290,11 @@ def fp8_linear(a: torch.Tensor, rhs: Tuple[torch.Tensor, torch.Tensor], out: Opt
     `workspace` (uint8, >= fp8_linear_workspace_bytes(M, K)) holds the quantized activations between the
     two kernels; when omitted a per-(device, size) buffer is allocated once and reused."""
     rhs_q, rhs_scales = rhs
+    if out is not None and _utils._num_sms is not None:
+        rc = _lib.fast().linear(a, rhs_q, rhs_scales, out, workspace, _workspaces, block_n, _utils._num_sms)
+        if rc != NOT_TAKEN:
+            _lib.check("yan_b200_fp8_linear_bf16", rc)
+            return out
     m, k = a.shape
     n = rhs_q.shape[0]
     assert a.is_cuda and a.dtype == torch.bfloat16 and a.is_contiguous() and k % 128 == 0

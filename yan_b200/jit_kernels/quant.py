@@ -26,6 +26,11 @@ def per_token_cast_to_fp8(x: torch.Tensor, out: Optional[Tuple[torch.Tensor, tor
     The scale tensor is column-major (stride (1, M)): M-contiguous per k-block, so the GEMM takes
     it without a transpose.  Rows of `x` may be strided (x.stride(0) >= K, multiple of 8).
     """
+    if out is not None:
+        rc = _lib.fast().per_token_cast(x, *out)
+        if rc != -1:  # -1: not an ordinary call, left to the checks below
+            _lib.check("yan_b200_per_token_cast_to_fp8", rc)
+            return out
     assert x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2
     m, k = x.shape
     assert m > 0 and k > 0 and k % 128 == 0, "K must be a positive multiple of 128"
