@@ -126,7 +126,12 @@ __device__ __forceinline__ void store_row(out_t* dst, const float (&acc)[kCols],
 // row, so the per-token-group quantizer runs in registers.  The values are rounded to bf16 first and then quantized
 // with the quantizer's own three fp32 operations (amax_c = max(amax, 1e-4); inv = 448 / amax_c; q = e4m3_rne(x * inv);
 // scale = amax_c / 448), so that the result is bit-identical to the bf16 GEMM followed by per_token_cast_to_fp8.
-__device__ __forceinline__ void store_row_e4m3(uint8_t* dst, float* scale_dst, float (&acc)[128]) {
+// The codes leave through the warp's shared-memory box, 64 bytes per row and pass, so that a store instruction covers
+// eight 64-byte row pieces; a thread that stores its own row touches 32 lines with every 16 bytes (M=8192 N=7168 K=2048
+// 155 -> 140 us, M=4096 N=7168 K=4096 139 -> 128 us).
+__device__ __forceinline__ void store_tile_e4m3(uint8_t* out, uint32_t ld, float* out_scales, uint32_t scales_ld, uint32_t row0,
+                                                uint32_t row_limit, uint32_t n_first, uint32_t n_limit, uint32_t box,
+                                                uint32_t lane_idx, float (&acc)[128]) {
     float amax = 0.0f;
 #pragma unroll
     for (uint32_t j = 0; j < 128; ++j) {
@@ -135,21 +140,36 @@ __device__ __forceinline__ void store_row_e4m3(uint8_t* dst, float* scale_dst, f
     }
     const float amax_c = fmaxf(amax, 1e-4f);
     const float inv = __fdiv_rn(448.0f, amax_c);
+    if (row0 + lane_idx < row_limit && n_first < n_limit)
+        out_scales[static_cast<size_t>(n_first / 128u) * scales_ld + row0 + lane_idx] = __fdiv_rn(amax_c, 448.0f);
+    const uint32_t row_addr = box + lane_idx * 64u, my_chunk = lane_idx % 4u;
 #pragma unroll
-    for (uint32_t j = 0; j < 8; ++j) {
-        uint32_t w[4];
+    for (uint32_t pass = 0; pass < 2; ++pass) {
+        __syncwarp();  // the read-back of the previous pass is over
+#pragma unroll
+        for (uint32_t j = 0; j < 4; ++j) {
+            uint32_t w[4];
+#pragma unroll
+            for (uint32_t i = 0; i < 4; ++i) {
+                const float* a = acc + pass * 64 + j * 16 + i * 4;
+                const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a[0], inv), __fmul_rn(a[1], inv)),
+                                                             __NV_SATFINITE, __NV_E4M3);
+                const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a[2], inv), __fmul_rn(a[3], inv)),
+                                                             __NV_SATFINITE, __NV_E4M3);
+                w[i] = lo | (hi << 16);
+            }
+            ptx::st_shared_v4(row_addr + ((j ^ ((lane_idx >> 1) & 3u)) << 4), make_uint4(w[0], w[1], w[2], w[3]));
+        }
+        __syncwarp();
+        const uint32_t n_chunk = n_first + pass * 64u + my_chunk * 16u;
 #pragma unroll
         for (uint32_t i = 0; i < 4; ++i) {
-            const float* a = acc + j * 16 + i * 4;
-            const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a[0], inv), __fmul_rn(a[1], inv)),
-                                                         __NV_SATFINITE, __NV_E4M3);
-            const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a[2], inv), __fmul_rn(a[3], inv)),
-                                                         __NV_SATFINITE, __NV_E4M3);
-            w[i] = lo | (hi << 16);
+            const uint32_t r = i * 8u + lane_idx / 4u;
+            const uint4 v = ptx::ld_shared_v4(box + r * 64u + ((my_chunk ^ ((r >> 1) & 3u)) << 4));
+            if (row0 + r < row_limit && n_chunk < n_limit)
+                *reinterpret_cast<uint4*>(out + static_cast<size_t>(row0 + r) * ld + n_chunk) = v;
         }
-        *reinterpret_cast<uint4*>(dst + j * 16) = make_uint4(w[0], w[1], w[2], w[3]);
     }
-    *scale_dst = __fdiv_rn(amax_c, 448.0f);
 }
 
 }  // namespace detail
@@ -172,7 +192,7 @@ struct GemmSmemLayout {
     // Output staging: every promotion warp owns one 32-row x 64-byte box (2 KB).  A lane writes 64 bytes of its own
     // output row into the box, the warp reads the box back eight rows at a time and stores 64 contiguous bytes per
     // row piece, so that one store instruction covers 8 x 64 bytes instead of 32 x 16 bytes of 32 different lines.
-    // kWideBoxes (the scatter instance, whose pieces cross NVLink): 32 rows x 128 bytes per box, so that a store
+    // kWideBoxes (fp32 output; the scatter instance, whose pieces cross NVLink): 32 rows x 128 bytes per box, so that a store
     // instruction covers 4 x 128 bytes -- whole 128-byte lines on the link instead of half lines.
     static constexpr uint32_t kStoreRowBytes = kWideBoxes ? 128 : 64;
     static constexpr uint32_t kStoreBoxBytes = 32 * kStoreRowBytes;
@@ -201,9 +221,10 @@ struct GemmSmemLayout {
 //                          warpgroup has read it.  0: one full-width stream, one barrier pair per buffer.
 //   YAN_PROMO_EARLY_PROBE  1: the next k-block's TMEM-full barrier is probed (without blocking) right after this
 //                          k-block's last load, so that the answer arrives under the last FMAs.
-//   YAN_WIDE_STORE_BOXES   1: every instance stages its output in 32 x 128-byte boxes (the scatter instance always does);
-//                          for a local output it measured within +-1 % on the large shapes and 3 % slower on
-//                          M=8192 N=3584 K=8192, so the default keeps the 64-byte rows and the 16 KB of shared memory.
+//   YAN_WIDE_STORE_BOXES   1: every instance stages its output in 32 x 128-byte boxes.  The scatter instance and fp32
+//                          output always do (half the passes: M=4096 N=8192 K=3584 145.5 -> 142.4 us, M=2000 N=4096
+//                          K=1024 18.4 -> 16.4); for a local bf16 output it measured within +-1 % on the large shapes
+//                          and 3 % slower on M=8192 N=3584 K=8192, so that keeps the 64-byte rows.
 // Measured and dropped: handing the TMEM read port back and forth between the two warps of a sub-partition through
 // mbarriers (an arrive-to-wait hand-over costs ~100 cycles: 778 and 1163 cycles per k-block for 64- and 32-column turns
 // against 343 without), and four promotion warpgroups (874 cycles per k-block against 733: the per-k-block bookkeeping
@@ -223,6 +244,12 @@ struct GemmSmemLayout {
 #ifndef YAN_WIDE_STORE_BOXES
 #define YAN_WIDE_STORE_BOXES 0
 #endif
+
+// The layout with 128-byte box rows where an instance asks for them and they fit, else the one with 64-byte rows.
+template <uint32_t BLOCK_N, uint32_t kNumStages, bool kWantWide>
+using GemmOutputLayout =
+    GemmSmemLayout<BLOCK_N, kNumStages,
+                   (kWantWide || YAN_WIDE_STORE_BOXES != 0) && GemmSmemLayout<BLOCK_N, kNumStages, true>::kStoreBytes != 0>;
 
 // -DYAN_PHASE_STAMPS: CTA 0 also accumulates, per role, the cycles it spends waiting and working and writes them
 // behind the four clock values of GemmParams::clock_probe (the per-SM clock64 stamps of the reference's
@@ -255,7 +282,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     fp8_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tensor_map_a,
                     const __grid_constant__ CUtensorMap tensor_map_b) {
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 1000)
-    using L = GemmSmemLayout<BLOCK_N, kNumStages, (kScatter || YAN_WIDE_STORE_BOXES != 0) && GemmSmemLayout<BLOCK_N, kNumStages, true>::kStoreBytes != 0>;
+    using L = GemmOutputLayout<BLOCK_N, kNumStages, kScatter || (sizeof(out_t) == 4 && !kTail)>;
     using Sched = Scheduler<kGemmType, kBlockM, BLOCK_N>;
     constexpr uint32_t kNumTmemBufs = L::kNumTmemBufs;
     constexpr uint32_t kNumMathWGs = get_num_math_warpgroups(BLOCK_N);
@@ -588,10 +615,9 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                             }
                         }
 #pragma unroll
-                        for (uint32_t j = 0; j < kChunk; ++j) {
-                            const float sc = group_scale((c * kChunk + j) / 16);
-                            acc[c * kChunk + j] = fmaf(sc, __uint_as_float(t[j]), acc[c * kChunk + j]);
-                        }
+                        for (uint32_t j = 0; j < kChunk; j += 2)
+                            ptx::fma_f32x2(acc[c * kChunk + j], acc[c * kChunk + j + 1], t[j], t[j + 1],
+                                           group_scale((c * kChunk + j) / 16));
                         YAN_STAMP(l2);
                         YAN_STAMP_ADD(in_fmas, l1, l2);
                     }
@@ -602,8 +628,8 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                         release_buffer();
                         const float sc = group_scale((kNumChunks * kChunk) / 16);
 #pragma unroll
-                        for (uint32_t j = 0; j < 16; ++j)
-                            acc[kNumChunks * kChunk + j] = fmaf(sc, __uint_as_float(t[j]), acc[kNumChunks * kChunk + j]);
+                        for (uint32_t j = 0; j < 16; j += 2)
+                            ptx::fma_f32x2(acc[kNumChunks * kChunk + j], acc[kNumChunks * kChunk + j + 1], t[j], t[j + 1], sc);
                     }
                     if (++buf == kNumTmemBufs) {
                         buf = 0;
@@ -612,15 +638,17 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                 }
             }
             YAN_STAMP(s0);
+            // the e4m3 output needs one 128-column group per thread (BLOCK_N = 256, two warpgroups): the launcher refuses every
+            // other shape of CTA
+            if constexpr (sizeof(out_t) == 1 && kColsPerWG == 128) {
+                if (alive)
+                    detail::store_tile_e4m3(reinterpret_cast<uint8_t*>(p.out), p.ldd, p.out_scales, p.out_scales_ld, row - lane_idx,
+                                            sched.get_row_limit(), n_first, p.shape_n,
+                                            ptx::smem_u32(smem + L::kOffStore + (warp_idx - 4) * L::kStoreBoxBytes), lane_idx, acc);
+            }
             if (alive && row_ok) {
-                if constexpr (sizeof(out_t) == 1 && kColsPerWG != 128) {
-                    // the e4m3 output needs one 128-column group per thread (BLOCK_N = 256, two warpgroups): the launcher
-                    // refuses every other shape of CTA
-                } else if constexpr (sizeof(out_t) == 1) {
-                    if (n_first < p.shape_n)
-                        detail::store_row_e4m3(
-                            reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(row) * p.ldd + n_first,
-                            p.out_scales + static_cast<size_t>(n_first / 128u) * p.out_scales_ld + row, acc);
+                if constexpr (sizeof(out_t) == 1) {
+                    // stored above
                 } else if constexpr (!kStagedStore) {
                     out_t* dst = reinterpret_cast<out_t*>(p.out) + static_cast<size_t>(row) * p.ldd + n_first;
                     detail::store_row<out_t, kColsPerWG>(dst, acc, n_first, p.shape_n);
@@ -809,7 +837,7 @@ inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintp
 
 template <uint32_t BLOCK_N, uint32_t kNumStages, GemmType kGemmType, typename out_t>
 struct GemmLauncher {
-    using L = GemmSmemLayout<BLOCK_N, kNumStages, YAN_WIDE_STORE_BOXES != 0 && GemmSmemLayout<BLOCK_N, kNumStages, true>::kStoreBytes != 0>;
+    using L = GemmOutputLayout<BLOCK_N, kNumStages, sizeof(out_t) == 4>;
     static constexpr uint32_t kSmemSize = L::kSmemSize;
 
     static int launch(const GemmArgs& a, cudaStream_t stream) {
