@@ -56,6 +56,8 @@ const char* yan_b200_return_code_string(int code);
  * for M <= 64 (split-K over a pair of CTAs), 2 = the weight-streaming kernel of 0 for small batches, asked for by
  * name for M <= 32, N % 32 = 0, K % 512 = 0, K <= 16384 (YAN_B200_BAD_ARGUMENT when the problem does not fit the kernel asked for).
  * num_sms: CTAs of the persistent grid (<= device SMs).
+ * With block_n = 0 the K of a tile may be shared by the CTAs of a cluster (M <= 64, or few tiles and long K; also fp32 output):
+ * deterministic, but the last bit can differ from a call with an explicit tile width.
  */
 void yan_b200_gemm_fp8_fp8_bf16_nt(const void* lhs, const void* lhs_scales, const void* rhs, const void* rhs_scales,
                                    void* out, int m, int n, int k, int ldd, void* stream, int num_sms, int block_n,

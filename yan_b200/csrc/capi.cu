@@ -91,7 +91,8 @@ inline void set_rc(int* rc, int v) {
 // k-block has a large fixed part, so a narrower tile is far from proportionally cheaper, and the widths without
 // shared-memory room for the staged epilogue (224, 192, 160, 96) or with a second B scale and a 16-column tail chunk
 // pay for that.  Large problems therefore get 256; narrower tiles win when they fill the machine better.
-int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail) {
+// `cost`, when given, receives the winner's cost.
+int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* cost_out = nullptr) {
     static const struct { int bn; double tile_cost; } candidates[8] = {
         {256, 1.000}, {224, 1.08}, {192, 0.84}, {160, 0.82}, {128, 0.67}, {96, 0.72}, {64, 0.57}, {32, 0.50}};
     int best = 256;
@@ -110,6 +111,26 @@ int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail) {
             best = c.bn;
         }
     }
+    if (cost_out != nullptr) *cost_out = best_cost;
+    return best;
+}
+
+// CTAs per tile when K is cut over clusters (64-wide tiles), or 0 to leave tiles whole.  Times in us, fitted to graph
+// timings on B200 over weights from HBM: a launch of whole tiles takes about 3.4 + 0.41 * waves * tile cost per k-block
+// (M=209 N=480 K=12928: 24.5, M=128 N=2048 K=7168: 15.8, M=256 N=1024 K=4096: 10.0, M=130 N=256 K=512: 4.2), a clustered one
+// about 5.9 + 0.235 per k-block of a slice (12.0, 10.0, 7.9 and 6.0 with four slices).  Clusters of four stop fitting the
+// GPU at once between 132 and 136 CTAs (M=128 K=7168: N=2112 10.1, N=2176 17.6), clusters of two at 148.
+int choose_cluster_slices(int m, int n, int k, int num_sms, double whole_tiles_cost) {
+    const long tiles = static_cast<long>((m + 127) / 128) * ((n + 63) / 64);
+    const int kb = k / 128;
+    const double whole = 3.4 + 0.41 * whole_tiles_cost * kb;
+    int best = 0;
+    double best_time = 0.97 * whole;
+    for (int slices = 2; slices <= 4; slices *= 2) {
+        if (tiles * slices > (slices == 2 ? num_sms : num_sms * 7 / 8) || kb < 2 * slices) continue;
+        const double t = 5.9 + 0.235 * ((kb + slices - 1) / slices);
+        if (t < best_time) best = slices, best_time = t;
+    }
     return best;
 }
 
@@ -118,10 +139,12 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
     if (a.m == 0 || a.n == 0 || a.k == 0) return yan::kBadArgument;
     if (a.num_sms <= 0) return yan::kBadArgument;
     const bool want_auto = (block_n == 0);
+    double whole_tiles_cost = 0.0;
     if (block_n == 0) {
         const int rows = (type == yan::GemmType::GroupedMasked) ? static_cast<int>(a.m * a.num_groups) : static_cast<int>(a.m);
         block_n = choose_block_n(rows, static_cast<int>(a.n), static_cast<int>(a.k), a.num_sms,
-                                 type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16 && a.tail_workspace != nullptr);
+                                 type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16 && a.tail_workspace != nullptr,
+                                 &whole_tiles_cost);
     }
     a.status = status_word_of_current_device();
     a.timeout_ns = g_timeout_ns;
@@ -152,6 +175,15 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
             return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || after_own_quantizer);
         }
     }
+    if (type == yan::GemmType::Normal && want_auto && out_kind != yan::OutKind::E4M3 && a.scatter_world == 0) {
+        const int slices = choose_cluster_slices(static_cast<int>(a.m), static_cast<int>(a.n), static_cast<int>(a.k), a.num_sms,
+                                                 whole_tiles_cost);
+        if (slices != 0) return yan::launch_gemm_cluster_k(static_cast<uint32_t>(slices), out_kind, a, s);
+    }
+    // e4m3 output: 128-wide tiles while every CTA has at most one of them (M=225 N=1152 K=8064, 10 wide tiles or 18)
+    if (out_kind == yan::OutKind::E4M3 &&
+        static_cast<uint64_t>((a.m + 127) / 128) * ((a.n + 127) / 128) <= static_cast<uint64_t>(a.num_sms))
+        return yan::launch_gemm_e4m3_bn128(a, s);
     switch (block_n) {
         case 32: return yan::launch_gemm_bn32(type, out_kind, a, s);
         case 64: return yan::launch_gemm_bn64(type, out_kind, a, s);

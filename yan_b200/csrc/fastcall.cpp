@@ -94,9 +94,10 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         const int64_t ldd = out->stride(0);
         if (out->size(0) != m || out->size(1) != n || out->stride(1) != 1 || ldd < n || ldd > INT32_MAX || ldd % (bf16 ? 8 : 4) != 0)
             return code(kNotTaken);
-        // the compiled-per-shape route and the cut last wave (which needs scratch) stay with the Python path
-        if (bf16 && (jit_requested() || (block_n == 0 && k >= 96 * 128 && ceil_div(m, 128) * ceil_div(n, 256) > num_sms &&
-                                         PyObject_IsTrue(args[7]))))
+        // the compiled-per-shape route, the cut last wave (which needs scratch) and whole tiles on request stay with the
+        // Python path
+        if (bf16 && jit_requested()) return code(kNotTaken);
+        if (bf16 && block_n == 0 && (PyObject_IsTrue(args[7]) ? k >= 96 * 128 && ceil_div(m, 128) * ceil_div(n, 256) > num_sms : m > 64))
             return code(kNotTaken);
         const void *pa = a->data_ptr(), *pb = b->data_ptr();
         void* pout = out->data_ptr();

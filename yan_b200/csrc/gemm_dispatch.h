@@ -18,6 +18,11 @@ int launch_gemm_bn192(GemmType type, OutKind out, const GemmArgs& args, cudaStre
 int launch_gemm_bn224(GemmType type, OutKind out, const GemmArgs& args, cudaStream_t stream);
 int launch_gemm_bn256(GemmType type, OutKind out, const GemmArgs& args, cudaStream_t stream);
 
+// K of every 64-wide tile shared by a cluster of `slices` CTAs (GemmClusterKLauncher), bf16 or fp32 output.
+int launch_gemm_cluster_k(uint32_t slices, OutKind out, const GemmArgs& args, cudaStream_t stream);
+// e4m3 output on 128-wide tiles, one per CTA.
+int launch_gemm_e4m3_bn128(const GemmArgs& args, cudaStream_t stream);
+
 // Default pipeline depth per BLOCK_N: 128-wide k-block stages (16 KB of A + BLOCK_N * 128 bytes of B each) that fit
 // in 227 KB next to the barriers, at most 8.
 #ifndef YAN_STAGES_256

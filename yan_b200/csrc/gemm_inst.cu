@@ -37,4 +37,17 @@ int YAN_CAT(launch_gemm_bn, YAN_BLOCK_N)(GemmType type, OutKind out, const GemmA
     return kBadArgument;
 }
 
+#if YAN_BLOCK_N == 64
+int launch_gemm_cluster_k(uint32_t slices, OutKind out, const GemmArgs& args, cudaStream_t stream) {
+    // six stages leave room for the exchanged rows
+    if (out == OutKind::BF16) return GemmClusterKLauncher<64, 6, __nv_bfloat16>::launch(args, slices, stream);
+    if (out == OutKind::F32) return GemmClusterKLauncher<64, 6, float>::launch(args, slices, stream);
+    return kBadArgument;
+}
+#elif YAN_BLOCK_N == 128
+int launch_gemm_e4m3_bn128(const GemmArgs& args, cudaStream_t stream) {
+    return GemmClusterKLauncher<128, default_num_stages(128), E4m3Out>::launch(args, 1, stream);
+}
+#endif
+
 }  // namespace yan

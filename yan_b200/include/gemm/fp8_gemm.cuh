@@ -172,6 +172,97 @@ __device__ __forceinline__ void store_tile_e4m3(uint8_t* out, uint32_t ld, float
     }
 }
 
+// Where the exchanged rows of a kClusterK tile go: 35 KB behind the ring for 64-wide tiles (one meeting of the cluster less,
+// 0.3 us), over the ring for 128-wide ones (their 68 KB would cost two of six stages).
+template <uint32_t BLOCK_N>
+constexpr bool kExchangeInRing = BLOCK_N > 64;
+
+// The end of a tile whose K is shared by the CTAs of a cluster (kClusterK).
+template <typename out_t, uint32_t BLOCK_N, uint32_t kCols>
+__device__ __forceinline__ void exchange_and_store(const GemmParams& p, uint32_t smem, uint32_t slice, uint32_t tile_row0,
+                                                   uint32_t tile_col0, uint32_t row_in_tile, uint32_t col0, uint32_t thread,
+                                                   bool alive, const float (&acc)[kCols]) {
+    // [slice][own row][BLOCK_N + 4] floats; the padding spreads the rows a warp writes over the banks
+    constexpr uint32_t kRowBytes = (BLOCK_N + 4) * 4;
+    const uint32_t slices = p.tail_slices, own_rows = kBlockM / slices;
+    ptx::cluster_wait();  // every CTA of the cluster has started (it arrived at the top of the kernel) ...
+    // ... or, where the rows land in the operand ring, is done with it: its products are complete
+    if constexpr (kExchangeInRing<BLOCK_N>) ptx::cluster_arrive(), ptx::cluster_wait();
+    const uint32_t owner = row_in_tile / own_rows;
+    const uint32_t dst = ptx::map_to_cta(smem, owner) + (slice * own_rows + row_in_tile % own_rows) * kRowBytes + col0 * 4;
+#pragma unroll
+    for (uint32_t j = 0; j < kCols; j += 4) ptx::st_cluster_v4_f32(dst + j * 4, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+    ptx::cluster_arrive(), ptx::cluster_wait();
+    // 2 * slices threads per row, BLOCK_N / (2 * slices) columns each, eight at a time
+    const uint32_t per_row = 2 * slices, part = thread % per_row;
+    const uint32_t row_local = thread / per_row, row = tile_row0 + slice * own_rows + row_local;
+    const uint32_t cols = BLOCK_N / per_row;
+    constexpr uint32_t kMaxCols = sizeof(out_t) == 1 ? BLOCK_N / 2 : BLOCK_N / 4;  // one slice, or at least two
+    float v[kMaxCols];
+    const uint32_t src = smem + row_local * kRowBytes + part * cols * 4;
+#pragma unroll
+    for (uint32_t c = 0; c < kMaxCols; ++c) v[c] = 0.0f;
+    for (uint32_t s = 0; s < slices; ++s) {
+#pragma unroll
+        for (uint32_t c = 0; c < kMaxCols; c += 4) {
+            if (c < cols) {
+                const float4 t = ptx::ld_shared_v4_f32(src + s * own_rows * kRowBytes + c * 4);
+                v[c] += t.x, v[c + 1] += t.y, v[c + 2] += t.z, v[c + 3] += t.w;
+            }
+        }
+    }
+    const uint32_t n0 = tile_col0 + part * cols;
+    const bool row_ok = alive && row < p.shape_m;
+    if constexpr (sizeof(out_t) == 1) {
+        // the row's 128 columns are one quantization group, spread over per_row neighbouring lanes (see store_tile_e4m3)
+        float amax = 0.0f;
+#pragma unroll
+        for (uint32_t c = 0; c < kMaxCols; ++c)
+            if (c < cols) {
+                v[c] = __bfloat162float(__float2bfloat16_rn(v[c]));
+                amax = fmaxf(amax, fabsf(v[c]));
+            }
+        for (uint32_t off = 1; off < per_row; off *= 2) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+        const float amax_c = fmaxf(amax, 1e-4f), inv = __fdiv_rn(448.0f, amax_c);
+        if (row_ok && part == 0)
+            p.out_scales[static_cast<size_t>(tile_col0 / 128u) * p.out_scales_ld + row] = __fdiv_rn(amax_c, 448.0f);
+        uint8_t* out = reinterpret_cast<uint8_t*>(p.out) + static_cast<size_t>(row) * p.ldd + n0;
+#pragma unroll
+        for (uint32_t c = 0; c < kMaxCols; c += 8) {
+            if (c < cols && row_ok) {
+                uint32_t w[2];
+#pragma unroll
+                for (uint32_t i = 0; i < 2; ++i) {
+                    const float* a = v + c + i * 4;
+                    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a[0], inv), __fmul_rn(a[1], inv)),
+                                                                 __NV_SATFINITE, __NV_E4M3);
+                    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(__fmul_rn(a[2], inv), __fmul_rn(a[3], inv)),
+                                                                 __NV_SATFINITE, __NV_E4M3);
+                    w[i] = lo | (hi << 16);
+                }
+                *reinterpret_cast<uint2*>(out + c) = make_uint2(w[0], w[1]);
+            }
+        }
+    } else {
+        out_t* out = reinterpret_cast<out_t*>(p.out) + static_cast<size_t>(row) * p.ldd + n0;
+#pragma unroll
+        for (uint32_t c = 0; c < kMaxCols; c += 8) {
+            if (c < cols && row_ok && n0 + c < p.shape_n) {
+                if constexpr (sizeof(out_t) == 2) {
+                    __nv_bfloat162 t0 = __floats2bfloat162_rn(v[c], v[c + 1]), t1 = __floats2bfloat162_rn(v[c + 2], v[c + 3]);
+                    __nv_bfloat162 t2 = __floats2bfloat162_rn(v[c + 4], v[c + 5]), t3 = __floats2bfloat162_rn(v[c + 6], v[c + 7]);
+                    *reinterpret_cast<uint4*>(out + c) =
+                        make_uint4(*reinterpret_cast<uint32_t*>(&t0), *reinterpret_cast<uint32_t*>(&t1),
+                                   *reinterpret_cast<uint32_t*>(&t2), *reinterpret_cast<uint32_t*>(&t3));
+                } else {
+                    *reinterpret_cast<float4*>(out + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+                    *reinterpret_cast<float4*>(out + c + 4) = make_float4(v[c + 4], v[c + 5], v[c + 6], v[c + 7]);
+                }
+            }
+        }
+    }
+}
+
 }  // namespace detail
 
 // Output element type of the quantized-output GEMM: e4m3 codes plus one fp32 scale per (row, 128 columns).
@@ -277,7 +368,13 @@ using GemmOutputLayout =
 // allreduce: every finished bf16 tile goes straight to the rank that will sum it (plain stores to peer-mapped memory,
 // 128 contiguous bytes per row piece), while the MMAs of the next tiles run; gather_staged_allreduce_bf16_kernel in
 // comm/peer_allreduce.cuh is the other half.  This is the per-tile hand-over of the reference's epilogue (comm/gemm_allreduce.cu:339-410) without NVSHMEM.
-template <uint32_t BLOCK_N, uint32_t kNumStages, GemmType kGemmType, typename out_t, bool kTail = false, bool kScatter = false>
+// kClusterK: the instance for few tiles and long K.  A cluster of `tail_slices` CTAs shares one tile, each computing one
+// slice of K as in the tail instance; then every CTA sends the rows of its fp32 partial tile to the CTA of the cluster that
+// owns them (128 / slices rows each, through distributed shared memory), which adds the slices in order, rounds once and
+// stores.  One launch, no scratch in global memory.  With one slice it is the way to quantize a 128-wide tile, whose groups
+// of 128 columns are spread over both warpgroups.
+template <uint32_t BLOCK_N, uint32_t kNumStages, GemmType kGemmType, typename out_t, bool kTail = false, bool kScatter = false,
+          bool kClusterK = false>
 __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     fp8_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tensor_map_a,
                     const __grid_constant__ CUtensorMap tensor_map_b) {
@@ -343,14 +440,18 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     const uint32_t num_sb_rows = ceil_div(p.shape_n, 128u);
     static_assert(!kTail || (kGemmType == GemmType::Normal && sizeof(out_t) == 4), "the tail instance writes fp32 partials");
     static_assert(!kScatter || (kGemmType == GemmType::Normal && sizeof(out_t) == 2 && !kTail), "the scatter instance writes bf16 tiles");
+    static_assert(!kClusterK || (kGemmType == GemmType::Normal && !kTail && !kScatter && BLOCK_N <= 128), "one tile per cluster");
+    constexpr bool kCutK = kTail || kClusterK;
+    constexpr uint32_t kExchangeOffset = detail::kExchangeInRing<BLOCK_N> ? 0 : align_up(L::kOffAbort + 4, 16u);
+    if constexpr (kClusterK) ptx::cluster_arrive_relaxed();                // waited for in front of the exchange
     // k-blocks [kb_begin, kb_begin + kb_count) of every tile this CTA computes: all of them, or the CTA's slice
-    const uint32_t tail_slice = kTail ? blockIdx.x % p.tail_slices : 0u, tail_tile = kTail ? blockIdx.x / p.tail_slices : 0u;
-    const uint32_t kb_begin = kTail ? (tail_slice * num_k_blocks) / p.tail_slices : 0u;
-    const uint32_t kb_count = kTail ? ((tail_slice + 1) * num_k_blocks) / p.tail_slices - kb_begin : num_k_blocks;
+    const uint32_t tail_slice = kCutK ? blockIdx.x % p.tail_slices : 0u, tail_tile = kCutK ? blockIdx.x / p.tail_slices : 0u;
+    const uint32_t kb_begin = kCutK ? (tail_slice * num_k_blocks) / p.tail_slices : 0u;
+    const uint32_t kb_count = kCutK ? ((tail_slice + 1) * num_k_blocks) / p.tail_slices - kb_begin : num_k_blocks;
     // next tile of this CTA: the persistent walk, or the tail instance's single tile
     [[maybe_unused]] bool tail_taken = false;
     auto next_tile = [&](Sched& sched, uint32_t& m_block_idx, uint32_t& n_block_idx) -> bool {
-        if constexpr (kTail) {
+        if constexpr (kCutK) {
             if (tail_taken || tail_tile >= p.tail_tiles) return false;
             tail_taken = true;
             sched.swizzle(p.tail_first_tile + tail_tile, sched.num_m_blocks, m_block_idx, n_block_idx);
@@ -503,6 +604,11 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
 #endif
         }
         __syncwarp();
+        if constexpr (kClusterK) {  // the two meetings of the exchange below
+            ptx::cluster_wait();
+            if constexpr (detail::kExchangeInRing<BLOCK_N>) ptx::cluster_arrive(), ptx::cluster_wait();
+            ptx::cluster_arrive(), ptx::cluster_wait();
+        }
     } else {
         // ------------------------------ promotion + epilogue warpgroups ------------------------------
         ptx::reg_alloc<get_num_math_registers(BLOCK_N)>();
@@ -529,15 +635,15 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             const bool row_ok = row < sched.get_row_limit();
             const uint32_t n_first = n_block_idx * BLOCK_N + col0;
             const uint32_t sb_row = min(n_first / 128u, num_sb_rows - 1);
-            const float* sa_ptr = p.scales_a + (kTail ? static_cast<size_t>(kb_begin) * p.sa_ld : 0) + row;
+            const float* sa_ptr = p.scales_a + (kCutK ? static_cast<size_t>(kb_begin) * p.sa_ld : 0) + row;
             const float* sb_ptr =
-                p.scales_b + (static_cast<size_t>(group) * num_sb_rows + sb_row) * num_k_blocks + (kTail ? kb_begin : 0u);
+                p.scales_b + (static_cast<size_t>(group) * num_sb_rows + sb_row) * num_k_blocks + (kCutK ? kb_begin : 0u);
             const float* sa_next = sa_ptr + static_cast<size_t>(kScaleDepth) * p.sa_ld;  // row's scale kScaleDepth k-blocks ahead
             // two-scale case: groups of 16 columns from `hi_from` on belong to the next 128-column block
             const uint32_t hi_from = kTwoScales ? (128u - n_first % 128u) / 16u : 0xFFFFu;
             const float* sb_hi_ptr = p.scales_b +
                                      (static_cast<size_t>(group) * num_sb_rows + min(sb_row + 1, num_sb_rows - 1)) * num_k_blocks +
-                                     (kTail ? kb_begin : 0u);
+                                     (kCutK ? kb_begin : 0u);
 
             // Scales are prefetched kScaleDepth k-blocks ahead: one L2 round trip is longer than one k-block.
             float sa_ring[kScaleDepth], sb_ring[kScaleDepth], sb_hi_ring[kTwoScales ? kScaleDepth : 1];
@@ -638,6 +744,12 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                 }
             }
             YAN_STAMP(s0);
+            if constexpr (kClusterK) {
+                detail::exchange_and_store<out_t, BLOCK_N>(p, ptx::smem_u32(smem) + kExchangeOffset, tail_slice, m_block_idx * kBlockM,
+                                                           n_block_idx * BLOCK_N, row_in_tile, col0, threadIdx.x - kNumControlThreads,
+                                                           alive && *abort_flag == 0, acc);
+                continue;
+            }
             // the e4m3 output needs one 128-column group per thread (BLOCK_N = 256, two warpgroups): the launcher refuses every
             // other shape of CTA
             if constexpr (sizeof(out_t) == 1 && kColsPerWG == 128) {
@@ -835,64 +947,73 @@ __global__ void __launch_bounds__(256) reduce_tail_partials_kernel(const float* 
 
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
+// Host-side checks of a launch (smem_size: what its kernel needs) and its device-side parameters.
+inline int check_and_fill(const GemmArgs& a, GemmType type, uint32_t out_bytes, uint32_t smem_size, GemmParams& p,
+                          uint64_t& a_rows, uint64_t& b_rows, int& max_smem) {
+    if (a.lhs == nullptr || a.lhs_scales == nullptr || a.rhs == nullptr || a.rhs_scales == nullptr ||
+        a.out == nullptr)
+        return kBadArgument;
+    if (a.m == 0 || a.n == 0 || a.k == 0 || a.k % kBlockK != 0 || a.n % 16 != 0 || a.num_groups == 0)
+        return kBadArgument;
+    const uint32_t vec = 16 / out_bytes;
+    if (a.ldd < a.n || a.ldd % vec != 0 || a.lhs_scales_ld == 0) return kBadArgument;
+    if (!is_aligned(a.lhs, 16) || !is_aligned(a.rhs, 16) || !is_aligned(a.out, 16) || !is_aligned(a.lhs_scales, 4) ||
+        !is_aligned(a.rhs_scales, 4))
+        return kBadArgument;
+    if (out_bytes == 1 &&
+        (a.out_scales == nullptr || a.out_scales_ld < a.m || a.n % 128 != 0 || !is_aligned(a.out_scales, 4)))
+        return kBadArgument;
+    if (type != GemmType::Normal && a.grouped_layout == nullptr) return kBadArgument;
+    if (type == GemmType::Normal && a.num_groups != 1) return kBadArgument;
+    if (a.num_sms <= 0) return kBadArgument;
+    
+    int device = 0, sm_count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) return kLaunchFailed;
+    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
+    if (static_cast<int>(smem_size) > max_smem) return kSmemTooLarge;
+    if (a.num_sms > sm_count) return kBadArgument;
+    
+    a_rows = (type == GemmType::GroupedMasked) ? static_cast<uint64_t>(a.m) * a.num_groups : a.m;
+    b_rows = static_cast<uint64_t>(a.n) * a.num_groups;
+    if (a_rows > 0x7fffffffull || b_rows > 0x7fffffffull) return kBadArgument;
+    if (type == GemmType::GroupedMasked ? a.lhs_scales_ld < a_rows : a.lhs_scales_ld < a.m)
+        return kBadArgument;
+
+    p.scales_a = a.lhs_scales;
+    p.scales_b = a.rhs_scales;
+    p.grouped_layout = a.grouped_layout;
+    p.out = a.out;
+    p.out_scales = a.out_scales;
+    p.out_scales_ld = a.out_scales_ld;
+    p.sa_ld = a.lhs_scales_ld;
+    p.ldd = a.ldd;
+    p.shape_m = a.m;
+    p.shape_n = a.n;
+    p.shape_k = a.k;
+    p.num_groups = a.num_groups;
+    p.status = a.status;
+    p.timeout_ns = a.timeout_ns;
+    p.clock_probe = a.clock_probe;
+    return kOk;
+}
+
 template <uint32_t BLOCK_N, uint32_t kNumStages, GemmType kGemmType, typename out_t>
 struct GemmLauncher {
     using L = GemmOutputLayout<BLOCK_N, kNumStages, sizeof(out_t) == 4>;
     static constexpr uint32_t kSmemSize = L::kSmemSize;
 
     static int launch(const GemmArgs& a, cudaStream_t stream) {
-        if (a.lhs == nullptr || a.lhs_scales == nullptr || a.rhs == nullptr || a.rhs_scales == nullptr ||
-            a.out == nullptr)
-            return kBadArgument;
-        if (a.m == 0 || a.n == 0 || a.k == 0 || a.k % kBlockK != 0 || a.n % 16 != 0 || a.num_groups == 0)
-            return kBadArgument;
-        constexpr uint32_t kVec = 16 / sizeof(out_t);
-        if (a.ldd < a.n || a.ldd % kVec != 0 || a.lhs_scales_ld == 0) return kBadArgument;
-        if (!is_aligned(a.lhs, 16) || !is_aligned(a.rhs, 16) || !is_aligned(a.out, 16) || !is_aligned(a.lhs_scales, 4) ||
-            !is_aligned(a.rhs_scales, 4))
-            return kBadArgument;
-        if (sizeof(out_t) == 1 &&
-            (a.out_scales == nullptr || a.out_scales_ld < a.m || a.n % 128 != 0 || !is_aligned(a.out_scales, 4)))
-            return kBadArgument;
-        if (kGemmType != GemmType::Normal && a.grouped_layout == nullptr) return kBadArgument;
-        if (kGemmType == GemmType::Normal && a.num_groups != 1) return kBadArgument;
-        if (a.num_sms <= 0) return kBadArgument;
-
-        int device = 0, max_smem = 0, sm_count = 0;
-        if (cudaGetDevice(&device) != cudaSuccess) return kLaunchFailed;
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
-        if (static_cast<int>(kSmemSize) > max_smem) return kSmemTooLarge;
-        if (a.num_sms > sm_count) return kBadArgument;
-
-        const uint64_t a_rows =
-            (kGemmType == GemmType::GroupedMasked) ? static_cast<uint64_t>(a.m) * a.num_groups : a.m;
-        const uint64_t b_rows = static_cast<uint64_t>(a.n) * a.num_groups;
-        if (a_rows > 0x7fffffffull || b_rows > 0x7fffffffull) return kBadArgument;
-        if (kGemmType == GemmType::GroupedMasked ? a.lhs_scales_ld < a_rows : a.lhs_scales_ld < a.m)
-            return kBadArgument;
+        GemmParams p;
+        int max_smem = 0;
+        uint64_t a_rows = 0, b_rows = 0;
+        const int rc = check_and_fill(a, kGemmType, sizeof(out_t), kSmemSize, p, a_rows, b_rows, max_smem);
+        if (rc != kOk) return rc;
 
         bool ok = true;
         const CUtensorMap map_a = make_2d_tma_desc_u8_sw128(a.lhs, a_rows, a.k, a.k, kBlockM, ok);
         const CUtensorMap map_b = make_2d_tma_desc_u8_sw128(a.rhs, b_rows, a.k, a.k, BLOCK_N, ok);
         if (!ok) return kTensorMapFailed;
-
-        GemmParams p;
-        p.scales_a = a.lhs_scales;
-        p.scales_b = a.rhs_scales;
-        p.grouped_layout = a.grouped_layout;
-        p.out = a.out;
-        p.out_scales = a.out_scales;
-        p.out_scales_ld = a.out_scales_ld;
-        p.sa_ld = a.lhs_scales_ld;
-        p.ldd = a.ldd;
-        p.shape_m = a.m;
-        p.shape_n = a.n;
-        p.shape_k = a.k;
-        p.num_groups = a.num_groups;
-        p.status = a.status;
-        p.timeout_ns = a.timeout_ns;
-        p.clock_probe = a.clock_probe;
 
         auto kernel = fp8_gemm_kernel<BLOCK_N, kNumStages, kGemmType, out_t>;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSize) != cudaSuccess) {
@@ -984,6 +1105,55 @@ struct GemmLauncher {
         }
         kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), kSmemSize, stream>>>(p, map_a, map_b);
         return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    }
+};
+
+// Few tiles, long K: one cluster of `slices` CTAs per tile (the kClusterK instance).
+template <uint32_t BLOCK_N, uint32_t kNumStages, typename out_t>
+struct GemmClusterKLauncher {
+    using L = GemmOutputLayout<BLOCK_N, kNumStages, sizeof(out_t) == 4>;
+
+    static int launch(const GemmArgs& a, uint32_t slices, cudaStream_t stream) {
+        constexpr uint32_t kRowsBytes = kBlockM * (BLOCK_N + 4) * 4;  // the exchanged rows
+        constexpr uint32_t kSmemSize = L::kSmemSize + (detail::kExchangeInRing<BLOCK_N> ? 0 : 16 + kRowsBytes);
+        static_assert(!detail::kExchangeInRing<BLOCK_N> || L::kOffStore >= kRowsBytes, "the rows fit in the ring");
+        // a thread finishes BLOCK_N / (2 * slices) columns of a row, eight at a time; e4m3 output is promised to equal the
+        // quantized bf16 output bit for bit, so its K is not cut
+        if (sizeof(out_t) == 1 ? slices != 1 : (slices != 2 && slices != 4)) return kBadArgument;
+        if (BLOCK_N / (2 * slices) < 8 || slices > a.k / kBlockK) return kBadArgument;
+        GemmParams p;
+        int max_smem = 0;
+        uint64_t a_rows = 0, b_rows = 0;
+        const int rc = check_and_fill(a, GemmType::Normal, sizeof(out_t), kSmemSize, p, a_rows, b_rows, max_smem);
+        if (rc != kOk) return rc;
+        bool ok = true;
+        const CUtensorMap map_a = make_2d_tma_desc_u8_sw128(a.lhs, a_rows, a.k, a.k, kBlockM, ok);
+        const CUtensorMap map_b = make_2d_tma_desc_u8_sw128(a.rhs, b_rows, a.k, a.k, BLOCK_N, ok);
+        if (!ok) return kTensorMapFailed;
+        p.tail_tiles = ceil_div(a.m, kBlockM) * ceil_div(a.n, BLOCK_N);
+        p.tail_slices = slices;
+        auto kernel = fp8_gemm_kernel<BLOCK_N, kNumStages, GemmType::Normal, out_t, false, false, true>;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemSize) != cudaSuccess) {
+            cudaGetLastError();
+            return kSmemTooLarge;
+        }
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = slices;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(p.tail_tiles * slices);
+        cfg.blockDim = dim3(get_num_threads_per_sm<>(BLOCK_N));
+        cfg.dynamicSmemBytes = kSmemSize;
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = slices > 1 ? 1 : 0;
+        if (cudaLaunchKernelEx(&cfg, kernel, p, map_a, map_b) != cudaSuccess) {
+            cudaGetLastError();
+            return kLaunchFailed;
+        }
+        return kOk;
     }
 };
 

@@ -158,6 +158,8 @@ def gemm_fp8_fp8_bf16_nt(lhs: Tuple[torch.Tensor, torch.Tensor], rhs: Tuple[torc
                   rhs_scales.data_ptr(), out.data_ptr(), m, n, k, out.stride(0), _stream_ptr(), num_sms, block_n,
                   ws.data_ptr(), ws.numel())
         return
+    if block_n == 0 and m > 64 and not tail_cut_enabled():
+        block_n = get_best_configs(m, n, k, num_sms)[0]  # whole tiles: the library would cut K where there are few of them
     _lib.call("yan_b200_gemm_fp8_fp8_bf16_nt", lhs_q.data_ptr(), lhs_scales.data_ptr(), rhs_q.data_ptr(),
               rhs_scales.data_ptr(), out.data_ptr(), m, n, k, out.stride(0), _stream_ptr(), num_sms, block_n)
 
@@ -171,8 +173,9 @@ def tail_cut_enabled() -> bool:
 
 
 def set_tail_cut(enabled: bool) -> None:
-    """Lets gemm_fp8_fp8_bf16_nt(block_n=0) cut the tiles of a nearly empty last wave along K (default on).  Off, or
-    with an explicit block_n, every tile is computed whole by one CTA and the result does not depend on the grid."""
+    """Lets gemm_fp8_fp8_bf16_nt(block_n=0) cut tiles along K: those of a nearly empty last wave, and all of them where there
+    are too few to occupy the GPU (default on).  Off, or with an explicit block_n, every tile of more than 64 rows is computed
+    whole by one CTA and the result does not depend on the grid."""
     _tail_cut[0] = bool(enabled)
 
 
