@@ -65,14 +65,6 @@ __host__ __device__ inline uint32_t small_m_tmem_cols(uint32_t m_pad, uint32_t k
     return cols;
 }
 
-namespace ptx {
-__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
-    float v;
-    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
-    return v;
-}
-}  // namespace ptx
-
 template <uint32_t M_PAD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
     fp8_gemm_small_m_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tensor_map_w,

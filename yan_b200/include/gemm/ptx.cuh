@@ -132,6 +132,22 @@ __device__ __forceinline__ float4 ld_shared_v4_f32(uint32_t addr) {
     return v;
 }
 
+__device__ __forceinline__ float ld_shared_f32(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// Asynchronous 4-byte copies global -> shared; the arrival (one of the barrier's count) happens when this thread's copies so
+// far have landed.
+__device__ __forceinline__ void cp_async_4(uint32_t smem_dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_mbar_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Thread-block clusters: the barrier of all threads of all CTAs (in two halves), the address of the same offset in another
 // CTA's shared memory, stores to it.
 __device__ __forceinline__ uint32_t cluster_ctarank() {

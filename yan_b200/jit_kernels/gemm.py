@@ -274,6 +274,10 @@ def m_grouped_gemm_fp8_fp8_bf16_nt_masked(lhs, rhs, out: torch.Tensor, masked_m:
     assert lhs_scales.shape == (g, m_max, k // 128) and rhs_scales.shape == (g, n // 128, k // 128)
     assert out.shape == (g, m_max, n) and out.dtype == torch.bfloat16
     assert masked_m.shape == (g,) and masked_m.dtype == torch.int32 and masked_m.is_contiguous()
+    if block_n == 0 and 64 < m_max <= 128 and expected_m > 96:
+        # nearly full groups: tiles of 128 rows beat the kernel that follows masked_m (16 groups of 120 rows, N=4096 K=2048:
+        # 35.8 us against 38.8; of 80 rows 35.3 against 35.7, of 24 33.4 against 30.1)
+        block_n = get_best_configs(g * m_max, n, k, get_num_sms())[0]
     # k-block-major over the flattened G*M_max rows
     sa = lhs_scales.reshape(g * m_max, k // 128)
     sa = get_col_major_tensor(sa)
