@@ -291,9 +291,15 @@ struct GemmSmemLayout {
     static constexpr uint32_t kOffStore = kOffB + kNumStages * SMEM_B_SIZE_PER_STAGE;
     static constexpr uint32_t kStoreBytes =
         (kOffStore + kNumStoreBoxes * kStoreBoxBytes + 2048 <= 232448) ? kNumStoreBoxes * kStoreBoxBytes : 0;
-    static constexpr uint32_t kOffBarriers = kOffStore + kStoreBytes;
+    // The scales of the k-blocks in flight, copied asynchronously by the producer warp (see there): [slot][128 sA, then the sB of up to
+    // three 128-column blocks].  kScaleRing: where they fit beside the rings and boxes; otherwise (the scatter instance's wide
+    // boxes, 96-wide tiles with eight stages) every promotion thread loads its scales into registers.
+    static constexpr uint32_t kNumScaleSlots = kNumStages + kNumTmemBufs + 1, kScaleSlotBytes = (128 + 4) * 4;
+    static constexpr uint32_t kOffScales = kOffStore + kStoreBytes;
+    static constexpr bool kScaleRing = kOffScales + kNumScaleSlots * kScaleSlotBytes + 2048 <= 232448;
+    static constexpr uint32_t kOffBarriers = kOffScales + (kScaleRing ? kNumScaleSlots * kScaleSlotBytes : 0);
     // ring full/empty, TMEM full/empty per buffer and column half
-    static constexpr uint32_t kNumBarriers = 2 * kNumStages + 4 * kNumTmemBufs;
+    static constexpr uint32_t kNumBarriers = 2 * kNumStages + 4 * kNumTmemBufs + (kScaleRing ? kNumScaleSlots : 0);
     static constexpr uint32_t kOffTmemSlot = kOffBarriers + kNumBarriers * 8;
     static constexpr uint32_t kOffAbort = kOffTmemSlot + 4;
     // +1024: the dynamic shared-memory base is re-aligned to 1024 bytes inside the kernel.
@@ -312,10 +318,9 @@ struct GemmSmemLayout {
 //                          warpgroup has read it.  0: one full-width stream, one barrier pair per buffer.
 //   YAN_PROMO_EARLY_PROBE  1: the next k-block's TMEM-full barrier is probed (without blocking) right after this
 //                          k-block's last load, so that the answer arrives under the last FMAs.
-//   YAN_WIDE_STORE_BOXES   1: every instance stages its output in 32 x 128-byte boxes.  The scatter instance and fp32
-//                          output always do (half the passes: M=4096 N=8192 K=3584 145.5 -> 142.4 us, M=2000 N=4096
-//                          K=1024 18.4 -> 16.4); for a local bf16 output it measured within +-1 % on the large shapes
-//                          and 3 % slower on M=8192 N=3584 K=8192, so that keeps the 64-byte rows.
+//   YAN_WIDE_STORE_BOXES   1: every instance stages its output in 32 x 128-byte boxes.  The scatter instance always does,
+//                          fp32 output on 256-wide tiles where K < YAN_WIDE_F32_MAX_K (see GemmLauncher); for a local bf16
+//                          output it measured within +-1 % on the large shapes and 3 % slower on M=8192 N=3584 K=8192.
 // Measured and dropped: handing the TMEM read port back and forth between the two warps of a sub-partition through
 // mbarriers (an arrive-to-wait hand-over costs ~100 cycles: 778 and 1163 cycles per k-block for 64- and 32-column turns
 // against 343 without), and four promotion warpgroups (874 cycles per k-block against 733: the per-k-block bookkeeping
@@ -328,6 +333,9 @@ struct GemmSmemLayout {
 #endif
 #ifndef YAN_TAIL_MIN_K_BLOCKS
 #define YAN_TAIL_MIN_K_BLOCKS 96
+#endif
+#ifndef YAN_WIDE_F32_MAX_K
+#define YAN_WIDE_F32_MAX_K 6144
 #endif
 #ifndef YAN_PROMO_EARLY_PROBE
 #define YAN_PROMO_EARLY_PROBE 0
@@ -373,13 +381,14 @@ using GemmOutputLayout =
 // owns them (128 / slices rows each, through distributed shared memory), which adds the slices in order, rounds once and
 // stores.  One launch, no scratch in global memory.  With one slice it is the way to quantize a 128-wide tile, whose groups
 // of 128 columns are spread over both warpgroups.
+// kWideBoxes: 128-byte box rows in the epilogue (always in the scatter instance).
 template <uint32_t BLOCK_N, uint32_t kNumStages, GemmType kGemmType, typename out_t, bool kTail = false, bool kScatter = false,
-          bool kClusterK = false>
+          bool kClusterK = false, bool kWideBoxes = kScatter>
 __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     fp8_gemm_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tensor_map_a,
                     const __grid_constant__ CUtensorMap tensor_map_b) {
 #if defined(__CUDA_ARCH__) && (__CUDA_ARCH__ >= 1000)
-    using L = GemmOutputLayout<BLOCK_N, kNumStages, kScatter || (sizeof(out_t) == 4 && !kTail)>;
+    using L = GemmOutputLayout<BLOCK_N, kNumStages, kWideBoxes>;
     using Sched = Scheduler<kGemmType, kBlockM, BLOCK_N>;
     constexpr uint32_t kNumTmemBufs = L::kNumTmemBufs;
     constexpr uint32_t kNumMathWGs = get_num_math_warpgroups(BLOCK_N);
@@ -431,6 +440,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     uint64_t* empty_barriers = full_barriers + kNumStages;
     uint64_t* tmem_full_barriers = empty_barriers + kNumStages;            // [buf][half]
     uint64_t* tmem_empty_barriers = tmem_full_barriers + 2 * kNumTmemBufs;  // [buf][half]
+    uint64_t* scale_full_barriers = tmem_empty_barriers + 2 * kNumTmemBufs;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffTmemSlot);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kOffAbort);
 
@@ -479,6 +489,10 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             ptx::mbar_init(tmem_full_barriers + i, 1);                             // tcgen05.commit
             ptx::mbar_init(tmem_empty_barriers + i, kNumMathWarps / kNumHalves);  // one arrival per promotion warp
         }
+        if constexpr (L::kScaleRing) {
+#pragma unroll
+            for (uint32_t i = 0; i < L::kNumScaleSlots; ++i) ptx::mbar_init(scale_full_barriers + i, 32);  // lanes of warp 0
+        }
         *abort_flag = 0;
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
@@ -499,40 +513,80 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     if (warp_idx < 4) {
         ptx::reg_dealloc<get_num_control_registers(BLOCK_N)>();
 
-        if (warp_idx == 0 && lane_idx == 0) {
-            // ------------------------------ TMA producer ------------------------------
+        if (warp_idx == 0 && (L::kScaleRing || lane_idx == 0)) {
+            // ------------------------------ producer ------------------------------
+            // Lane 0 loads a k-block's operands; with kScaleRing all lanes copy its scales to shared memory at the same time, so
+            // that they are there kNumStages k-blocks before the promotion needs them (loads into registers, however far ahead,
+            // end up waiting for an L2 round trip: a moved register waits for its load, and the loads in flight share a few
+            // scoreboards.  M=4096 N=7168 K=18432 whole tiles 764 -> 650 cycles per k-block, 597 -> 541 us; M=8192 N=7168
+            // K=2048 141.7 -> 139.0; M=8192 N=28672 K=8192 unchanged, held by the power cap).
+            // A scale slot is rewritten after kNumScaleSlots k-blocks: the MMAs that freed the operand stage had waited for an
+            // accumulator, and every promotion warp had read that accumulator, and the scales of the k-block before it, by then.
+            // The same warp has to do both: a warp that only copies scales could fall so far behind that a stage's barrier
+            // completes two phases, which looks like none.  (Two producers, one per operand, measured 1 - 20 % slower.)
             Sched sched(p.shape_m, p.shape_n, p.grouped_layout, p.num_groups);
             if (p.tile_limit != 0) sched.num_blocks = min(sched.num_blocks, p.tile_limit);
             uint32_t m_block_idx, n_block_idx, stage = 0, phase = 0;
+            [[maybe_unused]] uint32_t slot = 0;
+            [[maybe_unused]] const uint32_t s_scales = ptx::smem_u32(smem + L::kOffScales);
+            [[maybe_unused]] const bool sa_aligned = p.sa_ld % 4 == 0 && reinterpret_cast<uintptr_t>(p.scales_a) % 16 == 0;
             bool alive = true;
             [[maybe_unused]] long long waited_empty = 0;
             while (alive && next_tile(sched, m_block_idx, n_block_idx)) {
                 const int group = sched.get_group(m_block_idx);
                 if (group < 0) continue;
-                const int32_t a_row = static_cast<int32_t>(sched.get_row_base(m_block_idx));
+                const uint32_t row0 = sched.get_row_base(m_block_idx);
+                const int32_t a_row = static_cast<int32_t>(row0);
                 const int32_t b_row = static_cast<int32_t>(group * p.shape_n + n_block_idx * BLOCK_N);
+                [[maybe_unused]] const uint32_t row_limit = sched.get_row_limit();
+                [[maybe_unused]] const bool whole = sa_aligned && row0 % 4 == 0 && row0 + kBlockM <= row_limit;  // 16 bytes per lane
+                [[maybe_unused]] const float* sa_ptr = p.scales_a + static_cast<size_t>(kb_begin) * p.sa_ld + row0;
+                const uint32_t sb_row = min(n_block_idx * BLOCK_N / 128u + lane_idx, num_sb_rows - 1);
+                [[maybe_unused]] const float* sb_ptr =
+                    p.scales_b + (static_cast<size_t>(group) * num_sb_rows + sb_row) * num_k_blocks + kb_begin;
                 for (uint32_t kb = kb_begin; kb < kb_begin + kb_count; ++kb) {
                     YAN_STAMP(w0);
-                    if (!detail::bounded_wait(empty_barriers + stage, phase ^ 1, abort_flag, p, 1)) {
+                    bool ok = detail::bounded_wait(empty_barriers + stage, phase ^ 1, abort_flag, p, 1);
+                    if constexpr (L::kScaleRing) ok = __all_sync(0xffffffffu, ok);
+                    if (!ok) {
                         alive = false;
                         break;
                     }
                     YAN_STAMP(w1);
                     YAN_STAMP_ADD(waited_empty, w0, w1);
-                    ptx::mbar_arrive_expect_tx(full_barriers + stage,
-                                               L::SMEM_A_SIZE_PER_STAGE + L::SMEM_B_SIZE_PER_STAGE);
-                    ptx::tma_load_2d(smem + L::kOffA + stage * L::SMEM_A_SIZE_PER_STAGE, &tensor_map_a,
-                                     full_barriers + stage, static_cast<int32_t>(kb * kBlockK), a_row);
-                    ptx::tma_load_2d(smem + L::kOffB + stage * L::SMEM_B_SIZE_PER_STAGE, &tensor_map_b,
-                                     full_barriers + stage, static_cast<int32_t>(kb * kBlockK), b_row);
+                    if (!L::kScaleRing || lane_idx == 0) {
+                        ptx::mbar_arrive_expect_tx(full_barriers + stage,
+                                                   L::SMEM_A_SIZE_PER_STAGE + L::SMEM_B_SIZE_PER_STAGE);
+                        ptx::tma_load_2d(smem + L::kOffA + stage * L::SMEM_A_SIZE_PER_STAGE, &tensor_map_a,
+                                         full_barriers + stage, static_cast<int32_t>(kb * kBlockK), a_row);
+                        ptx::tma_load_2d(smem + L::kOffB + stage * L::SMEM_B_SIZE_PER_STAGE, &tensor_map_b,
+                                         full_barriers + stage, static_cast<int32_t>(kb * kBlockK), b_row);
+                    }
+                    if constexpr (L::kScaleRing) {
+                        __syncwarp();
+                        const uint32_t dst = s_scales + slot * L::kScaleSlotBytes;
+                        if (whole) {
+                            ptx::cp_async_16(dst + lane_idx * 16u, sa_ptr + lane_idx * 4u);
+                        } else {
+#pragma unroll
+                            for (uint32_t i = 0; i < kBlockM; i += 32u)
+                                if (row0 + lane_idx + i < row_limit) ptx::cp_async_4(dst + (lane_idx + i) * 4u, sa_ptr + lane_idx + i);
+                        }
+                        if (lane_idx < 3) ptx::cp_async_4(dst + (kBlockM + lane_idx) * 4u, sb_ptr);
+                        ptx::cp_async_mbar_arrive(scale_full_barriers + slot);
+                        sa_ptr += p.sa_ld;
+                        ++sb_ptr;
+                        slot = slot + 1 == L::kNumScaleSlots ? 0 : slot + 1;
+                    }
                     if (++stage == kNumStages) {
                         stage = 0;
                         phase ^= 1;
                     }
                 }
             }
+            if constexpr (L::kScaleRing) ptx::cp_async_wait_all();
 #ifdef YAN_PHASE_STAMPS
-            if (p.clock_probe != nullptr && blockIdx.x == 0) p.clock_probe[4] = waited_empty;
+            if (p.clock_probe != nullptr && blockIdx.x == 0 && lane_idx == 0) p.clock_probe[4] = waited_empty;
 #endif
             if (!alive) {
                 // Give copies still in flight time to land before the CTA's shared memory is released.
@@ -623,6 +677,8 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
         Sched sched(p.shape_m, p.shape_n, p.grouped_layout, p.num_groups);
         if (p.tile_limit != 0) sched.num_blocks = min(sched.num_blocks, p.tile_limit);
         uint32_t m_block_idx, n_block_idx, buf = 0, buf_phase = 0;
+        [[maybe_unused]] uint32_t slot = 0, slot_phase = 0;
+        [[maybe_unused]] const uint32_t s_scales = ptx::smem_u32(smem + L::kOffScales);
         bool alive = true, next_ready = false;
         float acc[kColsPerWG];
         [[maybe_unused]] long long waited_tmem_full = 0, in_loads = 0, in_fmas = 0, in_stores = 0, promoted = 0;
@@ -645,10 +701,11 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                                      (static_cast<size_t>(group) * num_sb_rows + min(sb_row + 1, num_sb_rows - 1)) * num_k_blocks +
                                      (kCutK ? kb_begin : 0u);
 
-            // Scales are prefetched kScaleDepth k-blocks ahead: one L2 round trip is longer than one k-block.
+            // Without the ring in shared memory, scales are prefetched into registers kScaleDepth k-blocks ahead.
+            [[maybe_unused]] const uint32_t sb_offset = (kBlockM + n_first / 128u - n_block_idx * BLOCK_N / 128u) * 4u;
             float sa_ring[kScaleDepth], sb_ring[kScaleDepth], sb_hi_ring[kTwoScales ? kScaleDepth : 1];
 #pragma unroll
-            for (uint32_t i = 0; i < kScaleDepth; ++i) {
+            for (uint32_t i = 0; i < kScaleDepth && !L::kScaleRing; ++i) {
                 sa_ring[i] = (row_ok && i < kb_count) ? __ldg(sa_ptr + static_cast<size_t>(i) * p.sa_ld) : 0.0f;
                 sb_ring[i] = (i < kb_count) ? __ldg(sb_ptr + i) : 0.0f;
                 if constexpr (kTwoScales) sb_hi_ring[i] = (i < kb_count) ? __ldg(sb_hi_ptr + i) : 0.0f;
@@ -656,90 +713,121 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
 #pragma unroll
             for (uint32_t j = 0; j < kColsPerWG; ++j) acc[j] = 0.0f;
 
-            // kShiftRing: one copy of the loop body, the ring of scales moved down one slot per k-block (a few register
-            // moves); otherwise the body is unrolled once per ring slot and every copy uses its own slot.
-            for (uint32_t kb0 = 0; kb0 < kb_count && alive; kb0 += kLoopUnroll) {
-#pragma unroll(kLoopUnroll)
-                for (uint32_t i = 0; i < kLoopUnroll; ++i) {
-                    const uint32_t kb = kb0 + i;
-                    if (!alive || (kLoopUnroll > 1 && kb >= kb_count)) continue;
-                    const uint32_t use = kShiftRing ? 0 : i, fill = kShiftRing ? kScaleDepth - 1 : i;
-                    const float scale = sa_ring[use] * sb_ring[use];
-                    float scale_hi = scale;
-                    if constexpr (kTwoScales) scale_hi = sa_ring[use] * sb_hi_ring[use];
-                    if constexpr (kShiftRing) {
+            // Adds the accumulator of the k-block whose products are complete, and hands it back.
+            auto promote = [&](const float scale, [[maybe_unused]] const float scale_hi) {
+                YAN_STAMP_ADD(promoted, 0, 1);
+                ptx::tcgen05_fence_after_thread_sync();
+                const uint32_t taddr = tmem_lane_base + buf * BLOCK_N;
+
+                // The TMEM buffer is handed back as soon as the last columns have landed, before their FMAs.
+                // Nothing is scheduled between a tcgen05.ld and its wait: FMAs issued while a load is
+                // outstanding were measured ~10x slower than after it (the load does not overlap with the
+                // issuing warp's own arithmetic), so the overlap has to come from the sibling warp.
+                auto release_buffer = [&]() {
+                    ptx::tcgen05_fence_before_thread_sync();
+                    __syncwarp();
+                    if (lane_idx == 0) ptx::mbar_arrive(tmem_empty_barriers + buf * 2 + half);
+                };
+                auto group_scale = [&](uint32_t group16) { return (kTwoScales && group16 >= hi_from) ? scale_hi : scale; };
 #pragma unroll
-                        for (uint32_t r = 0; r + 1 < kScaleDepth; ++r) {
-                            sa_ring[r] = sa_ring[r + 1];
-                            sb_ring[r] = sb_ring[r + 1];
-                            if constexpr (kTwoScales) sb_hi_ring[r] = sb_hi_ring[r + 1];
+                for (uint32_t c = 0; c < kNumChunks; ++c) {
+                    uint32_t t[kChunk];
+                    YAN_STAMP(l0);
+                    ptx::tmem_ld_32x32b<kChunk>(taddr + c * kChunk, t);
+                    ptx::tmem_ld_wait<kChunk>(t);
+                    YAN_STAMP(l1);
+                    YAN_STAMP_ADD(in_loads, l0, l1);
+                    if (kTailChunk == 0 && c + 1 == kNumChunks) {
+                        release_buffer();
+                        if constexpr (kEarlyProbe) {
+                            const uint32_t nb = (buf + 1 == kNumTmemBufs) ? 0 : buf + 1;
+                            const uint32_t np = (buf + 1 == kNumTmemBufs) ? buf_phase ^ 1 : buf_phase;
+                            next_ready = __all_sync(0xffffffffu, ptx::mbar_test_wait(tmem_full_barriers + nb * 2 + half, np));
                         }
                     }
-                    if (kb + kScaleDepth < kb_count) {
-                        sa_ring[fill] = row_ok ? __ldg(sa_next) : 0.0f;
-                        sa_next += p.sa_ld;
-                        sb_ring[fill] = __ldg(sb_ptr + kb + kScaleDepth);
-                        if constexpr (kTwoScales) sb_hi_ring[fill] = __ldg(sb_hi_ptr + kb + kScaleDepth);
+#pragma unroll
+                    for (uint32_t j = 0; j < kChunk; j += 2)
+                        ptx::fma_f32x2(acc[c * kChunk + j], acc[c * kChunk + j + 1], t[j], t[j + 1],
+                                       group_scale((c * kChunk + j) / 16));
+                    YAN_STAMP(l2);
+                    YAN_STAMP_ADD(in_fmas, l1, l2);
+                }
+                if constexpr (kTailChunk != 0) {
+                    uint32_t t[16];
+                    ptx::tmem_ld_32x32b<16>(taddr + kNumChunks * kChunk, t);
+                    ptx::tmem_ld_wait<16>(t);
+                    release_buffer();
+                    const float sc = group_scale((kNumChunks * kChunk) / 16);
+#pragma unroll
+                    for (uint32_t j = 0; j < 16; j += 2)
+                        ptx::fma_f32x2(acc[kNumChunks * kChunk + j], acc[kNumChunks * kChunk + j + 1], t[j], t[j + 1], sc);
+                }
+                if (++buf == kNumTmemBufs) {
+                    buf = 0;
+                    buf_phase ^= 1;
+                }
+            };
+            if constexpr (L::kScaleRing) {
+#pragma unroll 1
+                for (uint32_t kb = 0; kb < kb_count; ++kb) {
+                    // the scales were copied kNumStages k-blocks ago: read them while the products are awaited
+                    const bool scales_ok = detail::bounded_wait(scale_full_barriers + slot, slot_phase, abort_flag, p, 7);
+                    const uint32_t scales = s_scales + slot * L::kScaleSlotBytes;
+                    const float sa = ptx::ld_shared_f32(scales + row_in_tile * 4u);
+                    const float scale = sa * ptx::ld_shared_f32(scales + sb_offset);
+                    float scale_hi = scale;
+                    if constexpr (kTwoScales) scale_hi = sa * ptx::ld_shared_f32(scales + sb_offset + 4u);
+                    if (++slot == L::kNumScaleSlots) {
+                        slot = 0;
+                        slot_phase ^= 1;
                     }
                     YAN_STAMP(w0);
                     const bool ok = (kEarlyProbe && next_ready) ||
                                     detail::bounded_wait(tmem_full_barriers + buf * 2 + half, buf_phase, abort_flag, p, 4);
-                    if (!__all_sync(0xffffffffu, ok)) {
+                    if (!__all_sync(0xffffffffu, ok && scales_ok)) {
                         alive = false;
-                        continue;
+                        break;
                     }
                     YAN_STAMP(w1);
                     YAN_STAMP_ADD(waited_tmem_full, w0, w1);
-                    YAN_STAMP_ADD(promoted, 0, 1);
-                    ptx::tcgen05_fence_after_thread_sync();
-                    const uint32_t taddr = tmem_lane_base + buf * BLOCK_N;
-
-                    // The TMEM buffer is handed back as soon as the last columns have landed, before their FMAs.
-                    // Nothing is scheduled between a tcgen05.ld and its wait: FMAs issued while a load is
-                    // outstanding were measured ~10x slower than after it (the load does not overlap with the
-                    // issuing warp's own arithmetic), so the overlap has to come from the sibling warp.
-                    auto release_buffer = [&]() {
-                        ptx::tcgen05_fence_before_thread_sync();
-                        __syncwarp();
-                        if (lane_idx == 0) ptx::mbar_arrive(tmem_empty_barriers + buf * 2 + half);
-                    };
-                    auto group_scale = [&](uint32_t group16) { return (kTwoScales && group16 >= hi_from) ? scale_hi : scale; };
+                    promote(scale, scale_hi);
+                }
+            } else {
+                // kShiftRing: one copy of the loop body, the ring of scales moved down one slot per k-block (a few register
+                // moves); otherwise the body is unrolled once per ring slot and every copy uses its own slot.
+                for (uint32_t kb0 = 0; kb0 < kb_count && alive; kb0 += kLoopUnroll) {
+#pragma unroll(kLoopUnroll)
+                    for (uint32_t i = 0; i < kLoopUnroll; ++i) {
+                        const uint32_t kb = kb0 + i;
+                        if (!alive || (kLoopUnroll > 1 && kb >= kb_count)) continue;
+                        const uint32_t use = kShiftRing ? 0 : i, fill = kShiftRing ? kScaleDepth - 1 : i;
+                        const float scale = sa_ring[use] * sb_ring[use];
+                        float scale_hi = scale;
+                        if constexpr (kTwoScales) scale_hi = sa_ring[use] * sb_hi_ring[use];
+                        if constexpr (kShiftRing) {
 #pragma unroll
-                    for (uint32_t c = 0; c < kNumChunks; ++c) {
-                        uint32_t t[kChunk];
-                        YAN_STAMP(l0);
-                        ptx::tmem_ld_32x32b<kChunk>(taddr + c * kChunk, t);
-                        ptx::tmem_ld_wait<kChunk>(t);
-                        YAN_STAMP(l1);
-                        YAN_STAMP_ADD(in_loads, l0, l1);
-                        if (kTailChunk == 0 && c + 1 == kNumChunks) {
-                            release_buffer();
-                            if constexpr (kEarlyProbe) {
-                                const uint32_t nb = (buf + 1 == kNumTmemBufs) ? 0 : buf + 1;
-                                const uint32_t np = (buf + 1 == kNumTmemBufs) ? buf_phase ^ 1 : buf_phase;
-                                next_ready = __all_sync(0xffffffffu, ptx::mbar_test_wait(tmem_full_barriers + nb * 2 + half, np));
+                            for (uint32_t r = 0; r + 1 < kScaleDepth; ++r) {
+                                sa_ring[r] = sa_ring[r + 1];
+                                sb_ring[r] = sb_ring[r + 1];
+                                if constexpr (kTwoScales) sb_hi_ring[r] = sb_hi_ring[r + 1];
                             }
                         }
-#pragma unroll
-                        for (uint32_t j = 0; j < kChunk; j += 2)
-                            ptx::fma_f32x2(acc[c * kChunk + j], acc[c * kChunk + j + 1], t[j], t[j + 1],
-                                           group_scale((c * kChunk + j) / 16));
-                        YAN_STAMP(l2);
-                        YAN_STAMP_ADD(in_fmas, l1, l2);
-                    }
-                    if constexpr (kTailChunk != 0) {
-                        uint32_t t[16];
-                        ptx::tmem_ld_32x32b<16>(taddr + kNumChunks * kChunk, t);
-                        ptx::tmem_ld_wait<16>(t);
-                        release_buffer();
-                        const float sc = group_scale((kNumChunks * kChunk) / 16);
-#pragma unroll
-                        for (uint32_t j = 0; j < 16; j += 2)
-                            ptx::fma_f32x2(acc[kNumChunks * kChunk + j], acc[kNumChunks * kChunk + j + 1], t[j], t[j + 1], sc);
-                    }
-                    if (++buf == kNumTmemBufs) {
-                        buf = 0;
-                        buf_phase ^= 1;
+                        if (kb + kScaleDepth < kb_count) {
+                            sa_ring[fill] = row_ok ? __ldg(sa_next) : 0.0f;
+                            sa_next += p.sa_ld;
+                            sb_ring[fill] = __ldg(sb_ptr + kb + kScaleDepth);
+                            if constexpr (kTwoScales) sb_hi_ring[fill] = __ldg(sb_hi_ptr + kb + kScaleDepth);
+                        }
+                        YAN_STAMP(w0);
+                        const bool ok = (kEarlyProbe && next_ready) ||
+                                        detail::bounded_wait(tmem_full_barriers + buf * 2 + half, buf_phase, abort_flag, p, 4);
+                        if (!__all_sync(0xffffffffu, ok)) {
+                            alive = false;
+                            continue;
+                        }
+                        YAN_STAMP(w1);
+                        YAN_STAMP_ADD(waited_tmem_full, w0, w1);
+                        promote(scale, scale_hi);
                     }
                 }
             }
@@ -1000,7 +1088,7 @@ inline int check_and_fill(const GemmArgs& a, GemmType type, uint32_t out_bytes, 
 
 template <uint32_t BLOCK_N, uint32_t kNumStages, GemmType kGemmType, typename out_t>
 struct GemmLauncher {
-    using L = GemmOutputLayout<BLOCK_N, kNumStages, sizeof(out_t) == 4>;
+    using L = GemmOutputLayout<BLOCK_N, kNumStages, false>;
     static constexpr uint32_t kSmemSize = L::kSmemSize;
 
     static int launch(const GemmArgs& a, cudaStream_t stream) {
@@ -1103,6 +1191,23 @@ struct GemmLauncher {
                 return kOk;
             }
         }
+        // fp32 output on 256-wide tiles: 128-byte box rows halve the passes of the epilogue but leave no room for the ring of
+        // scales; the epilogue is what counts while K is short (M=4096 N=8192: K=3584 143.1 us with wide boxes, 145.3 with the
+        // ring; K=14336 525 and 502).
+        if constexpr (kGemmType == GemmType::Normal && sizeof(out_t) == 4 && BLOCK_N == 256) {
+            using Wide = GemmSmemLayout<BLOCK_N, kNumStages, true>;
+            if constexpr (Wide::kStoreBytes != 0 && !Wide::kScaleRing) {
+                if (a.k < YAN_WIDE_F32_MAX_K && static_cast<int>(Wide::kSmemSize) <= max_smem) {
+                    auto wide_kernel = fp8_gemm_kernel<BLOCK_N, kNumStages, GemmType::Normal, out_t, false, false, false, true>;
+                    if (cudaFuncSetAttribute(wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Wide::kSmemSize) != cudaSuccess) {
+                        cudaGetLastError();
+                        return kSmemTooLarge;
+                    }
+                    wide_kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), Wide::kSmemSize, stream>>>(p, map_a, map_b);
+                    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+                }
+            }
+        }
         kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), kSmemSize, stream>>>(p, map_a, map_b);
         return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
     }
@@ -1111,7 +1216,7 @@ struct GemmLauncher {
 // Few tiles, long K: one cluster of `slices` CTAs per tile (the kClusterK instance).
 template <uint32_t BLOCK_N, uint32_t kNumStages, typename out_t>
 struct GemmClusterKLauncher {
-    using L = GemmOutputLayout<BLOCK_N, kNumStages, sizeof(out_t) == 4>;
+    using L = GemmOutputLayout<BLOCK_N, kNumStages, false>;
 
     static int launch(const GemmArgs& a, uint32_t slices, cudaStream_t stream) {
         constexpr uint32_t kRowsBytes = kBlockM * (BLOCK_N + 4) * 4;  // the exchanged rows

@@ -12,7 +12,7 @@
 namespace yan {
 
 // --- CTA role layout -------------------------------------------------------------------------
-// warp 0      : TMA producer (one elected lane)
+// warp 0      : producer: TMA (one elected lane) and the asynchronous copies of the scales (all lanes)
 // warp 1      : MMA issuer   (one elected lane)
 // warp 2      : TMEM allocator / deallocator
 // warp 3      : spare (keeps the first four warps a full warpgroup for setmaxnreg)
