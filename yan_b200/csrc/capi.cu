@@ -87,17 +87,19 @@ inline void set_rc(int* rc, int v) {
     if (rc != nullptr) *rc = v;
 }
 
-// Picks BLOCK_N by a wave model: cost = waves * (time of one tile relative to a 256-wide one).  The relative tile
-// times are measured (time per wave on M = 8192, N = 26880, K = 4096, a shape every width divides): the promotion of a
-// k-block has a large fixed part, so a narrower tile is far from proportionally cheaper, and the widths without
-// shared-memory room for the staged epilogue (224, 192, 160, 96) or with a second B scale and a 16-column tail chunk
-// pay for that.  Large problems therefore get 256; narrower tiles win when they fill the machine better.
-// `cost`, when given, receives the winner's cost.
-int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* cost_out = nullptr) {
-    static const struct { int bn; double tile_cost; } candidates[8] = {
-        {256, 1.000}, {224, 1.08}, {192, 0.84}, {160, 0.82}, {128, 0.67}, {96, 0.72}, {64, 0.57}, {32, 0.50}};
+// Picks BLOCK_N by a wave model: time = start + waves * (k-blocks * per_kb + epilogue), in us, fitted to graph timings on B200
+// (37 tile rows, 1 to 5 full waves, K = 512 to 6144; within 6 %; 224 and 160 made slower, as they are in long runs).  A narrower
+// tile is far from proportionally cheaper: the promotion of a k-block has a large fixed part, the widths without shared-memory
+// room for the staged epilogue (224, 160, 96) or with a second B scale and a 16-column tail chunk pay for that; but with four
+// accumulators instead of two its epilogue hides better.  Large problems therefore get 256; narrower tiles win when they fill
+// the machine better or K is short.
+// `time_out`, when given, receives the winner's time.
+int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* time_out = nullptr) {
+    static const struct { int bn; double start, per_kb, epilogue; } candidates[8] = {
+        {256, 3.15, 0.426, 2.02}, {224, 4.19, 0.470, 3.54}, {192, 3.14, 0.351, 1.66}, {160, 3.28, 0.330, 2.60},
+        {128, 3.76, 0.254, 0.89}, {96, 3.80, 0.257, 1.49},  {64, 3.44, 0.215, 0.48},  {32, 3.29, 0.209, 0.41}};
     int best = 256;
-    double best_cost = -1.0;
+    double best_time = -1.0;
     for (const auto& c : candidates) {
         if (c.bn > 32 && n < c.bn) continue;
         const long tiles = static_cast<long>((m + 127) / 128) * ((n + c.bn - 1) / c.bn);
@@ -106,30 +108,28 @@ int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* 
         if (can_cut_tail && (c.bn == 256 || c.bn == 128 || c.bn == 64) &&
             yan::choose_tail_slices(static_cast<uint32_t>(tiles), static_cast<uint32_t>(num_sms), static_cast<uint32_t>(k / 128)) != 0)
             waves = static_cast<double>(tiles / num_sms) + 0.35;
-        const double cost = waves * c.tile_cost;
-        if (best_cost < 0.0 || cost < best_cost * 0.98) {  // a narrower tile must win by 2 % to be taken
-            best_cost = cost;
+        const double time = c.start + waves * (k / 128 * c.per_kb + c.epilogue);
+        if (best_time < 0.0 || time < best_time * 0.98) {  // a narrower tile must win by 2 % to be taken
+            best_time = time;
             best = c.bn;
         }
     }
-    if (cost_out != nullptr) *cost_out = best_cost;
+    if (time_out != nullptr) *time_out = best_time;
     return best;
 }
 
-// CTAs per tile when K is cut over clusters (64-wide tiles), or 0 to leave tiles whole.  Times in us, fitted to graph
-// timings on B200 over weights from HBM: a launch of whole tiles takes about 3.4 + 0.41 * waves * tile cost per k-block
-// (M=209 N=480 K=12928: 24.5, M=128 N=2048 K=7168: 15.8, M=256 N=1024 K=4096: 10.0, M=130 N=256 K=512: 4.2), a clustered one
-// about 5.9 + 0.235 per k-block of a slice (12.0, 10.0, 7.9 and 6.0 with four slices).  Clusters of four stop fitting the
-// GPU at once between 132 and 136 CTAs (M=128 K=7168: N=2112 10.1, N=2176 17.6), clusters of two at 148.
-int choose_cluster_slices(int m, int n, int k, int num_sms, double whole_tiles_cost) {
+// CTAs per tile when K is cut over clusters (64-wide tiles), or 0 to leave tiles whole.  `whole` is the time of whole tiles by
+// the model above; a clustered launch takes about 6.0 us + 0.215 per k-block of a slice (M=209 N=480 K=12928, four slices: 11.7
+// against 24.5; M=128 N=2048 K=7168 9.8 against 15.8; M=600 N=512 K=4096, two slices: 8.6 against 10.0).  Clusters of four stop
+// fitting the GPU at once between 132 and 136 CTAs (M=128 K=7168: N=2112 10.1, N=2176 17.6), clusters of two at 148.
+int choose_cluster_slices(int m, int n, int k, int num_sms, double whole) {
     const long tiles = static_cast<long>((m + 127) / 128) * ((n + 63) / 64);
     const int kb = k / 128;
-    const double whole = 3.4 + 0.41 * whole_tiles_cost * kb;
     int best = 0;
     double best_time = 0.97 * whole;
     for (int slices = 2; slices <= 4; slices *= 2) {
         if (tiles * slices > (slices == 2 ? num_sms : num_sms * 7 / 8) || kb < 2 * slices) continue;
-        const double t = 5.9 + 0.235 * ((kb + slices - 1) / slices);
+        const double t = 6.0 + 0.215 * ((kb + slices - 1) / slices);
         if (t < best_time) best = slices, best_time = t;
     }
     return best;
@@ -140,12 +140,12 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
     if (a.m == 0 || a.n == 0 || a.k == 0) return yan::kBadArgument;
     if (a.num_sms <= 0) return yan::kBadArgument;
     const bool want_auto = (block_n == 0);
-    double whole_tiles_cost = 0.0;
+    double whole_tiles_time = 0.0;
     if (block_n == 0) {
         const int rows = (type == yan::GemmType::GroupedMasked) ? static_cast<int>(a.m * a.num_groups) : static_cast<int>(a.m);
         block_n = choose_block_n(rows, static_cast<int>(a.n), static_cast<int>(a.k), a.num_sms,
                                  type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16 && a.tail_workspace != nullptr,
-                                 &whole_tiles_cost);
+                                 &whole_tiles_time);
     }
     a.status = status_word_of_current_device();
     a.timeout_ns = g_timeout_ns;
@@ -178,7 +178,7 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
     }
     if (type == yan::GemmType::Normal && want_auto && out_kind != yan::OutKind::E4M3 && a.scatter_world == 0) {
         const int slices = choose_cluster_slices(static_cast<int>(a.m), static_cast<int>(a.n), static_cast<int>(a.k), a.num_sms,
-                                                 whole_tiles_cost);
+                                                 whole_tiles_time);
         if (slices != 0) return yan::launch_gemm_cluster_k(static_cast<uint32_t>(slices), out_kind, a, s);
     }
     // Groups of at most 128 rows: the kernel that follows masked_m, unless 32-wide tiles of the general one fit the GPU at once

@@ -57,28 +57,32 @@ _DEFAULT_STAGES = {32: 8, 64: 8, 96: 8, 128: 6, 160: 6, 192: 5, 224: 5, 256: 4}
 
 def get_smem_size(block_n: int, num_stages: int) -> int:
     """Dynamic shared memory of one CTA: stages x (A 128x128 + B BLOCK_Nx128 e4m3) + the output staging boxes
-    (8 x 2 KB, where the ring leaves room) + mbarriers + 1024 bytes of alignment slack (GemmSmemLayout in
-    include/gemm/fp8_gemm.cuh)."""
+    (8 x 2 KB, where the ring leaves room) + the ring of scales (where that leaves room) + mbarriers + 1024 bytes of
+    alignment slack (GemmSmemLayout in include/gemm/fp8_gemm.cuh)."""
     num_tmem_bufs = 2 if block_n > 128 else 4
     ring = num_stages * (128 * 128 + block_n * 128)
     store = 8 * 2048 if ring + 8 * 2048 + 2048 <= 232448 else 0
-    return ring + store + (2 * num_stages + 4 * num_tmem_bufs) * 8 + 8 + 1024
+    slots = num_stages + num_tmem_bufs + 1
+    if ring + store + slots * 528 + 2048 > 232448:
+        slots = 0
+    return ring + store + slots * 528 + (2 * num_stages + 4 * num_tmem_bufs + slots) * 8 + 8 + 1024
 
 
-# time of one tile relative to a 256-wide one (measured; see choose_block_n in csrc/capi.cu)
-_TILE_COST = {256: 1.000, 224: 1.08, 192: 0.84, 160: 0.82, 128: 0.67, 96: 0.72, 64: 0.57, 32: 0.50}
+# start, time per k-block and epilogue of a wave of tiles, in us (measured; see choose_block_n in csrc/capi.cu)
+_TILE_TIMES = {256: (3.15, 0.426, 2.02), 224: (4.19, 0.470, 3.54), 192: (3.14, 0.351, 1.66), 160: (3.28, 0.330, 2.60),
+               128: (3.76, 0.254, 0.89), 96: (3.80, 0.257, 1.49), 64: (3.44, 0.215, 0.48), 32: (3.29, 0.209, 0.41)}
 
 
 def get_best_configs(m: int, n: int, k: int, num_sms: int) -> Tuple[int, int, int]:
     """(BLOCK_N, NUM_STAGES, smem_size) by the same wave model as the C library's default."""
-    best, best_cost = 256, None
-    for bn, tile_cost in _TILE_COST.items():
+    best, best_time = 256, None
+    for bn, (start, per_kb, epilogue) in _TILE_TIMES.items():
         if bn > 32 and n < bn:
             continue
         waves = ceil_div(ceil_div(m, 128) * ceil_div(n, bn), num_sms)
-        cost = waves * tile_cost
-        if best_cost is None or cost < best_cost * 0.98:
-            best, best_cost = bn, cost
+        t = start + waves * (k // 128 * per_kb + epilogue)
+        if best_time is None or t < best_time * 0.98:
+            best, best_time = bn, t
     stages = _DEFAULT_STAGES[best]
     return best, stages, get_smem_size(best, stages)
 
