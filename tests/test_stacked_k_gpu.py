@@ -85,3 +85,29 @@ def test_output_that_only_the_streaming_kernels_take(cuda_lib):
     torch.cuda.synchronize()
     assert ref.rel_frobenius(out[:, :256].cpu(), d_ref) <= 1e-3
     assert call(256, 384) == 1 and call(240, 512) == 1
+
+
+def test_clusters_of_several_streams_share_the_gpu(cuda_lib):
+    """Kernels whose CTAs wait for one another inside a cluster, side by side on three streams: every one gives its tensor
+    memory back before it waits, so they finish, with the results they have alone."""
+    import yan_b200
+    # clusters of two and four of this kernel, the pair kernel, the general kernel's clusters
+    cases = [(16, 2048, 4096, 0), (32, 4096, 2048, 0), (16, 1024, 8192, 0), (16, 4096, 2048, 1), (128, 2048, 7168, 0)]
+    calls, want = [], []
+    for m, n, k, block_n in cases:
+        a, b = ref.make_inputs(m, n, k, seed=m + n + block_n)
+        lhs, rhs = yan_b200.per_token_cast_to_fp8(a.cuda()), yan_b200.per_block_cast_to_fp8(b.cuda())
+        calls.append((lhs, rhs, block_n))
+        want.append(torch.empty(m, n, dtype=torch.bfloat16, device="cuda"))
+        yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, want[-1], block_n=block_n)
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    outs = [[torch.empty_like(w) for w in want] for _ in streams]
+    for i in range(60):
+        for j, stream in enumerate(streams):
+            lhs, rhs, block_n = calls[(i + 2 * j) % len(calls)]
+            with torch.cuda.stream(stream):
+                yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, outs[j][(i + 2 * j) % len(calls)], block_n=block_n)
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    assert all(torch.equal(o, w) for out in outs for o, w in zip(out, want))

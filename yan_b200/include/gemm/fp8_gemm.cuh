@@ -31,9 +31,6 @@
 
 namespace yan {
 
-constexpr uint32_t kBlockM = 128;
-constexpr uint32_t kBlockK = 128;
-
 // Device-side view of one launch.
 struct GemmParams {
     const float* scales_a;      // [K/128][sa_ld], element (kb, row) at kb * sa_ld + row
@@ -658,7 +655,16 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
 #endif
         }
         __syncwarp();
-        if constexpr (kClusterK) {  // the two meetings of the exchange below
+        if constexpr (kClusterK) {
+            // Tensor memory goes back before this CTA waits for the others of its cluster (see fp8_gemm_stacked_k.cuh): the
+            // promotion warps have read the last accumulator, and warp 1 issues no more products.
+            if (warp_idx == 1) ptx::named_barrier_arrive(2, kNumMathWarps * 32 + 64);
+            if (warp_idx == 2) {
+                ptx::named_barrier_sync(2, kNumMathWarps * 32 + 64);
+                ptx::tcgen05_fence_after_thread_sync();
+                ptx::tmem_dealloc(tmem_base, L::kTmemCols);
+            }
+            // the two meetings of the exchange below
             ptx::cluster_wait();
             if constexpr (detail::kExchangeInRing<BLOCK_N>) ptx::cluster_arrive(), ptx::cluster_wait();
             ptx::cluster_arrive(), ptx::cluster_wait();
@@ -833,6 +839,8 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             }
             YAN_STAMP(s0);
             if constexpr (kClusterK) {
+                ptx::tcgen05_fence_before_thread_sync();
+                ptx::named_barrier_arrive(2, kNumMathWarps * 32 + 64);
                 detail::exchange_and_store<out_t, BLOCK_N>(p, ptx::smem_u32(smem) + kExchangeOffset, tail_slice, m_block_idx * kBlockM,
                                                            n_block_idx * BLOCK_N, row_in_tile, col0, threadIdx.x - kNumControlThreads,
                                                            alive && *abort_flag == 0, acc);
@@ -938,7 +946,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     }
     ptx::tcgen05_fence_before_thread_sync();
     __syncthreads();
-    if (warp_idx == 2) {
+    if (warp_idx == 2 && !kClusterK) {
         ptx::tcgen05_fence_after_thread_sync();
         ptx::tmem_dealloc(tmem_base, L::kTmemCols);
     }

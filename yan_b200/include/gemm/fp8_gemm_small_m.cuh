@@ -177,12 +177,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
             }
         }
         ptx::tcgen05_fence_before_thread_sync();
+        ptx::named_barrier_arrive(2, 160);
     }
 
     // Both CTAs of the pair are past their MMAs and TMEM reads: the weight tiles of CTA 0 are dead and become
     // the landing area for CTA 1's partial sums, one padded row of M_PAD floats per weight row (= per thread), so that
     // both sides move 16 bytes per instruction.
     ptx::cluster_arrive();
+    if (warp_idx == 4) {
+        // Tensor memory goes back before this CTA waits for the other one (see fp8_gemm_stacked_k.cuh).
+        ptx::named_barrier_sync(2, 160);
+        ptx::tcgen05_fence_after_thread_sync();
+        ptx::tmem_dealloc(tmem_base, tmem_cols);
+    }
     ptx::cluster_wait();
     constexpr uint32_t kRowBytes = small_m_exchange_row_bytes(M_PAD);
     const uint32_t n_in_tile = warp_idx * 32 + lane_idx;
@@ -221,13 +228,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
             for (uint32_t m = 0; m < M_PAD; ++m)
                 if (m < p.shape_m) out[static_cast<size_t>(m) * p.ldd + n_in_tile] = __float2bfloat16_rn(acc[m]);
         }
-    }
-
-    ptx::tcgen05_fence_before_thread_sync();
-    __syncthreads();
-    if (warp_idx == 4) {
-        ptx::tcgen05_fence_after_thread_sync();
-        ptx::tmem_dealloc(tmem_base, tmem_cols);
     }
 #endif
 }

@@ -24,6 +24,9 @@
 // kSlots step slots of shared memory and kTmemSlots of tensor memory rotate: the loads of step s + kSlots go out as soon as
 // the MMAs of step s are complete, the MMAs of step s + kTmemSlots wait until the promotion warps have read the accumulator
 // of step s.
+// Tensor memory goes back before a CTA waits for the others of its cluster: two CTAs of different clusters on an SM (another
+// stream's launch, or this launch's next cluster) may need more columns than there are, and one that kept its own while it
+// waited for a CTA that in turn waits for columns elsewhere would close a circle of waits that nothing bounds.
 // Weights are loaded before griddepcontrol.wait (parameters), activations and their scales after it; waits are bounded.
 
 #include <cstdint>
@@ -32,35 +35,9 @@
 #include <cuda_runtime.h>
 
 #include "fp8_gemm_small_m.cuh"
+#include "stacked_k_plan.h"
 
 namespace yan {
-
-constexpr uint32_t kStackedThreads = 192;
-
-struct StackedSmem {
-    uint32_t off_w, off_x, off_scales, off_exchange, off_barriers, off_tmem_slot, off_abort, total;
-};
-
-__host__ __device__ inline StackedSmem stacked_k_smem_layout(uint32_t m_pad, uint32_t stack, uint32_t steps, uint32_t slots,
-                                                             uint32_t cluster) {
-    StackedSmem s;
-    const uint32_t used = steps < slots ? steps : slots;
-    const uint32_t sums = 128u * m_pad * 4u;                          // [stack][m_pad][128 / stack] floats
-    const uint32_t rings = used * (16384u + stack * m_pad * 128u);
-    s.off_w = 0;                                                      // slots x [128 x 128 B]; at the end the sums
-    s.off_x = s.off_w + used * 16384u;                                // slots x [stack*m_pad x 128 B]
-    s.off_scales = s.off_w + (rings > sums ? rings : sums);           // [stack][steps][m_pad] floats: sA * sB
-    s.off_exchange = s.off_scales + stack * steps * m_pad * 4u;       // [cluster - 1][m_pad][128 / stack] floats
-    s.off_barriers = align_up(s.off_exchange + (cluster - 1) * m_pad * (128u / stack) * 4u, 8u);
-    s.off_tmem_slot = s.off_barriers + 4 * 8u * 8u;  // full, empty, done, tmem_empty: at most 8 of each
-    s.off_abort = s.off_tmem_slot + 4;
-    s.total = s.off_abort + 4 + 1024;
-    return s;
-}
-
-__host__ __device__ inline uint32_t stacked_k_steps(uint32_t k, uint32_t stack, uint32_t cluster) {
-    return ceil_div(k / kBlockK, stack * cluster);
-}
 
 // What may still be running when a CTA of this launch starts (every launch has programmatic stream serialization).
 // Tensor memory is never taken while a kernel that might itself still have to take some could be waiting for this one's:
@@ -73,7 +50,7 @@ enum StackedOrder : uint32_t {
                               // once, tensor memory is taken after the wait
 };
 
-template <uint32_t M_PAD, uint32_t kStack, uint32_t kSlots, uint32_t kTmemSlots>
+template <uint32_t M_PAD, uint32_t kStack, uint32_t kSlots, uint32_t kTmemSlots = stacked_k_tmem_slots(kSlots)>
 __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <= 256 ? 2 : 1)
     fp8_gemm_stacked_k_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tensor_map_w,
                               const __grid_constant__ CUtensorMap tensor_map_x, const uint32_t cluster,
@@ -83,11 +60,11 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     constexpr uint32_t kMmaN = kStack * M_PAD;
     constexpr uint32_t kWarpsPerPart = 4 / kStack;  // promotion warps (of 32 weight rows each) that share a k-part
     constexpr uint32_t kStepBytes = 16384u + kMmaN * 128u;
-    constexpr uint32_t kTmemCols = kTmemSlots * kMmaN;
+    constexpr uint32_t kTmemCols = stacked_k_tmem_cols(M_PAD, kStack, kSlots);
     static_assert(M_PAD == 16 || M_PAD == 32 || M_PAD == 64, "activation rows are padded to 16, 32 or 64");
     static_assert(kStack == 1 || kStack == 2 || kStack == 4, "whole lane quarters of the 128-row operand");
     static_assert(kSlots <= 8 && kTmemSlots <= 8 && kSlots * kStack <= 32, "one producer lane per (slot, k-part)");
-    static_assert(kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "a power of two of at most 512 columns");
+    static_assert(kTmemCols == kTmemSlots * kMmaN && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "a power of two of at most 512 columns");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
 
@@ -200,6 +177,10 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
             }
         }
         __syncwarp();
+        // the promotion warps have read the last accumulator
+        ptx::named_barrier_sync(2, 160);
+        ptx::tcgen05_fence_after_thread_sync();
+        ptx::tmem_dealloc(tmem_base, kTmemCols);
     }
 
     // Promotion warps: TMEM lane 32 * warp + lane = (k-part q, weight row n0 + r)
@@ -248,6 +229,8 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
                 }
             }
         }
+        ptx::tcgen05_fence_before_thread_sync();
+        ptx::named_barrier_arrive(2, 160);
         // The k-parts of a weight row sit in different warps: exchange through shared memory, [q][m][r], in the weight slots,
         // which are dead once every warp has seen the last step's MMAs complete.
         ptx::named_barrier_sync(1, 128);
@@ -286,20 +269,13 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
                 if (m0 + j < p.shape_m) out[static_cast<size_t>(m0 + j) * p.ldd] = __float2bfloat16_rn(v[j]);
         }
     }
-
-    ptx::tcgen05_fence_before_thread_sync();
-    __syncthreads();
-    if (warp_idx == 5) {
-        ptx::tcgen05_fence_after_thread_sync();
-        ptx::tmem_dealloc(tmem_base, kTmemCols);
-    }
 #endif
 }
 
-template <uint32_t M_PAD, uint32_t kStack, uint32_t kSlots, uint32_t kTmemSlots>
+template <uint32_t M_PAD, uint32_t kStack, uint32_t kSlots>
 inline int launch_stacked_k_instance(const GemmParams& p, const CUtensorMap& map_w, const CUtensorMap& map_x,
                                      uint32_t cluster, cudaStream_t stream, StackedOrder order) {
-    auto kernel = fp8_gemm_stacked_k_kernel<M_PAD, kStack, kSlots, kTmemSlots>;
+    auto kernel = fp8_gemm_stacked_k_kernel<M_PAD, kStack, kSlots>;
     const uint32_t smem_bytes = stacked_k_smem_layout(M_PAD, kStack, stacked_k_steps(p.shape_k, kStack, cluster), kSlots, cluster).total;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) {
         cudaGetLastError();
@@ -331,50 +307,6 @@ inline int launch_stacked_k_instance(const GemmParams& p, const CUtensorMap& map
         return kLaunchFailed;
     }
     return kOk;
-}
-
-// What a caller may ask for by name (block_n = 2).
-inline bool stacked_k_supported(uint32_t m, uint32_t n, uint32_t k) {
-    return m >= 1 && m <= 32 && n % 32 == 0 && k % 512 == 0 && k / 512 <= 32;
-}
-
-struct StackedConfig {
-    uint32_t m_pad, stack, slots, cluster;
-};
-
-// Which CTAs share the work (B200, graph of launches over weights that come from HBM, quantizer included, in us):
-//   * 32 weight rows per CTA (stack 4) for M <= 16, 64 (stack 2) above: each CTA re-reads all activations.
-//   * up to one CTA per SM: as many slots as tensor memory has (M=16 N=4096 K=7168 with 8 slots 11.0, with 4 12.4;
-//     M=64 N=7168 K=4096 with 6 operand slots 13.4, with 4 14.8).  More row groups than SMs: 4 slots, two CTAs per SM
-//     (M=16 N=7168 K=2048: 7.0; with 8 slots, one CTA per SM and two waves of them: 8.0).
-//   * a cluster along K where row groups leave SMs idle, as long as it saves every CTA four steps: the exchange costs about
-//     0.45 us and a step 0.15 - 0.3 (M=16 N=2048 K=7168: 9.2 / 8.6 / 9.8 for clusters of 1 / 2 / 4; M=8 N=528 K=13440:
-//     14.2 / 9.6 / 7.4 / 9.2 for 1 / 2 / 4 / 8; M=16 N=1024 K=1024: 4.0 / 4.5 for 1 / 2).
-inline StackedConfig choose_stacked_config(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t max_smem) {
-    StackedConfig c;
-    c.m_pad = m <= 16 ? 16 : m <= 32 ? 32 : 64;
-    c.stack = c.m_pad == 16 ? 4 : 2;
-    const uint32_t groups = ceil_div(n, 128u / c.stack);
-    c.cluster = 1;
-    while (c.cluster < 4 && groups * c.cluster * 2 <= num_sms &&
-           stacked_k_steps(k, c.stack, c.cluster) >= stacked_k_steps(k, c.stack, c.cluster * 2) + 4)
-        c.cluster *= 2;
-    c.slots = groups > num_sms && c.m_pad != 64 ? 4 : c.m_pad == 64 ? 6 : 8;
-    // the scale table grows with K, the exchange with M and the cluster: where they leave no room, four slots
-    if (stacked_k_smem_layout(c.m_pad, c.stack, stacked_k_steps(k, c.stack, c.cluster), c.slots, c.cluster).total > max_smem) c.slots = 4;
-    return c;
-}
-
-// True where this kernel is the default: while all CTAs are resident at once (M=32 N=16384 K=2048 10.9 us against 18.4 with
-// the pair kernel, but N=28672 K=1024 14.4 against 12.8 with 256-wide tiles of the general one; M=64 N=9216 K=2048 9.8
-// against 12.4, but N=14336 K=1024 15.6 against 9.7), and for M <= 16, where several waves of CTAs hold up against the
-// general kernel unless K is long too (N=28672: K=4096 28.0 against 31.0, K=8192 49.1 against 49.0, K=18432 104 against 92).
-inline bool stacked_k_preferred(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t max_smem) {
-    if (m > 64 || n % 16 != 0 || k % kBlockK != 0) return false;
-    const StackedConfig c = choose_stacked_config(m, n, k, num_sms, max_smem);
-    const uint32_t groups = ceil_div(n, 128u / c.stack), steps = stacked_k_steps(k, c.stack, c.cluster);
-    if (groups > num_sms * (c.m_pad == 64 ? 1 : 2) && (m > 16 || steps > 16)) return false;
-    return stacked_k_smem_layout(c.m_pad, c.stack, steps, c.slots, c.cluster).total <= max_smem;
 }
 
 // Host launcher.  Arguments as GemmLauncher::launch (Normal GEMM, bf16 output).
@@ -410,15 +342,15 @@ inline int launch_fp8_gemm_stacked_k(const GemmArgs& a, cudaStream_t stream, Sta
     p.status = a.status;
     p.timeout_ns = a.timeout_ns;
     if (c.m_pad == 16) {
-        if (c.slots == 8) return launch_stacked_k_instance<16, 4, 8, 8>(p, map_w, map_x, c.cluster, stream, order);
-        return launch_stacked_k_instance<16, 4, 4, 4>(p, map_w, map_x, c.cluster, stream, order);
+        if (c.slots == 8) return launch_stacked_k_instance<16, 4, 8>(p, map_w, map_x, c.cluster, stream, order);
+        return launch_stacked_k_instance<16, 4, 4>(p, map_w, map_x, c.cluster, stream, order);
     }
     if (c.m_pad == 32) {
-        if (c.slots == 8) return launch_stacked_k_instance<32, 2, 8, 8>(p, map_w, map_x, c.cluster, stream, order);
-        return launch_stacked_k_instance<32, 2, 4, 4>(p, map_w, map_x, c.cluster, stream, order);
+        if (c.slots == 8) return launch_stacked_k_instance<32, 2, 8>(p, map_w, map_x, c.cluster, stream, order);
+        return launch_stacked_k_instance<32, 2, 4>(p, map_w, map_x, c.cluster, stream, order);
     }
-    if (c.slots == 4) return launch_stacked_k_instance<64, 2, 4, 4>(p, map_w, map_x, c.cluster, stream, order);
-    return launch_stacked_k_instance<64, 2, 6, 4>(p, map_w, map_x, c.cluster, stream, order);
+    if (c.slots == 4) return launch_stacked_k_instance<64, 2, 4>(p, map_w, map_x, c.cluster, stream, order);
+    return launch_stacked_k_instance<64, 2, 6>(p, map_w, map_x, c.cluster, stream, order);
 }
 
 }  // namespace yan

@@ -330,6 +330,11 @@ __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t count) 
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 
+// The non-blocking half: this warp counts towards `count`, the warps that bar.sync on the same barrier wait for it.
+__device__ __forceinline__ void named_barrier_arrive(uint32_t id, uint32_t count) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // register reallocation between warpgroups (same mechanism the reference uses at
 // fp8_gemm.cuh:171-181 through cutlass::arch::warpgroup_reg_alloc/dealloc)

@@ -6,6 +6,10 @@
 
 namespace yan {
 
+// The tile sides that every GEMM kernel here is built around.
+constexpr uint32_t kBlockM = 128;
+constexpr uint32_t kBlockK = 128;
+
 template <typename T>
 __host__ __device__ constexpr T ceil_div(T a, T b) {
     return (a + b - 1) / b;
