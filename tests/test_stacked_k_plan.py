@@ -55,3 +55,12 @@ def test_tensor_memory_of_the_ctas_that_share_an_sm(walk):
     per_sm = np.minimum(SMEM_PER_SM // (rows[:, 5] + SMEM_RESERVED), THREADS_PER_SM // threads)
     bad = rows[per_sm * rows[:, 6] > TMEM_COLS]
     assert len(bad) == 0, f"{len(bad)} configurations, e.g. (M, N, K, cluster, CTAs, smem, columns) = {bad[:3].tolist()}"
+
+
+def test_clusters_are_resident_at_once(walk):
+    """Clusters of two up to one CTA per SM; clusters of four, which not every SM can be part of, up to 132 CTAs unless two fit
+    an SM."""
+    rows, _ = walk
+    assert set(rows[:, 3]) == {2, 4} and rows[:, 4].max() <= SMS
+    one_per_sm = 2 * (rows[:, 5] + SMEM_RESERVED) > SMEM_PER_SM
+    assert rows[(rows[:, 3] == 4) & one_per_sm][:, 4].max() == 132

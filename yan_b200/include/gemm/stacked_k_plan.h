@@ -59,15 +59,22 @@ struct StackedConfig {
 //   * a cluster along K where row groups leave SMs idle, as long as it saves every CTA four steps: the exchange costs about
 //     0.45 us and a step 0.15 - 0.3 (M=16 N=2048 K=7168: 9.2 / 8.6 / 9.8 for clusters of 1 / 2 / 4; M=8 N=528 K=13440:
 //     14.2 / 9.6 / 7.4 / 9.2 for 1 / 2 / 4 / 8; M=16 N=1024 K=1024: 4.0 / 4.5 for 1 / 2).
+//   * clusters of four: as many as can be resident at once.  Where a CTA has an SM to itself that is 33 (132 CTAs: the SMs of a
+//     processing cluster are no multiple of four); the others would start when the first have ended (M=64 K=7168: N=2112 8.5,
+//     N=2176 14.1 against 10.6 with clusters of two, N=2368 14.4 against 10.7; M=32 N=2304 K=8192 12.8 against 9.3; M=16
+//     N=1184 K=16384 12.3 against 9.2).  Where two CTAs fit an SM all of them start at once (M=16 N=1184 K=8192 5.9 against 6.7).
 inline StackedConfig choose_stacked_config(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t max_smem) {
     StackedConfig c;
     c.m_pad = m <= 16 ? 16 : m <= 32 ? 32 : 64;
     c.stack = c.m_pad == 16 ? 4 : 2;
     const uint32_t groups = ceil_div(n, 128u / c.stack);
-    c.cluster = 1;
-    while (c.cluster < 4 && groups * c.cluster * 2 <= num_sms &&
-           stacked_k_steps(k, c.stack, c.cluster) >= stacked_k_steps(k, c.stack, c.cluster * 2) + 4)
-        c.cluster *= 2;
+    for (c.cluster = 1; c.cluster < 4; c.cluster *= 2) {
+        const uint32_t next = c.cluster * 2, next_steps = stacked_k_steps(k, c.stack, next);
+        if (groups * next > num_sms || stacked_k_steps(k, c.stack, c.cluster) < next_steps + 4) break;
+        const bool two_per_sm =
+            next_steps <= 4 && 2 * (stacked_k_smem_layout(c.m_pad, c.stack, next_steps, 4, next).total + 1024) <= max_smem + 1024;
+        if (next == 4 && groups * next > num_sms * 9 / 10 && !two_per_sm) break;
+    }
     const uint32_t steps = stacked_k_steps(k, c.stack, c.cluster);
     c.slots = c.m_pad == 64 ? 6 : groups > num_sms || steps <= 4 ? 4 : 8;
     // the scale table grows with K, the exchange with M and the cluster: where they leave no room, four slots
