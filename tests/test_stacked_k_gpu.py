@@ -111,3 +111,30 @@ def test_clusters_of_several_streams_share_the_gpu(cuda_lib):
     torch.cuda.synchronize()
     assert yan_b200.read_device_status() == 0
     assert all(torch.equal(o, w) for out in outs for o, w in zip(out, want))
+
+
+def test_output_that_only_the_streaming_kernels_take_beyond_their_default(cuda_lib):
+    """The same where the general kernel is the default for other outputs: M <= 16, more row groups than two per SM, long K."""
+    import ctypes
+    import yan_b200
+    from yan_b200 import _lib
+    m, n, k = 9, 9600, 8704
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    lhs = yan_b200.per_token_cast_to_fp8(torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16))
+    rhs = yan_b200.per_block_cast_to_fp8((torch.randn(n, k, generator=gen, device="cuda") * 0.02).to(torch.bfloat16))
+    out = torch.zeros(m, n + 1, dtype=torch.bfloat16, device="cuda")
+    general = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def call(n, k):
+        return _lib.call_rc("yan_b200_gemm_fp8_fp8_bf16_nt", lhs[0].data_ptr(), lhs[1].data_ptr(), rhs[0].data_ptr(),
+                            rhs[1].data_ptr(), out.data_ptr(), m, n, k, n + 1, stream, sms, 0)
+
+    assert call(n, k) == 0
+    yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, general, block_n=32)
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    # both kernels sum in fp32, in another order: bf16 results differ by one rounding of few values
+    assert ref.rel_frobenius(out[:, :n].cpu(), general.cpu()) <= 1e-3 and not out[:, n].any()
+    assert call(n, k - 128) == 1 and call(n - 16, k) == 1

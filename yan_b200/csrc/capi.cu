@@ -175,6 +175,8 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
             if (!small_m_ok) return yan::kBadArgument;
             return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || after_own_quantizer);
         }
+        // what the general kernel is faster at, with an output that it does not take
+        if (want_auto && !general_ok && any_output) return yan::launch_fp8_gemm_stacked_k(a, s, order);
     }
     if (type == yan::GemmType::Normal && want_auto && out_kind != yan::OutKind::E4M3 && a.scatter_world == 0) {
         const int slices = choose_cluster_slices(static_cast<int>(a.m), static_cast<int>(a.n), static_cast<int>(a.k), a.num_sms,
