@@ -67,3 +67,27 @@ def test_e4m3_output_on_128_wide_tiles(cuda_lib, m, n, k):
     assert yan_b200.read_device_status() == 0
     assert torch.equal(q[:m].view(torch.uint8), q_ref.view(torch.uint8)) and torch.equal(s[:m], s_ref)
     assert not q[m:].view(torch.uint8).any() and bool((s[m:] == 7.0).all()), "stored behind the last row"
+
+
+@pytest.mark.parametrize("op,m", [("f32", 200), ("f32", 33), ("linear", 200), ("linear", 65)])
+def test_whole_tiles_on_request_of_the_other_operators(cuda_lib, op, m):
+    """set_tail_cut(False) holds for fp32 output and fp8_linear too: bit for bit the result of an explicit width."""
+    import yan_b200
+    n, k = 512, 12800
+    lhs, rhs, _ = _operands(m, n, k, seed=10)
+    x = ref.make_inputs(m, n, k, seed=10, outliers=True)[0].cuda()
+    outs = [torch.empty(m, n, dtype=torch.float32 if op == "f32" else torch.bfloat16, device="cuda") for _ in range(3)]
+    run = (lambda out, **kw: yan_b200.gemm_fp8_fp8_f32_nt(lhs, rhs, out, **kw)) if op == "f32" else \
+        (lambda out, **kw: yan_b200.fp8_linear(x, rhs, out, **kw))
+    yan_b200.get_num_sms()
+    yan_b200.set_tail_cut(False)
+    try:
+        run(outs[0])
+    finally:
+        yan_b200.set_tail_cut(True)
+    run(outs[1], block_n=256)
+    run(outs[2])
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    assert torch.equal(outs[0], outs[1])
+    assert op != "f32" or not torch.equal(outs[0], outs[2]), "this shape is one whose K is cut by default"

@@ -97,8 +97,10 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         // the compiled-per-shape route, the cut last wave (which needs scratch) and whole tiles on request stay with the
         // Python path
         if (bf16 && jit_requested()) return code(kNotTaken);
-        if (bf16 && block_n == 0 && (PyObject_IsTrue(args[7]) ? k >= 96 * 128 && ceil_div(m, 128) * ceil_div(n, 256) > num_sms : m > 64))
-            return code(kNotTaken);
+        if (block_n == 0) {
+            const bool cut = PyObject_IsTrue(args[7]) == 1;
+            if (bf16 ? (cut ? k >= 96 * 128 && ceil_div(m, 128) * ceil_div(n, 256) > num_sms : m > 64) : !cut) return code(kNotTaken);
+        }
         const void *pa = a->data_ptr(), *pb = b->data_ptr();
         void* pout = out->data_ptr();
         if (!aligned(pa, 16) || !aligned(pb, 16) || !aligned(pout, 16)) return code(kNotTaken);
@@ -116,17 +118,18 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
 }
 
-// linear(a, rhs_q, rhs_scales, out, workspace or None, workspaces, block_n, num_sms); `workspaces` maps (device, bytes) to
-// the caller's buffers
+// linear(a, rhs_q, rhs_scales, out, workspace or None, workspaces, block_n, num_sms, tail_cut); `workspaces` maps (device, bytes)
+// to the caller's buffers
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     try {
         long block_n, num_sms;
-        if (nargs != 8 || !as_long(args[6], &block_n) || !as_long(args[7], &num_sms)) return code(kNotTaken);
+        if (nargs != 9 || !as_long(args[6], &block_n) || !as_long(args[7], &num_sms)) return code(kNotTaken);
         const at::Tensor *a = cuda_tensor(args[0]), *b = cuda_tensor(args[1]), *sb = cuda_tensor(args[2]),
                          *out = cuda_tensor(args[3]);
         if (!a || !b || !sb || !out || a->dim() != 2 || b->dim() != 2 || out->dim() != 2) return code(kNotTaken);
         const int64_t m = a->size(0), k = a->size(1), n = b->size(0), ldd = out->stride(0);
         if (!fits_int(m) || !fits_int(n) || !fits_int(k) || k % 128 != 0) return code(kNotTaken);
+        if (block_n == 0 && m > 64 && PyObject_IsTrue(args[8]) != 1) return code(kNotTaken);  // whole tiles: see the Python path
         if (a->scalar_type() != at::kBFloat16 || !a->is_contiguous() || !weights_ok(*b, *sb, n, k)) return code(kNotTaken);
         if (out->scalar_type() != at::kBFloat16 || out->size(0) != m || out->size(1) != n || out->stride(1) != 1 || !fits_int(ldd))
             return code(kNotTaken);

@@ -177,9 +177,10 @@ def tail_cut_enabled() -> bool:
 
 
 def set_tail_cut(enabled: bool) -> None:
-    """Lets gemm_fp8_fp8_bf16_nt(block_n=0) cut tiles along K: those of a nearly empty last wave, and all of them where there
-    are too few to occupy the GPU (default on).  Off, or with an explicit block_n, every tile of more than 64 rows is computed
-    whole by one CTA and the result does not depend on the grid."""
+    """Lets gemm_fp8_fp8_bf16_nt, gemm_fp8_fp8_f32_nt and fp8_linear with block_n=0 cut tiles along K: those of a nearly empty
+    last wave (the first of the three), and all of them where there are too few to occupy the GPU (default on).  Off, or with
+    an explicit block_n, every tile (bf16 output: of more than 64 rows) is computed whole by one CTA and the result does not
+    depend on the grid."""
     _tail_cut[0] = bool(enabled)
 
 
@@ -200,13 +201,15 @@ def gemm_fp8_fp8_f32_nt(lhs, rhs, out: torch.Tensor, block_n: int = 0) -> None:
     lhs_q, lhs_scales = lhs
     rhs_q, rhs_scales = rhs
     if _utils._num_sms is not None:
-        rc = _lib.fast().gemm_f32(lhs_q, lhs_scales, rhs_q, rhs_scales, out, block_n, _utils._num_sms, False)
+        rc = _lib.fast().gemm_f32(lhs_q, lhs_scales, rhs_q, rhs_scales, out, block_n, _utils._num_sms, _tail_cut[0])
         if rc != NOT_TAKEN:
             return _lib.check("yan_b200_gemm_fp8_fp8_f32_nt", rc)
     m, n, k = _check_operands(lhs_q, lhs_scales, rhs_q, rhs_scales, out, torch.float32)
     lhs_scales = get_col_major_tensor(lhs_scales)
     if m == 1 or lhs_scales.stride(1) != m:
         lhs_scales = lhs_scales.t().contiguous().t()
+    if block_n == 0 and not tail_cut_enabled():
+        block_n = get_best_configs(m, n, k, get_num_sms())[0]  # whole tiles
     _lib.call("yan_b200_gemm_fp8_fp8_f32_nt", lhs_q.data_ptr(), lhs_scales.data_ptr(), rhs_q.data_ptr(),
               rhs_scales.data_ptr(), out.data_ptr(), m, n, k, out.stride(0), _stream_ptr(), get_num_sms(), block_n)
 
@@ -302,7 +305,8 @@ def fp8_linear(a: torch.Tensor, rhs: Tuple[torch.Tensor, torch.Tensor], out: Opt
     two kernels; when omitted a per-(device, size) buffer is allocated once and reused."""
     rhs_q, rhs_scales = rhs
     if out is not None and _utils._num_sms is not None:
-        rc = _lib.fast().linear(a, rhs_q, rhs_scales, out, workspace, _workspaces, block_n, _utils._num_sms)
+        rc = _lib.fast().linear(a, rhs_q, rhs_scales, out, workspace, _workspaces, block_n, _utils._num_sms,
+                                _tail_cut[0])
         if rc != NOT_TAKEN:
             _lib.check("yan_b200_fp8_linear_bf16", rc)
             return out
@@ -314,6 +318,8 @@ def fp8_linear(a: torch.Tensor, rhs: Tuple[torch.Tensor, torch.Tensor], out: Opt
     if out is None:
         out = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     assert out.shape == (m, n) and out.dtype == torch.bfloat16 and out.stride(1) == 1
+    if block_n == 0 and m > 64 and not tail_cut_enabled():
+        block_n = get_best_configs(m, n, k, get_num_sms())[0]  # whole tiles
     need = fp8_linear_workspace_bytes(m, k)
     if workspace is None:
         key = (a.device.index, need)
