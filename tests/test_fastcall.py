@@ -77,3 +77,34 @@ def test_errors_are_raised_as_before(cuda_lib):
     from yan_b200._lib import YanB200Error
     with pytest.raises(YanB200Error):
         yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out, block_n=48)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("native", [True, False])
+def test_default_workspace_of_fp8_linear_belongs_to_a_stream(cuda_lib, native, monkeypatch):
+    """Calls of the same sizes on two streams, one right behind the other: neither may see the other's activations."""
+    import yan_b200
+    from yan_b200 import _lib
+    from yan_b200.jit_kernels import gemm
+    if not native:
+        class NotTaken:
+            def __getattr__(self, name):
+                return lambda *args: -1
+        monkeypatch.setattr(_lib, "_fast", NotTaken())
+    monkeypatch.setattr(gemm, "_workspaces", {})
+    m, n, k = 512, 4096, 2048
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    rhs = yan_b200.per_block_cast_to_fp8((torch.randn(n, k, generator=gen, device="cuda") * 0.02).to(torch.bfloat16))
+    xs = [torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(2)]
+    want = [yan_b200.fp8_linear(x, rhs).clone() for x in xs]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = [[torch.empty(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(20)] for _ in streams]
+    torch.cuda.synchronize()
+    for i in range(20):
+        for x, stream, out in zip(xs, streams, outs):
+            with torch.cuda.stream(stream):
+                yan_b200.fp8_linear(x, rhs, out[i])
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    assert len({ws.data_ptr() for ws in gemm._workspaces.values()}) == 3, "the default stream's and the two others'"
+    assert all(torch.equal(o, w) for w, out in zip(want, outs) for o in out)

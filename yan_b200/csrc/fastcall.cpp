@@ -118,8 +118,8 @@ PyObject* gemm(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     }
 }
 
-// linear(a, rhs_q, rhs_scales, out, workspace or None, workspaces, block_n, num_sms, tail_cut); `workspaces` maps (device, bytes)
-// to the caller's buffers
+// linear(a, rhs_q, rhs_scales, out, workspace or None, workspaces, block_n, num_sms, tail_cut); `workspaces` maps (device,
+// stream, bytes) to the caller's buffers
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     try {
         long block_n, num_sms;
@@ -133,11 +133,14 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         if (a->scalar_type() != at::kBFloat16 || !a->is_contiguous() || !weights_ok(*b, *sb, n, k)) return code(kNotTaken);
         if (out->scalar_type() != at::kBFloat16 || out->size(0) != m || out->size(1) != n || out->stride(1) != 1 || !fits_int(ldd))
             return code(kNotTaken);
+        void* stream = current_stream();
         const size_t need = g_entries.workspace_bytes(static_cast<int>(m), static_cast<int>(k));
         PyObject* ws_obj = args[4];
         if (ws_obj == Py_None) {
             if (!PyDict_CheckExact(args[5])) return code(kNotTaken);
-            PyObject* key = Py_BuildValue("(in)", static_cast<int>(a->get_device()), static_cast<Py_ssize_t>(need));
+            PyObject* key = Py_BuildValue("(iKn)", static_cast<int>(a->get_device()),
+                                          static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)),
+                                          static_cast<Py_ssize_t>(need));
             if (key == nullptr) {
                 PyErr_Clear();
                 return code(kNotTaken);
@@ -150,7 +153,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
         if (!ws_ptr || ws_ptr->scalar_type() != at::kByte || static_cast<size_t>(ws_ptr->numel()) < need) return code(kNotTaken);
         const at::Tensor ws = *ws_ptr;  // held: the dictionary may change while the interpreter runs other threads
         const void *pa = a->data_ptr(), *pb = b->data_ptr(), *psb = sb->data_ptr();
-        void *pout = out->data_ptr(), *pws = ws.data_ptr(), *stream = current_stream();
+        void *pout = out->data_ptr(), *pws = ws.data_ptr();
         const size_t ws_bytes = static_cast<size_t>(ws.numel());
         int rc = 0;
         Py_BEGIN_ALLOW_THREADS

@@ -302,7 +302,9 @@ def fp8_linear(a: torch.Tensor, rhs: Tuple[torch.Tensor, torch.Tensor], out: Opt
                workspace: Optional[torch.Tensor] = None, block_n: int = 0) -> torch.Tensor:
     """bf16 a [M,K] -> quantize (1x128) -> FP8 GEMM with rhs -> bf16 [M,N], one C-ABI call.
     `workspace` (uint8, >= fp8_linear_workspace_bytes(M, K)) holds the quantized activations between the
-    two kernels; when omitted a per-(device, size) buffer is allocated once and reused."""
+    two kernels; when omitted a per-(device, stream, size) buffer is allocated once and reused: calls on one stream are
+    ordered, calls on different streams must not share it.  (CUDA graphs captured on the same stream do share it: give
+    graphs that are replayed at the same time a workspace of their own.)"""
     rhs_q, rhs_scales = rhs
     if out is not None and _utils._num_sms is not None:
         rc = _lib.fast().linear(a, rhs_q, rhs_scales, out, workspace, _workspaces, block_n, _utils._num_sms,
@@ -322,7 +324,7 @@ def fp8_linear(a: torch.Tensor, rhs: Tuple[torch.Tensor, torch.Tensor], out: Opt
         block_n = get_best_configs(m, n, k, get_num_sms())[0]  # whole tiles
     need = fp8_linear_workspace_bytes(m, k)
     if workspace is None:
-        key = (a.device.index, need)
+        key = (a.device.index, _stream_ptr().value or 0, need)
         if key not in _workspaces:
             _workspaces[key] = torch.empty(need, dtype=torch.uint8, device=a.device)
         workspace = _workspaces[key]
