@@ -138,3 +138,32 @@ def test_output_that_only_the_streaming_kernels_take_beyond_their_default(cuda_l
     # both kernels sum in fp32, in another order: bf16 results differ by one rounding of few values
     assert ref.rel_frobenius(out[:, :n].cpu(), general.cpu()) <= 1e-3 and not out[:, n].any()
     assert call(n, k - 128) == 1 and call(n - 16, k) == 1
+
+
+def test_num_sms_caps_the_grid(cuda_lib, tmp_path):
+    """set_num_sms leaves SMs to another stream: no GEMM of a small batch may have more CTAs than that, whichever kernel it
+    goes to (row groups that fit, M <= 16 in wider ones, the general kernel)."""
+    import json
+    import yan_b200
+    from torch.profiler import ProfilerActivity, profile
+    shapes = [(16, 1024, 2048), (16, 4096, 2048), (9, 9600, 1024), (64, 7168, 2048), (40, 528, 7168), (32, 6400, 640)]
+    calls = []
+    for m, n, k in shapes:
+        lhs, rhs, d_ref = _operands(m, n, k, seed=m + n + k)
+        calls.append((*_device(lhs, rhs), torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), d_ref))
+    sms = yan_b200.get_num_sms()
+    yan_b200.set_num_sms(100)
+    try:
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            for lhs, rhs, out, _ in calls:
+                yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out)
+            torch.cuda.synchronize()
+    finally:
+        yan_b200.set_num_sms(sms)
+    assert yan_b200.read_device_status() == 0
+    for _, _, out, d_ref in calls:
+        assert ref.rel_frobenius(out.cpu(), d_ref) <= 1e-3
+    prof.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
+    grids = [e["args"]["grid"] for e in events if e.get("cat") == "kernel" and "yan::" in e.get("name", "")]
+    assert len(grids) == len(shapes) and all(x * y * z <= 100 for x, y, z in grids), grids

@@ -169,13 +169,14 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
         const bool general_ok = yan::is_aligned(a.out, 16) && a.ldd % 8 == 0 && a.num_sms <= sm_count;
         const bool any_output = small_m_ok || (stacked_ok && (a.m <= 16 || a.n / 32 <= static_cast<uint32_t>(sm_count)));
         if (want_auto && (general_ok || any_output) &&
-            yan::stacked_k_preferred(a.m, a.n, a.k, static_cast<uint32_t>(sm_count), static_cast<uint32_t>(max_smem)))
+            yan::stacked_k_preferred(a.m, a.n, a.k, static_cast<uint32_t>(a.num_sms), static_cast<uint32_t>(sm_count),
+                                     static_cast<uint32_t>(max_smem)))
             return yan::launch_fp8_gemm_stacked_k(a, s, order);
         if (block_n == 1 || (want_auto && !general_ok && small_m_ok)) {
             if (!small_m_ok) return yan::kBadArgument;
             return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || after_own_quantizer);
         }
-        // what the general kernel is faster at, with an output that it does not take
+        // what the general kernel is the default for, with an output that it does not take
         if (want_auto && !general_ok && any_output) return yan::launch_fp8_gemm_stacked_k(a, s, order);
     }
     if (type == yan::GemmType::Normal && want_auto && out_kind != yan::OutKind::E4M3 && a.scatter_world == 0) {

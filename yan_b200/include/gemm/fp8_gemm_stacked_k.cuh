@@ -319,7 +319,8 @@ inline int launch_fp8_gemm_stacked_k(const GemmArgs& a, cudaStream_t stream, Sta
     if (cudaGetDevice(&device) != cudaSuccess) return kLaunchFailed;
     cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    const StackedConfig c = choose_stacked_config(a.m, a.n, a.k, static_cast<uint32_t>(sm_count), static_cast<uint32_t>(max_smem));
+    const StackedConfig c = choose_stacked_config(a.m, a.n, a.k, static_cast<uint32_t>(a.num_sms), static_cast<uint32_t>(sm_count),
+                                                  static_cast<uint32_t>(max_smem));
 
     bool ok = true;
     const CUtensorMap map_w = make_2d_tma_desc_u8_sw128(a.rhs, a.n, a.k, a.k, 128 / c.stack, ok);

@@ -63,9 +63,14 @@ struct StackedConfig {
 //     processing cluster are no multiple of four); the others would start when the first have ended (M=64 K=7168: N=2112 8.5,
 //     N=2176 14.1 against 10.6 with clusters of two, N=2368 14.4 against 10.7; M=32 N=2304 K=8192 12.8 against 9.3; M=16
 //     N=1184 K=16384 12.3 against 9.2).  Where two CTAs fit an SM all of them start at once (M=16 N=1184 K=8192 5.9 against 6.7).
-inline StackedConfig choose_stacked_config(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t max_smem) {
+// `num_sms` below `sm_count` is a cap on the CTAs of a launch (the other SMs are somebody else's): M <= 16 then takes the
+// twice as wide row groups of M <= 32 where those fit the cap and its own do not.
+inline StackedConfig choose_stacked_config(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t sm_count,
+                                           uint32_t max_smem) {
     StackedConfig c;
     c.m_pad = m <= 16 ? 16 : m <= 32 ? 32 : 64;
+    if (num_sms > sm_count) num_sms = sm_count;
+    if (c.m_pad == 16 && num_sms < sm_count && ceil_div(n, 32u) > num_sms && ceil_div(n, 64u) <= num_sms) c.m_pad = 32;
     c.stack = c.m_pad == 16 ? 4 : 2;
     const uint32_t groups = ceil_div(n, 128u / c.stack);
     for (c.cluster = 1; c.cluster < 4; c.cluster *= 2) {
@@ -86,11 +91,14 @@ inline StackedConfig choose_stacked_config(uint32_t m, uint32_t n, uint32_t k, u
 // the pair kernel, but N=28672 K=1024 14.4 against 12.8 with 256-wide tiles of the general one; M=64 N=9216 K=2048 9.8
 // against 12.4, but N=14336 K=1024 15.6 against 9.7), and for M <= 16, where several waves of CTAs hold up against the
 // general kernel unless K is long too (N=28672: K=4096 28.0 against 31.0, K=8192 49.1 against 49.0, K=18432 104 against 92).
-inline bool stacked_k_preferred(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t max_smem) {
+// Under a cap it is the default only with at most that many CTAs: its grid is not persistent and would spread over all SMs.
+inline bool stacked_k_preferred(uint32_t m, uint32_t n, uint32_t k, uint32_t num_sms, uint32_t sm_count, uint32_t max_smem) {
     if (m > 64 || n % 16 != 0 || k % kBlockK != 0) return false;
-    const StackedConfig c = choose_stacked_config(m, n, k, num_sms, max_smem);
+    const StackedConfig c = choose_stacked_config(m, n, k, num_sms, sm_count, max_smem);
     const uint32_t groups = ceil_div(n, 128u / c.stack), steps = stacked_k_steps(k, c.stack, c.cluster);
-    if (groups > num_sms * (c.m_pad == 64 ? 1 : 2) && (m > 16 || steps > 16)) return false;
+    if (num_sms < sm_count ? groups * c.cluster > num_sms
+                           : groups > sm_count * (c.m_pad == 64 ? 1 : 2) && (m > 16 || steps > 16))
+        return false;
     return stacked_k_smem_layout(c.m_pad, c.stack, steps, c.slots, c.cluster).total <= max_smem;
 }
 
