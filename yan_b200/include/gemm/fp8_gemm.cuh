@@ -90,6 +90,18 @@ __device__ __forceinline__ bool bounded_wait(uint64_t* bar, uint32_t parity, vol
     return true;
 }
 
+// A role that gave up gives copies still in flight time to land before the CTA's shared memory is released.
+__device__ __forceinline__ void drain_copies() {
+    const uint64_t t0 = ptx::globaltimer_ns();
+    while (ptx::globaltimer_ns() - t0 < 1000000ull) __nanosleep(1000);
+}
+
+// A CTA that gave up tells another CTA of its cluster, between two meetings of the cluster of which the first says that the
+// other's flag has been initialized: incomplete sums must not be stored.
+__device__ __forceinline__ void abort_cta(volatile uint32_t* abort_flag, uint32_t cta_rank) {
+    ptx::st_cluster_u32(ptx::map_to_cta(ptx::smem_u32(const_cast<uint32_t*>(abort_flag)), cta_rank), 1u);
+}
+
 template <typename out_t, uint32_t kCols>
 __device__ __forceinline__ void store_row(out_t* dst, const float (&acc)[kCols], uint32_t n_first, uint32_t shape_n) {
     if constexpr (sizeof(out_t) == 2) {
@@ -178,17 +190,19 @@ constexpr bool kExchangeInRing = BLOCK_N > 64;
 template <typename out_t, uint32_t BLOCK_N, uint32_t kCols>
 __device__ __forceinline__ void exchange_and_store(const GemmParams& p, uint32_t smem, uint32_t slice, uint32_t tile_row0,
                                                    uint32_t tile_col0, uint32_t row_in_tile, uint32_t col0, uint32_t thread,
-                                                   bool alive, const float (&acc)[kCols]) {
+                                                   bool alive, volatile uint32_t* abort_flag, const float (&acc)[kCols]) {
     // [slice][own row][BLOCK_N + 4] floats; the padding spreads the rows a warp writes over the banks
     constexpr uint32_t kRowBytes = (BLOCK_N + 4) * 4;
     const uint32_t slices = p.tail_slices, own_rows = kBlockM / slices;
-    ptx::cluster_wait();  // every CTA of the cluster has started (it arrived at the top of the kernel) ...
+    ptx::cluster_wait();  // every CTA of the cluster has started (it arrived behind its prologue) ...
     // ... or, where the rows land in the operand ring, is done with it: its products are complete
     if constexpr (kExchangeInRing<BLOCK_N>) ptx::cluster_arrive(), ptx::cluster_wait();
     const uint32_t owner = row_in_tile / own_rows;
     const uint32_t dst = ptx::map_to_cta(smem, owner) + (slice * own_rows + row_in_tile % own_rows) * kRowBytes + col0 * 4;
 #pragma unroll
     for (uint32_t j = 0; j < kCols; j += 4) ptx::st_cluster_v4_f32(dst + j * 4, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
+    if (!alive && thread % 32u == 0)
+        for (uint32_t r = 0; r < slices; ++r) abort_cta(abort_flag, r);
     ptx::cluster_arrive(), ptx::cluster_wait();
     // 2 * slices threads per row, BLOCK_N / (2 * slices) columns each, eight at a time
     const uint32_t per_row = 2 * slices, part = thread % per_row;
@@ -209,7 +223,7 @@ __device__ __forceinline__ void exchange_and_store(const GemmParams& p, uint32_t
         }
     }
     const uint32_t n0 = tile_col0 + part * cols;
-    const bool row_ok = alive && row < p.shape_m;
+    const bool row_ok = alive && *abort_flag == 0 && row < p.shape_m;
     if constexpr (sizeof(out_t) == 1) {
         // the row's 128 columns are one quantization group, spread over per_row neighbouring lanes (see store_tile_e4m3)
         float amax = 0.0f;
@@ -450,7 +464,6 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     static_assert(!kClusterK || (kGemmType == GemmType::Normal && !kTail && !kScatter && BLOCK_N <= 128), "one tile per cluster");
     constexpr bool kCutK = kTail || kClusterK;
     constexpr uint32_t kExchangeOffset = detail::kExchangeInRing<BLOCK_N> ? 0 : align_up(L::kOffAbort + 4, 16u);
-    if constexpr (kClusterK) ptx::cluster_arrive_relaxed();                // waited for in front of the exchange
     // k-blocks [kb_begin, kb_begin + kb_count) of every tile this CTA computes: all of them, or the CTA's slice
     const uint32_t tail_slice = kCutK ? blockIdx.x % p.tail_slices : 0u, tail_tile = kCutK ? blockIdx.x / p.tail_slices : 0u;
     const uint32_t kb_begin = kCutK ? (tail_slice * num_k_blocks) / p.tail_slices : 0u;
@@ -502,6 +515,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     __syncthreads();
     ptx::tcgen05_fence_after_thread_sync();
     const uint32_t tmem_base = *tmem_slot;
+    if constexpr (kClusterK) ptx::cluster_arrive();  // waited for in front of the exchange
     if (p.clock_probe != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
         p.clock_probe[0] = clock64();
         p.clock_probe[1] = static_cast<long long>(ptx::globaltimer_ns());
@@ -585,11 +599,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
 #ifdef YAN_PHASE_STAMPS
             if (p.clock_probe != nullptr && blockIdx.x == 0 && lane_idx == 0) p.clock_probe[4] = waited_empty;
 #endif
-            if (!alive) {
-                // Give copies still in flight time to land before the CTA's shared memory is released.
-                const uint64_t t0 = ptx::globaltimer_ns();
-                while (ptx::globaltimer_ns() - t0 < 1000000ull) __nanosleep(1000);
-            }
+            if (!alive) detail::drain_copies();
         } else if (warp_idx == 1 && lane_idx == 0) {
             // ------------------------------ MMA issuer ------------------------------
             Sched sched(p.shape_m, p.shape_n, p.grouped_layout, p.num_groups);
@@ -843,7 +853,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                 ptx::named_barrier_arrive(2, kNumMathWarps * 32 + 64);
                 detail::exchange_and_store<out_t, BLOCK_N>(p, ptx::smem_u32(smem) + kExchangeOffset, tail_slice, m_block_idx * kBlockM,
                                                            n_block_idx * BLOCK_N, row_in_tile, col0, threadIdx.x - kNumControlThreads,
-                                                           alive && *abort_flag == 0, acc);
+                                                           alive, abort_flag, acc);
                 continue;
             }
             // the e4m3 output needs one 128-column group per thread (BLOCK_N = 256, two warpgroups): the launcher refuses every

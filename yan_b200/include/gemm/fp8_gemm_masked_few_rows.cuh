@@ -179,11 +179,7 @@ __global__ void __launch_bounds__(kFewRowsThreads, 1)
                 }
             }
         }
-        if (!alive) {
-            // Give copies still in flight time to land before the CTA's shared memory is released.
-            const uint64_t t0 = ptx::globaltimer_ns();
-            while (ptx::globaltimer_ns() - t0 < 1000000ull) __nanosleep(1000);
-        }
+        if (!alive) detail::drain_copies();
     } else if (warp_idx == 1 && lane_idx == 0) {
         // ------------------------------ MMA issuer ------------------------------
         uint32_t stage = 0, phase = 0, buf = 0, buf_phase = 0;

@@ -199,6 +199,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
 #pragma unroll
         for (uint32_t m = 0; m < M_PAD; m += 4)
             ptx::st_cluster_v4_f32(remote + m * 4u, acc[m], acc[m + 1], acc[m + 2], acc[m + 3]);
+        if (!alive && lane_idx == 0) detail::abort_cta(abort_flag, 0);
     }
     ptx::cluster_arrive();
     ptx::cluster_wait();
