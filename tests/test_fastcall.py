@@ -18,6 +18,22 @@ def test_leaves_unusual_arguments_to_python():
         f.bind(1)
 
 
+def test_a_missing_or_foreign_front_leaves_everything_to_python(monkeypatch, tmp_path):
+    """Another torch's extension is not loaded, whatever the file times say; the operators then run without it."""
+    from yan_b200 import _lib
+    assert _lib.front_built_for(_lib.front_key())
+    with open(_lib.FASTCALL_PATH, "rb") as f:
+        built = f.read()
+    foreign = tmp_path / "_fastcall.so"
+    foreign.write_bytes(built.replace(b"yan_b200 front|torch ", b"yan_b200 front|torch 0"))
+    for path in (str(tmp_path / "missing.so"), str(foreign)):
+        monkeypatch.setattr(_lib, "FASTCALL_PATH", path)
+        monkeypatch.setattr(_lib, "_fast", None)
+        with pytest.warns(RuntimeWarning, match="python -m yan_b200.build"):
+            assert _lib.fast().gemm_bf16(1, 2) == -1
+        assert _lib.fast().per_token_cast() == -1
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("m", [1, 7, 130])
 @pytest.mark.parametrize("k", [128, 512])

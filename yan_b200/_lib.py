@@ -10,6 +10,8 @@ from __future__ import annotations
 
 import ctypes
 import os
+import sys
+import warnings
 from typing import Optional
 
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
@@ -87,18 +89,45 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def front_key() -> str:
+    """What the native front depends on besides its source: it is compiled against torch's C++ interface, which changes from
+    one torch to the next without an error at load time."""
+    import torch
+    return f"yan_b200 front|torch {torch.__version__}|{sys.implementation.cache_tag}|"
+
+
+def front_built_for(key: str) -> bool:
+    """Whether the native front is there and was compiled with a key that begins like this (it holds its key as a string)."""
+    try:
+        with open(FASTCALL_PATH, "rb") as f:
+            return key.encode() in f.read()
+    except OSError:
+        return False
+
+
+class _NoFront:
+    """Leaves every call to the Python path."""
+
+    def __getattr__(self, name):
+        return lambda *args: -1
+
+
 def fast():
-    """The native front of the hot operators (csrc/fastcall.cpp), bound to the loaded library."""
+    """The native front of the hot operators (csrc/fastcall.cpp), bound to the loaded library.  Where it is missing or was built
+    for another torch, the operators run through their Python path: the same kernels, a few microseconds more per call."""
     global _fast
     if _fast is None:
-        if not os.path.exists(FASTCALL_PATH):
-            raise ImportError(f"{FASTCALL_PATH} is missing: build it with `python -m yan_b200.build`")
+        handle = lib()
+        if not front_built_for(front_key()):
+            warnings.warn(f"{FASTCALL_PATH} is missing or was built for another torch: calls go through ctypes "
+                          "(build it with `python -m yan_b200.build`)", RuntimeWarning)
+            _fast = _NoFront()
+            return _fast
         import importlib.util
-        import torch  # noqa: F401  (its libraries have to be loaded first)
         spec = importlib.util.spec_from_file_location("yan_b200.lib._fastcall", FASTCALL_PATH)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
-        module.bind(*(ctypes.cast(getattr(lib(), name), _P).value for name in
+        module.bind(*(ctypes.cast(getattr(handle, name), _P).value for name in
                       ("yan_b200_gemm_fp8_fp8_bf16_nt", "yan_b200_gemm_fp8_fp8_f32_nt", "yan_b200_fp8_linear_bf16",
                        "yan_b200_fp8_linear_workspace_bytes", "yan_b200_per_token_cast_to_fp8")))
         _fast = module

@@ -9,6 +9,7 @@ checkout; the JIT layer in yan_b200/jit remains for user templates and per-shape
 from __future__ import annotations
 
 import argparse
+import hashlib
 import os
 import shutil
 import subprocess
@@ -78,9 +79,11 @@ def _run(cmd: List[str], verbose: bool) -> None:
 def build_fastcall(force: bool = False, verbose: bool = False) -> str:
     """Compiles the native front of the Python operators (a CPython extension against the installed torch)."""
     import torch
+    from . import _lib
     torch_dir = os.path.dirname(torch.__file__)
-    if not force and os.path.exists(FASTCALL_PATH) and os.path.getmtime(FASTCALL_PATH) > max(
-            os.path.getmtime(FASTCALL_SRC), os.path.getmtime(os.path.join(torch_dir, "version.py"))):
+    with open(FASTCALL_SRC, "rb") as f:
+        key = f"{_lib.front_key()}{hashlib.sha256(f.read()).hexdigest()[:16]}|"
+    if not force and _lib.front_built_for(key):
         return FASTCALL_PATH
     cxx = os.environ.get("CXX") or shutil.which("g++")
     if not cxx:
@@ -89,6 +92,7 @@ def build_fastcall(force: bool = False, verbose: bool = False) -> str:
     cuda_home = os.path.dirname(os.path.dirname(find_nvcc()))
     tmp = FASTCALL_PATH + f".tmp.{os.getpid()}"
     _run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+          f'-DYAN_FRONT_KEY="{key}"',
           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", f"-I{torch_dir}/include",
           f"-I{torch_dir}/include/torch/csrc/api/include", f"-I{sysconfig.get_paths()['include']}", f"-I{cuda_home}/include",
           FASTCALL_SRC, "-o", tmp, f"-L{torch_dir}/lib", "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"], verbose)
@@ -97,8 +101,8 @@ def build_fastcall(force: bool = False, verbose: bool = False) -> str:
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compiles the library and the native front of its operators if they are missing or older than any source.  Returns
-    the library's path."""
+    """Compiles the library if it is missing or older than any source, and the native front of its operators if it is missing
+    or was built from another source or for another torch.  Returns the library's path."""
     with ThreadPoolExecutor(max_workers=1) as pool:
         front = pool.submit(build_fastcall, force, verbose)
         path = _build_cuda_library(force, verbose)

@@ -17,6 +17,9 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+// What this file was compiled from and for, read out of the built file before it is loaded (front_key in _lib.py).
+extern "C" __attribute__((used)) const char yan_b200_front_key[] = YAN_FRONT_KEY;
+
 namespace {
 
 constexpr int kNotTaken = -1;
