@@ -124,3 +124,12 @@ def test_default_workspace_of_fp8_linear_belongs_to_a_stream(cuda_lib, native, m
     assert yan_b200.read_device_status() == 0
     assert len({ws.data_ptr() for ws in gemm._workspaces.values()}) == 3, "the default stream's and the two others'"
     assert all(torch.equal(o, w) for w, out in zip(want, outs) for o in out)
+
+
+@pytest.mark.gpu
+def test_quantizer_returns_a_tuple_whatever_holds_its_outputs(cuda_lib):
+    import yan_b200
+    x = torch.ones(8, 256, dtype=torch.bfloat16, device="cuda")
+    q, s = yan_b200.per_token_cast_to_fp8(x)
+    result = yan_b200.per_token_cast_to_fp8(x, out=[q, s])
+    assert isinstance(result, tuple) and result[0] is q and result[1] is s

@@ -30,7 +30,7 @@ def per_token_cast_to_fp8(x: torch.Tensor, out: Optional[Tuple[torch.Tensor, tor
         rc = _lib.fast().per_token_cast(x, *out)
         if rc != -1:  # -1: not an ordinary call, left to the checks below
             _lib.check("yan_b200_per_token_cast_to_fp8", rc)
-            return out
+            return tuple(out)
     assert x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2
     m, k = x.shape
     assert m > 0 and k > 0 and k % 128 == 0, "K must be a positive multiple of 128"
