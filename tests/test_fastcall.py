@@ -74,6 +74,45 @@ def test_same_results_as_the_python_path(cuda_lib, m, k, monkeypatch):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 16, 200])
+def test_takes_the_ordinary_calls_and_no_others(cuda_lib, m):
+    """Return codes of the native front itself: 0 where it made the call, -1 where it left it."""
+    import yan_b200
+    from yan_b200 import _lib
+    f, n, k, sms = _lib.fast(), 256, 512, yan_b200.get_num_sms()
+    a, b = ref.make_inputs(m, n, k, seed=m)
+    x, (w, ws) = a.cuda(), (t.cuda() for t in ref.per_block_cast_to_fp8(b))
+    q, s = yan_b200.per_token_cast_to_fp8(x)
+    out, f32 = torch.empty(m, n, dtype=torch.bfloat16, device="cuda"), torch.empty(m, n, device="cuda")
+    wide = torch.empty(m, 512, dtype=torch.bfloat16, device="cuda")[:, :n]
+    scratch = torch.empty(yan_b200.fp8_linear_workspace_bytes(m, k), dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    kept = {(0, stream, scratch.numel()): scratch}
+
+    assert f.per_token_cast(x, q, s) == 0
+    assert f.gemm_bf16(q, s, w, ws, out, 0, sms, True) == 0 and f.gemm_bf16(q, s, w, ws, wide, 0, sms, True) == 0
+    assert f.gemm_bf16(q, s, w, ws, out, 64, sms, False) == 0
+    assert f.gemm_f32(q, s, w, ws, f32, 0, sms, True) == 0
+    assert f.linear(x, w, ws, out, scratch, {}, 0, sms, True) == 0 and f.linear(x, w, ws, out, None, kept, 0, sms, True) == 0
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    assert f.gemm_bf16(q, s, w, ws, out, 48, sms, True) == 1, "the library's own refusal"
+
+    row_major = torch.empty(m + 1, k // 128, device="cuda")[:m]
+    assert f.per_token_cast(x, q, row_major) == -1 and f.per_token_cast(x.float(), q, s) == -1
+    s_wide = torch.empty(k // 128, m + 3, device="cuda").t()[:m]
+    for args in ((q, s_wide, w, ws, out), (q, s, w.t(), ws, out), (q, s, w, ws, f32), (q.cpu(), s, w, ws, out), (q, s, w, s, out)):
+        assert f.gemm_bf16(*args, 0, sms, True) == -1
+    assert f.gemm_f32(q, s, w, ws, out, 0, sms, True) == -1
+    assert f.gemm_f32(q, s, w, ws, f32, 0, sms, False) == -1, "whole tiles on request"
+    assert (f.gemm_bf16(q, s, w, ws, out, 0, sms, False) == -1) == (m > 64)
+    assert (f.linear(x, w, ws, out, scratch, {}, 0, sms, False) == -1) == (m > 64)
+    assert f.linear(x, w, ws, out, None, {}, 0, sms, True) == -1, "no scratch yet"
+    assert f.linear(x, w, ws, out, scratch[1:], {}, 0, sms, True) == -1 and f.linear(x.float(), w, ws, out, scratch, {}, 0, sms, True) == -1
+    torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
 def test_errors_are_raised_as_before(cuda_lib):
     import yan_b200
     a, b = ref.make_inputs(16, 256, 512, seed=1)

@@ -45,8 +45,8 @@ def test_edges_match_oracle_and_general_kernel(cuda_lib, m, n, k):
 
 @pytest.mark.parametrize("m", [16, 64])
 def test_fp8_linear_sees_weights_written_just_before(cuda_lib, m):
-    """The weight quantizer, then fp8_linear on its result, many times over the same buffers: every launch may start
-    early, none may read the weights of the round before."""
+    """Weights copied in, then fp8_linear on them, many times over the same buffers: none may read the weights of the round
+    before."""
     import yan_b200
     n, k = 2048, 2048
     gen = torch.Generator().manual_seed(3)
@@ -64,6 +64,40 @@ def test_fp8_linear_sees_weights_written_just_before(cuda_lib, m):
     torch.cuda.synchronize()
     assert yan_b200.read_device_status() == 0
     assert all(torch.equal(g, want[i % 4]) for i, g in enumerate(got))
+
+
+@pytest.mark.parametrize("m", [16, 64, 200])
+def test_fp8_linear_waits_for_a_kernel_that_lets_it_start_early(cuda_lib, m):
+    """The weight codes are written by the activation quantizer, a kernel that lets its successors start before it has finished,
+    directly in front of fp8_linear: no copy between them that would separate them.  The quantizer of fp8_linear must not let its
+    GEMM load weights before that kernel has completed, nor the next writer overwrite them before the GEMM has."""
+    import yan_b200
+    n, k = 7168, 2048
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    ws = [torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    codes = (torch.empty(n, k, dtype=torch.float8_e4m3fn, device="cuda"), torch.empty(k // 128, n, device="cuda").t())
+    rhs = (codes[0], torch.full((n // 128, k // 128), 0.01, device="cuda"))
+    workspace = torch.empty(yan_b200.fp8_linear_workspace_bytes(m, k), dtype=torch.uint8, device="cuda")
+    outs = [torch.empty(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(16)]
+    yan_b200.get_num_sms()
+
+    def run(sync):
+        for i, out in enumerate(outs):
+            yan_b200.per_token_cast_to_fp8(ws[i % 4], out=codes)
+            if sync:
+                torch.cuda.synchronize()
+            yan_b200.fp8_linear(x, rhs, out, workspace)
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    want = run(True)
+    assert not torch.equal(want[0], want[1])
+    for _ in range(3):
+        assert all(torch.equal(g, w) for g, w in zip(run(False), want))
+    assert yan_b200.read_device_status() == 0
 
 
 def test_output_that_only_the_streaming_kernels_take(cuda_lib):
