@@ -189,9 +189,9 @@ def test_num_sms_caps_the_grid(cuda_lib, tmp_path):
     yan_b200.set_num_sms(100)
     try:
         with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            for lhs, rhs, out, _ in calls:
+            for lhs, rhs, out, _ in calls * 2:  # the profiler may miss the first launches
                 yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out)
-            torch.cuda.synchronize()
+                torch.cuda.synchronize()
     finally:
         yan_b200.set_num_sms(sms)
     assert yan_b200.read_device_status() == 0
@@ -200,4 +200,4 @@ def test_num_sms_caps_the_grid(cuda_lib, tmp_path):
     prof.export_chrome_trace(str(tmp_path / "trace.json"))
     events = json.loads((tmp_path / "trace.json").read_text())["traceEvents"]
     grids = [e["args"]["grid"] for e in events if e.get("cat") == "kernel" and "yan::" in e.get("name", "")]
-    assert len(grids) == len(shapes) and all(x * y * z <= 100 for x, y, z in grids), grids
+    assert len(grids) >= len(shapes) and all(x * y * z <= 100 for x, y, z in grids), grids
