@@ -91,3 +91,19 @@ def test_whole_tiles_on_request_of_the_other_operators(cuda_lib, op, m):
     assert yan_b200.read_device_status() == 0
     assert torch.equal(outs[0], outs[1])
     assert op != "f32" or not torch.equal(outs[0], outs[2]), "this shape is one whose K is cut by default"
+
+
+# the two epilogues of fp32 output on 256-wide tiles: 128-byte box rows up to K = 3456, the ring of scales from K = 3584 on
+@pytest.mark.parametrize("k", [128, 3456, 3584])
+@pytest.mark.parametrize("m,n", [(129, 272), (300, 2304)])
+def test_f32_output_on_256_wide_tiles(cuda_lib, m, n, k):
+    import yan_b200
+    lhs, rhs, d_ref = _operands(m, n, k, seed=m + k)
+    outs = [torch.full((m + 1, n + 4), 7.0, device="cuda") for _ in range(2)]
+    for out, block_n in zip(outs, (256, 128)):
+        yan_b200.gemm_fp8_fp8_f32_nt(lhs, rhs, out[:m, :n], block_n=block_n)
+    torch.cuda.synchronize()
+    assert yan_b200.read_device_status() == 0
+    assert torch.equal(*outs), "the same products in the same order"
+    assert ref.rel_frobenius(outs[0][:m, :n].cpu(), d_ref) <= 1e-5
+    assert bool((outs[0][m:] == 7.0).all()) and bool((outs[0][:, n:] == 7.0).all())
