@@ -96,11 +96,12 @@ __device__ __forceinline__ void drain_copies() {
     while (ptx::globaltimer_ns() - t0 < 1000000ull) __nanosleep(1000);
 }
 
-// A CTA that gave up tells another CTA of its cluster, between two meetings of the cluster of which the first says that the
-// other's flag has been initialized: incomplete sums must not be stored.
-__device__ __forceinline__ void abort_cta(volatile uint32_t* abort_flag, uint32_t cta_rank) {
-    ptx::st_cluster_u32(ptx::map_to_cta(ptx::smem_u32(const_cast<uint32_t*>(abort_flag)), cta_rank), 1u);
-}
+// What a thread that gave up sends to another CTA of its cluster in place of incomplete sums, which must not be stored: a NaN that
+// arithmetic does not produce (its NaN is 0x7fffffff).  It travels with the sums, so nothing has to be ordered for it: a flag in
+// the other CTA would have to be initialized there first, and an arrival behind that costs 0.75 us (a release waits for the loads
+// issued before it).
+constexpr uint32_t kGaveUpSum = 0x7fdeadadu;
+__device__ __forceinline__ bool is_complete(float sum) { return __float_as_uint(sum) != kGaveUpSum; }
 
 template <typename out_t, uint32_t kCols>
 __device__ __forceinline__ void store_row(out_t* dst, const float (&acc)[kCols], uint32_t n_first, uint32_t shape_n) {
@@ -190,19 +191,18 @@ constexpr bool kExchangeInRing = BLOCK_N > 64;
 template <typename out_t, uint32_t BLOCK_N, uint32_t kCols>
 __device__ __forceinline__ void exchange_and_store(const GemmParams& p, uint32_t smem, uint32_t slice, uint32_t tile_row0,
                                                    uint32_t tile_col0, uint32_t row_in_tile, uint32_t col0, uint32_t thread,
-                                                   bool alive, volatile uint32_t* abort_flag, const float (&acc)[kCols]) {
+                                                   bool alive, const float (&acc)[kCols]) {
     // [slice][own row][BLOCK_N + 4] floats; the padding spreads the rows a warp writes over the banks
     constexpr uint32_t kRowBytes = (BLOCK_N + 4) * 4;
     const uint32_t slices = p.tail_slices, own_rows = kBlockM / slices;
-    ptx::cluster_wait();  // every CTA of the cluster has started (it arrived behind its prologue) ...
+    ptx::cluster_wait();  // every CTA of the cluster has started (it arrived at the top of the kernel) ...
     // ... or, where the rows land in the operand ring, is done with it: its products are complete
     if constexpr (kExchangeInRing<BLOCK_N>) ptx::cluster_arrive(), ptx::cluster_wait();
     const uint32_t owner = row_in_tile / own_rows;
     const uint32_t dst = ptx::map_to_cta(smem, owner) + (slice * own_rows + row_in_tile % own_rows) * kRowBytes + col0 * 4;
 #pragma unroll
-    for (uint32_t j = 0; j < kCols; j += 4) ptx::st_cluster_v4_f32(dst + j * 4, acc[j], acc[j + 1], acc[j + 2], acc[j + 3]);
-    if (!alive && thread % 32u == 0)
-        for (uint32_t r = 0; r < slices; ++r) abort_cta(abort_flag, r);
+    for (uint32_t j = 0; j < kCols; j += 4)
+        ptx::st_cluster_v4_f32(dst + j * 4, j % 8 != 0 || alive ? acc[j] : __uint_as_float(kGaveUpSum), acc[j + 1], acc[j + 2], acc[j + 3]);
     ptx::cluster_arrive(), ptx::cluster_wait();
     // 2 * slices threads per row, BLOCK_N / (2 * slices) columns each, eight at a time
     const uint32_t per_row = 2 * slices, part = thread % per_row;
@@ -213,17 +213,19 @@ __device__ __forceinline__ void exchange_and_store(const GemmParams& p, uint32_t
     const uint32_t src = smem + row_local * kRowBytes + part * cols * 4;
 #pragma unroll
     for (uint32_t c = 0; c < kMaxCols; ++c) v[c] = 0.0f;
+    bool complete = alive;
     for (uint32_t s = 0; s < slices; ++s) {
 #pragma unroll
         for (uint32_t c = 0; c < kMaxCols; c += 4) {
             if (c < cols) {
                 const float4 t = ptx::ld_shared_v4_f32(src + s * own_rows * kRowBytes + c * 4);
+                if (c % 8 == 0) complete = complete && is_complete(t.x);
                 v[c] += t.x, v[c + 1] += t.y, v[c + 2] += t.z, v[c + 3] += t.w;
             }
         }
     }
     const uint32_t n0 = tile_col0 + part * cols;
-    const bool row_ok = alive && *abort_flag == 0 && row < p.shape_m;
+    const bool row_ok = complete && row < p.shape_m;
     if constexpr (sizeof(out_t) == 1) {
         // the row's 128 columns are one quantization group, spread over per_row neighbouring lanes (see store_tile_e4m3)
         float amax = 0.0f;
@@ -464,6 +466,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     static_assert(!kClusterK || (kGemmType == GemmType::Normal && !kTail && !kScatter && BLOCK_N <= 128), "one tile per cluster");
     constexpr bool kCutK = kTail || kClusterK;
     constexpr uint32_t kExchangeOffset = detail::kExchangeInRing<BLOCK_N> ? 0 : align_up(L::kOffAbort + 4, 16u);
+    if constexpr (kClusterK) ptx::cluster_arrive_relaxed();                // waited for in front of the exchange
     // k-blocks [kb_begin, kb_begin + kb_count) of every tile this CTA computes: all of them, or the CTA's slice
     const uint32_t tail_slice = kCutK ? blockIdx.x % p.tail_slices : 0u, tail_tile = kCutK ? blockIdx.x / p.tail_slices : 0u;
     const uint32_t kb_begin = kCutK ? (tail_slice * num_k_blocks) / p.tail_slices : 0u;
@@ -515,7 +518,6 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     __syncthreads();
     ptx::tcgen05_fence_after_thread_sync();
     const uint32_t tmem_base = *tmem_slot;
-    if constexpr (kClusterK) ptx::cluster_arrive();  // waited for in front of the exchange
     if (p.clock_probe != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
         p.clock_probe[0] = clock64();
         p.clock_probe[1] = static_cast<long long>(ptx::globaltimer_ns());
@@ -853,7 +855,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                 ptx::named_barrier_arrive(2, kNumMathWarps * 32 + 64);
                 detail::exchange_and_store<out_t, BLOCK_N>(p, ptx::smem_u32(smem) + kExchangeOffset, tail_slice, m_block_idx * kBlockM,
                                                            n_block_idx * BLOCK_N, row_in_tile, col0, threadIdx.x - kNumControlThreads,
-                                                           alive, abort_flag, acc);
+                                                           alive, acc);
                 continue;
             }
             // the e4m3 output needs one 128-column group per thread (BLOCK_N = 256, two warpgroups): the launcher refuses every

@@ -187,6 +187,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
     if (warp_idx == 4) {
         // Tensor memory goes back before this CTA waits for the other one (see fp8_gemm_stacked_k.cuh).
         ptx::named_barrier_sync(2, 160);
+        if (*abort_flag != 0) detail::drain_copies();  // a role gave up: loads and products may be in flight
         ptx::tcgen05_fence_after_thread_sync();
         ptx::tmem_dealloc(tmem_base, tmem_cols);
     }
@@ -199,7 +200,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
 #pragma unroll
         for (uint32_t m = 0; m < M_PAD; m += 4)
             ptx::st_cluster_v4_f32(remote + m * 4u, acc[m], acc[m + 1], acc[m + 2], acc[m + 3]);
-        if (!alive && lane_idx == 0) detail::abort_cta(abort_flag, 0);
+        // it gave up: CTA 0, whose flag has been initialized (the two have met since), must not store incomplete sums
+        if (!alive && lane_idx == 0)
+            ptx::st_cluster_u32(ptx::map_to_cta(ptx::smem_u32(const_cast<uint32_t*>(abort_flag)), 0), 1u);
     }
     ptx::cluster_arrive();
     ptx::cluster_wait();

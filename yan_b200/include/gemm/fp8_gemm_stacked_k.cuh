@@ -89,6 +89,7 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     // k-block of (k-part q, step s): (part0 + q) * steps + s
     const uint32_t part0 = rank * kStack;
 
+    if (cluster > 1) ptx::cluster_arrive();  // waited for in front of the exchange: by then every CTA of it has started
     if (order == kAfterAnyKernel) ptx::grid_dependency_wait();
     if (order == kConstantWeights) ptx::grid_dependency_launch_dependents();
     if (warp_idx == 5) {
@@ -137,7 +138,6 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     __syncthreads();  // barriers and the tensor memory address exist
     ptx::tcgen05_fence_after_thread_sync();
     const uint32_t tmem_base = *tmem_slot;
-    if (cluster > 1) ptx::cluster_arrive();  // waited for in front of the exchange: by then every CTA of it has got here
 
     if (warp_idx == 4) {
         ptx::grid_dependency_wait();
@@ -149,10 +149,7 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
                 const uint32_t it = s / kSlots;
                 bool ok = detail::bounded_wait(empty_barriers + slot, (it - 1) & 1, abort_flag, p, 7);
                 ok = __all_sync(group_mask, ok);
-                if (!ok) {
-                    detail::drain_copies();
-                    break;
-                }
+                if (!ok) break;
                 if (part == 0) ptx::mbar_arrive_expect_tx(full_barriers + slot, kStepBytes);
                 __syncwarp(group_mask);
                 ptx::tma_load_2d(w_dst, &tensor_map_w, full_barriers + slot, static_cast<int32_t>((kb_lane + s) * kBlockK),
@@ -164,12 +161,10 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     } else if (warp_idx == 5) {
         if (lane_idx == 0) {
             constexpr uint32_t idesc = make_instr_desc_e4m3_f32(128, kMmaN);
-            bool ok = true;
             for (uint32_t s = 0; s < steps; ++s) {
                 const uint32_t r = s % kSlots, b = s % kTmemSlots, b_it = s / kTmemSlots;
-                ok = detail::bounded_wait(full_barriers + r, (s / kSlots) & 1, abort_flag, p, 5) &&
-                     (b_it == 0 || detail::bounded_wait(tmem_empty_barriers + b, (b_it - 1) & 1, abort_flag, p, 8));
-                if (!ok) break;
+                if (!detail::bounded_wait(full_barriers + r, (s / kSlots) & 1, abort_flag, p, 5)) break;
+                if (b_it > 0 && !detail::bounded_wait(tmem_empty_barriers + b, (b_it - 1) & 1, abort_flag, p, 8)) break;
                 ptx::tcgen05_fence_after_thread_sync();
                 const uint64_t w_desc = make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L.off_w + r * 16384u));
                 const uint64_t x_desc = make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L.off_x + r * (kMmaN * 128u)));
@@ -180,11 +175,11 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
                 ptx::umma_commit(done_barriers + b);
                 if (!kOneRing && s + kSlots < steps) ptx::umma_commit(empty_barriers + r);
             }
-            if (!ok) detail::drain_copies();  // and products
         }
         __syncwarp();
-        // the promotion warps have read the last accumulator
+        // the promotion warps have read the last accumulator, or a role gave up: then loads and products may be in flight
         ptx::named_barrier_sync(2, 160);
+        if (*abort_flag != 0) detail::drain_copies();
         ptx::tcgen05_fence_after_thread_sync();
         ptx::tmem_dealloc(tmem_base, kTmemCols);
     }
@@ -256,10 +251,10 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
         __syncwarp();
         ptx::cluster_wait();
         if (warp_idx < 4 && rank != 0) {
+            if (*abort_flag != 0) v[0] = __uint_as_float(detail::kGaveUpSum);
             const uint32_t remote = ptx::map_to_cta(exchange + (rank - 1) * (M_PAD * kRows * 4u), 0);
 #pragma unroll
             for (uint32_t j = 0; j < kMPerThread; ++j) ptx::st_cluster_f32(remote + (m0 + j) * (kRows * 4u), v[j]);
-            if (!alive && lane_idx == 0) detail::abort_cta(abort_flag, 0);
         }
         ptx::cluster_arrive();
         ptx::cluster_wait();
@@ -267,9 +262,13 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     if (warp_idx < 4 && rank == 0 && alive && *abort_flag == 0) {
         for (uint32_t c = 0; c + 1 < cluster; ++c) {
 #pragma unroll
-            for (uint32_t j = 0; j < kMPerThread; ++j) v[j] += ptx::ld_shared_f32(exchange + (c * M_PAD + m0 + j) * (kRows * 4u));
+            for (uint32_t j = 0; j < kMPerThread; ++j) {
+                const float sum = ptx::ld_shared_f32(exchange + (c * M_PAD + m0 + j) * (kRows * 4u));
+                if (j == 0) alive = alive && detail::is_complete(sum);
+                v[j] += sum;
+            }
         }
-        if (n0 + rr < p.shape_n) {
+        if (alive && n0 + rr < p.shape_n) {
             __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + n0 + rr;
 #pragma unroll
             for (uint32_t j = 0; j < kMPerThread; ++j)
