@@ -93,8 +93,8 @@ def test_whole_tiles_on_request_of_the_other_operators(cuda_lib, op, m):
     assert op != "f32" or not torch.equal(outs[0], outs[2]), "this shape is one whose K is cut by default"
 
 
-# the two epilogues of fp32 output on 256-wide tiles: 128-byte box rows up to K = 3456, the ring of scales from K = 3584 on
-@pytest.mark.parametrize("k", [128, 3456, 3584])
+# the two epilogues of fp32 output on 256-wide tiles: 128-byte box rows up to K = 3968, the ring of scales from K = 4096 on
+@pytest.mark.parametrize("k", [128, 3968, 4096])
 @pytest.mark.parametrize("m,n", [(129, 272), (300, 2304)])
 def test_f32_output_on_256_wide_tiles(cuda_lib, m, n, k):
     import yan_b200
