@@ -185,7 +185,9 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
         if (slices != 0) return yan::launch_gemm_cluster_k(static_cast<uint32_t>(slices), out_kind, a, s);
     }
     // Groups of at most 128 rows: the kernel that follows masked_m, unless 32-wide tiles of the general one fit the GPU at once
-    // (6 groups, N=768 K=4096: 14.9 us against 14.1; 8 groups, N=768 K=7168: 22.3 against 31.4).
+    // (6 groups, N=768 K=4096: 14.9 us against 14.1; 8 groups, N=768 K=7168: 22.3 against 31.4).  Full groups of 128 rows lose up
+    // to 15 % against 128-row tiles, groups of 64 gain 7 to 23 % (figures in jit_kernels/gemm.py); the counts are on the device, so
+    // a caller who knows that groups are nearly full says so with a width.
     if (type == yan::GemmType::GroupedMasked && want_auto && a.m <= 128 &&
         static_cast<uint64_t>(a.num_groups) * ((a.n + 31) / 32) > static_cast<uint64_t>(a.num_sms))
         return a.m <= 64 ? yan::launch_masked_few_rows<64>(a, s) : yan::launch_masked_few_rows<128>(a, s);
@@ -326,7 +328,7 @@ YAN_EXPORT void yan_b200_gemm_fp8_fp8_e4m3_nt(const void* lhs, const void* lhs_s
     a.out_scales_ld = static_cast<uint32_t>(out_scales_ld);
     a.m = m, a.n = n, a.k = k;
     a.num_sms = num_sms;
-    // the epilogue quantizes one 1 x 128 group per thread, which only the 256-wide tile provides
+    // 256: a thread holds one whole 1 x 128 group; dispatch_gemm takes 128-wide tiles instead where every CTA has at most one
     set_rc(return_code, dispatch_gemm(yan::GemmType::Normal, yan::OutKind::E4M3, a, 256, stream));
 }
 

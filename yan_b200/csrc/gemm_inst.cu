@@ -18,7 +18,7 @@ int YAN_CAT(launch_gemm_bn, YAN_BLOCK_N)(GemmType type, OutKind out, const GemmA
         return GemmLauncher<BN, S, GemmType::Normal, float>::launch(args, stream);
     }
     if (out == OutKind::E4M3) {
-        // one 1 x 128 quantization group per epilogue thread: only the 256-wide tile has it
+        // one 1 x 128 quantization group per epilogue thread: only the 256-wide tile has it (launch_gemm_e4m3_bn128 spreads a group)
         if constexpr (BN == 256) {
             if (type != GemmType::Normal) return kBadArgument;
             return GemmLauncher<BN, S, GemmType::Normal, E4m3Out>::launch(args, stream);

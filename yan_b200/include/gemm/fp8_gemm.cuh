@@ -1288,7 +1288,7 @@ struct GemmClusterKLauncher {
 // (yan/jit_kernels/gemm.py:20-30).  Template parameter order and the member names are the
 // template's; the eighth parameter (the reference's TMA multicast width) is accepted for source
 // compatibility and must be 1: this kernel never multicasts.  The scale and output "descriptors" carry plain pointers because the kernel
-// reads scales with ordinary loads and writes D with 16-byte stores.
+// copies scales with cp.async (or loads them) and writes D with 16-byte stores.
 // ---------------------------------------------------------------------------------------------
 // A kernel library compiled by the JIT layer (-DYAN_JIT_KERNEL) has a status word and a wait bound of its own, read
 // and set through two extra exports next to `launch`; the prebuilt library passes its own through GemmArgs instead.

@@ -16,7 +16,7 @@
 // weight row meeting in ONE CTA: the sum over them is a shared-memory exchange between its four promotion warps.
 //
 // K is cut into F * cluster parts of `steps` k-blocks (the last ones may be short or empty: their loads are out of bounds
-// and read zeros).  A cluster of 2, 4 or 8 CTAs shares the R weight rows when N / R CTAs alone would leave SMs idle; its
+// and read zeros).  A cluster of 2 or 4 CTAs shares the R weight rows when N / R CTAs alone would leave SMs idle; its
 // CTAs send their M_PAD x R sums to the first one through distributed shared memory.
 //
 //   warps 0-3: promotion (thread = TMEM lane = (k-part, weight row)); warp 4: producer, lane = (slot, k-part);
