@@ -311,8 +311,8 @@ struct GemmSmemLayout {
     static constexpr uint32_t kOffScales = kOffStore + kStoreBytes;
     static constexpr bool kScaleRing = kOffScales + kNumScaleSlots * kScaleSlotBytes + 2048 <= 232448;
     static constexpr uint32_t kOffBarriers = kOffScales + (kScaleRing ? kNumScaleSlots * kScaleSlotBytes : 0);
-    // ring full/empty, TMEM full/empty per buffer and column half
-    static constexpr uint32_t kNumBarriers = 2 * kNumStages + 4 * kNumTmemBufs + (kScaleRing ? kNumScaleSlots : 0);
+    // ring full/empty, TMEM full/empty
+    static constexpr uint32_t kNumBarriers = 2 * kNumStages + 2 * kNumTmemBufs + (kScaleRing ? kNumScaleSlots : 0);
     static constexpr uint32_t kOffTmemSlot = kOffBarriers + kNumBarriers * 8;
     static constexpr uint32_t kOffAbort = kOffTmemSlot + 4;
     // +1024: the dynamic shared-memory base is re-aligned to 1024 bytes inside the kernel.
@@ -324,11 +324,6 @@ struct GemmSmemLayout {
 // Compile-time knobs of the promotion (defaults = the measured best on B200; the others stay selectable for the tuner
 // and for measurements):
 //   YAN_PROMO_CHUNK        columns per tcgen05.ld (8, 16 or 32).
-//   YAN_PROMO_SPLIT_HALVES 1: the MMA thread issues each k-block as two half-width MMA streams (columns [0, N/2) then
-//                          [N/2, N)), each with its own TMEM-full / TMEM-empty barrier: warpgroup 0 is released half a
-//                          k-block before warpgroup 1 (so the two warps that share an SM sub-partition do not load and
-//                          multiply in lockstep) and each half of a TMEM buffer is recycled as soon as its own
-//                          warpgroup has read it.  0: one full-width stream, one barrier pair per buffer.
 //   YAN_PROMO_EARLY_PROBE  1: the next k-block's TMEM-full barrier is probed (without blocking) right after this
 //                          k-block's last load, so that the answer arrives under the last FMAs.
 //   YAN_WIDE_STORE_BOXES   1: every instance stages its output in 32 x 128-byte boxes.  The scatter instance always does,
@@ -340,9 +335,6 @@ struct GemmSmemLayout {
 // of sixteen warps fills the issue slots).
 #ifndef YAN_PROMO_CHUNK
 #define YAN_PROMO_CHUNK 16
-#endif
-#ifndef YAN_PROMO_SPLIT_HALVES
-#define YAN_PROMO_SPLIT_HALVES 0
 #endif
 #ifndef YAN_TAIL_MIN_K_BLOCKS
 #define YAN_TAIL_MIN_K_BLOCKS 96
@@ -405,7 +397,6 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     using Sched = Scheduler<kGemmType, kBlockM, BLOCK_N>;
     constexpr uint32_t kNumTmemBufs = L::kNumTmemBufs;
     constexpr uint32_t kNumMathWGs = get_num_math_warpgroups(BLOCK_N);
-    static_assert(kNumMathWGs == 2 || YAN_PROMO_SPLIT_HALVES == 0, "the half-width streams assume two promotion warpgroups");
     static_assert(RegisterBudgetCheck<BLOCK_N>::ok);
     constexpr uint32_t kColsPerWG = BLOCK_N / kNumMathWGs;
     constexpr uint32_t kNumMathWarps = 4 * kNumMathWGs;
@@ -438,22 +429,22 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
 #endif
     constexpr bool kShiftRing = YAN_PROMO_SHIFT_RING >= 0 ? (YAN_PROMO_SHIFT_RING != 0) : (kScaleDepth == 2);
     constexpr uint32_t kLoopUnroll = kShiftRing ? 1 : kScaleDepth;
+    // Narrow tiles are bound by the thread that issues their products; wide ones by the promotion, and under the power cap they gain
+    // nothing from a faster issue (M=8192 N=28672 K=8192 1909 -> 1927 us, M=4096 N=7168 K=18432 540 -> 549).
+    constexpr bool kUnrolledIssue = BLOCK_N <= 160;
     // bf16 / fp32 output through the staging boxes (see GemmSmemLayout) when a warpgroup's columns are whole 64-byte pieces.
     constexpr bool kStagedStore = L::kStoreBytes != 0 && sizeof(out_t) >= 2 && kNumMathWarps == L::kNumStoreBoxes &&
                                   (kColsPerWG * sizeof(out_t)) % L::kStoreRowBytes == 0;
     constexpr uint32_t kStoreCols = L::kStoreRowBytes / (sizeof(out_t) >= 2 ? sizeof(out_t) : 2);  // columns per box row
-    // Half-width MMA streams: each warpgroup's columns are produced and recycled on their own barriers.
-    constexpr bool kSplitHalves = (YAN_PROMO_SPLIT_HALVES != 0);
-    constexpr uint32_t kNumHalves = kSplitHalves ? 2 : 1;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
 
     uint64_t* full_barriers = reinterpret_cast<uint64_t*>(smem + L::kOffBarriers);
     uint64_t* empty_barriers = full_barriers + kNumStages;
-    uint64_t* tmem_full_barriers = empty_barriers + kNumStages;            // [buf][half]
-    uint64_t* tmem_empty_barriers = tmem_full_barriers + 2 * kNumTmemBufs;  // [buf][half]
-    uint64_t* scale_full_barriers = tmem_empty_barriers + 2 * kNumTmemBufs;
+    uint64_t* tmem_full_barriers = empty_barriers + kNumStages;
+    uint64_t* tmem_empty_barriers = tmem_full_barriers + kNumTmemBufs;
+    uint64_t* scale_full_barriers = tmem_empty_barriers + kNumTmemBufs;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kOffTmemSlot);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem + L::kOffAbort);
 
@@ -498,9 +489,9 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             ptx::mbar_init(empty_barriers + i, 1);  // tcgen05.commit of the MMA thread
         }
 #pragma unroll
-        for (uint32_t i = 0; i < 2 * kNumTmemBufs; ++i) {
+        for (uint32_t i = 0; i < kNumTmemBufs; ++i) {
             ptx::mbar_init(tmem_full_barriers + i, 1);                             // tcgen05.commit
-            ptx::mbar_init(tmem_empty_barriers + i, kNumMathWarps / kNumHalves);  // one arrival per promotion warp
+            ptx::mbar_init(tmem_empty_barriers + i, kNumMathWarps);  // one arrival per promotion warp
         }
         if constexpr (L::kScaleRing) {
 #pragma unroll
@@ -526,9 +517,9 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     if (warp_idx < 4) {
         ptx::reg_dealloc<get_num_control_registers(BLOCK_N)>();
 
-        if (warp_idx == 0 && (L::kScaleRing || lane_idx == 0)) {
+        if (warp_idx == 0) {
             // ------------------------------ producer ------------------------------
-            // Lane 0 loads a k-block's operands; with kScaleRing all lanes copy its scales to shared memory at the same time, so
+            // One lane loads a k-block's operands; with kScaleRing all lanes copy its scales to shared memory at the same time, so
             // that they are there kNumStages k-blocks before the promotion needs them (loads into registers, however far ahead,
             // end up waiting for an L2 round trip: a moved register waits for its load, and the loads in flight share a few
             // scoreboards.  M=4096 N=7168 K=18432 whole tiles 764 -> 650 cycles per k-block, 597 -> 541 us; M=8192 N=7168
@@ -544,6 +535,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             [[maybe_unused]] const uint32_t s_scales = ptx::smem_u32(smem + L::kOffScales);
             [[maybe_unused]] const bool sa_aligned = p.sa_ld % 4 == 0 && reinterpret_cast<uintptr_t>(p.scales_a) % 16 == 0;
             bool alive = true;
+            [[maybe_unused]] bool stage_free = false;
             [[maybe_unused]] long long waited_empty = 0;
             while (alive && next_tile(sched, m_block_idx, n_block_idx)) {
                 const int group = sched.get_group(m_block_idx);
@@ -559,15 +551,14 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                     p.scales_b + (static_cast<size_t>(group) * num_sb_rows + sb_row) * num_k_blocks + kb_begin;
                 for (uint32_t kb = kb_begin; kb < kb_begin + kb_count; ++kb) {
                     YAN_STAMP(w0);
-                    bool ok = detail::bounded_wait(empty_barriers + stage, phase ^ 1, abort_flag, p, 1);
-                    if constexpr (L::kScaleRing) ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) {
+                    const bool ok = (kUnrolledIssue && stage_free) || detail::bounded_wait(empty_barriers + stage, phase ^ 1, abort_flag, p, 1);
+                    if (!__all_sync(0xffffffffu, ok)) {
                         alive = false;
                         break;
                     }
                     YAN_STAMP(w1);
                     YAN_STAMP_ADD(waited_empty, w0, w1);
-                    if (!L::kScaleRing || lane_idx == 0) {
+                    if (kUnrolledIssue ? ptx::elect_one() : lane_idx == 0) {
                         ptx::mbar_arrive_expect_tx(full_barriers + stage,
                                                    L::SMEM_A_SIZE_PER_STAGE + L::SMEM_B_SIZE_PER_STAGE);
                         ptx::tma_load_2d(smem + L::kOffA + stage * L::SMEM_A_SIZE_PER_STAGE, &tensor_map_a,
@@ -575,8 +566,13 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                         ptx::tma_load_2d(smem + L::kOffB + stage * L::SMEM_B_SIZE_PER_STAGE, &tensor_map_b,
                                          full_barriers + stage, static_cast<int32_t>(kb * kBlockK), b_row);
                     }
+                    __syncwarp();
+                    if (++stage == kNumStages) {
+                        stage = 0;
+                        phase ^= 1;
+                    }
+                    if constexpr (kUnrolledIssue) stage_free = ptx::mbar_test_wait(empty_barriers + stage, phase ^ 1);
                     if constexpr (L::kScaleRing) {
-                        __syncwarp();
                         const uint32_t dst = s_scales + slot * L::kScaleSlotBytes;
                         if (whole) {
                             ptx::cp_async_16(dst + lane_idx * 16u, sa_ptr + lane_idx * 4u);
@@ -591,10 +587,6 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                         ++sb_ptr;
                         slot = slot + 1 == L::kNumScaleSlots ? 0 : slot + 1;
                     }
-                    if (++stage == kNumStages) {
-                        stage = 0;
-                        phase ^= 1;
-                    }
                 }
             }
             if constexpr (L::kScaleRing) ptx::cp_async_wait_all();
@@ -602,61 +594,78 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             if (p.clock_probe != nullptr && blockIdx.x == 0 && lane_idx == 0) p.clock_probe[4] = waited_empty;
 #endif
             if (!alive) detail::drain_copies();
-        } else if (warp_idx == 1 && lane_idx == 0) {
+        } else if (warp_idx == 1 && (kUnrolledIssue ? ptx::elect_one() : lane_idx == 0)) {
             // ------------------------------ MMA issuer ------------------------------
+            // kUnrolledIssue: both waits of the next k-block are probed before this one's products are issued: a wait that succeeds at once still
+            // takes some 75 cycles.
             Sched sched(p.shape_m, p.shape_n, p.grouped_layout, p.num_groups);
             if (p.tile_limit != 0) sched.num_blocks = min(sched.num_blocks, p.tile_limit);
-            constexpr uint32_t kUmmaN = BLOCK_N / kNumHalves;
-            constexpr uint32_t idesc = make_instr_desc_e4m3_f32(kBlockM, kUmmaN);
-            // rows [kUmmaN, BLOCK_N) of the B tile start kUmmaN 128-byte rows further on (whole 8-row swizzle atoms)
-            constexpr uint32_t kDescHalfStep = (kUmmaN * kBlockK) >> 4;
-            static_assert(kUmmaN % 16 == 0, "UMMA with M = 128 needs N % 16 == 0");
-            uint32_t m_block_idx, n_block_idx, stage = 0, phase = 0, buf = 0, buf_phase = 0;
+            constexpr uint32_t idesc = make_instr_desc_e4m3_f32(kBlockM, BLOCK_N);
+            const uint32_t a_low = make_smem_desc_low(ptx::smem_u32(smem + L::kOffA));
+            const uint32_t b_low = make_smem_desc_low(ptx::smem_u32(smem + L::kOffB));
+            uint32_t m_block_idx, n_block_idx, phase = 0, buf_phase = 0;
+            [[maybe_unused]] uint32_t stage = 0, buf = 0, pos = 0;
             bool alive = true;
+            [[maybe_unused]] bool operands_ready = false, buffer_ready = false;
             [[maybe_unused]] long long waited_full = 0, waited_tmem = 0;
             YAN_STAMP(mma_begin);
             while (alive && next_tile(sched, m_block_idx, n_block_idx)) {
                 if (sched.get_group(m_block_idx) < 0) continue;
-                for (uint32_t kb = 0; kb < kb_count && alive; ++kb) {
-                    YAN_STAMP(w0);
-                    if (!detail::bounded_wait(full_barriers + stage, phase, abort_flag, p, 2)) {
-                        alive = false;
-                        break;
-                    }
-                    YAN_STAMP(w1);
-                    YAN_STAMP_ADD(waited_full, w0, w1);
-                    const uint64_t a_desc =
-                        make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L::kOffA + stage * L::SMEM_A_SIZE_PER_STAGE));
-                    const uint64_t b_desc =
-                        make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L::kOffB + stage * L::SMEM_B_SIZE_PER_STAGE));
-#pragma unroll
-                    for (uint32_t h = 0; h < kNumHalves; ++h) {
-                        YAN_STAMP(w2);
-                        if (!detail::bounded_wait(tmem_empty_barriers + buf * 2 + h, buf_phase ^ 1, abort_flag, p, 3)) {
+                if constexpr (!kUnrolledIssue) {
+                    for (uint32_t kb = 0; kb < kb_count; ++kb) {
+                        YAN_STAMP(w0);
+                        if (!detail::bounded_wait(full_barriers + stage, phase, abort_flag, p, 2)) {
                             alive = false;
                             break;
                         }
-                        YAN_STAMP(w3);
-                        YAN_STAMP_ADD(waited_tmem, w2, w3);
+                        YAN_STAMP(w1);
+                        YAN_STAMP_ADD(waited_full, w0, w1);
+                        if (!detail::bounded_wait(tmem_empty_barriers + buf, buf_phase ^ 1, abort_flag, p, 3)) {
+                            alive = false;
+                            break;
+                        }
+                        YAN_STAMP(w2);
+                        YAN_STAMP_ADD(waited_tmem, w1, w2);
                         ptx::tcgen05_fence_after_thread_sync();
-                        const uint32_t tmem_d = tmem_base + buf * BLOCK_N + h * kUmmaN;
+                        const uint64_t a_desc = make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L::kOffA + stage * L::SMEM_A_SIZE_PER_STAGE));
+                        const uint64_t b_desc = make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L::kOffB + stage * L::SMEM_B_SIZE_PER_STAGE));
 #pragma unroll
                         for (uint32_t k = 0; k < kBlockK / kUmmaK; ++k)
-                            ptx::umma_f8f6f4_ss(tmem_d, a_desc + k * kDescKStep, b_desc + h * kDescHalfStep + k * kDescKStep,
-                                                idesc, k > 0);
-                        if (h + 1 == kNumHalves)
-                            ptx::umma_commit(empty_barriers + stage);       // smem stage reusable once these MMAs are done
-                        ptx::umma_commit(tmem_full_barriers + buf * 2 + h);  // partial sum of this k-block is complete
+                            ptx::umma_f8f6f4_ss(tmem_base + buf * BLOCK_N, a_desc + k * kDescKStep, b_desc + k * kDescKStep, idesc, k > 0);
+                        ptx::umma_commit(empty_barriers + stage);    // smem stage reusable once these MMAs are done
+                        ptx::umma_commit(tmem_full_barriers + buf);  // partial sum of this k-block is complete
+                        if (++stage == kNumStages) {
+                            stage = 0;
+                            phase ^= 1;
+                        }
+                        if (++buf == kNumTmemBufs) {
+                            buf = 0;
+                            buf_phase ^= 1;
+                        }
                     }
-                    if (++stage == kNumStages) {
-                        stage = 0;
-                        phase ^= 1;
-                    }
-                    if (++buf == kNumTmemBufs) {
-                        buf = 0;
-                        buf_phase ^= 1;
-                    }
+                    continue;
                 }
+                alive = ring_steps<common_round(kNumStages, kNumTmemBufs)>(pos, kb_count, [&](const uint32_t u) {
+                    const uint32_t stage = u % kNumStages, buf = u % kNumTmemBufs;
+                    YAN_STAMP(w0);
+                    if (!operands_ready && !detail::bounded_wait(full_barriers + stage, phase, abort_flag, p, 2)) return false;
+                    YAN_STAMP(w1);
+                    YAN_STAMP_ADD(waited_full, w0, w1);
+                    if (!buffer_ready && !detail::bounded_wait(tmem_empty_barriers + buf, buf_phase ^ 1, abort_flag, p, 3))
+                        return false;
+                    YAN_STAMP(w2);
+                    YAN_STAMP_ADD(waited_tmem, w1, w2);
+                    ptx::tcgen05_fence_after_thread_sync();
+                    if (stage + 1 == kNumStages) phase ^= 1;
+                    if (buf + 1 == kNumTmemBufs) buf_phase ^= 1;
+                    operands_ready = ptx::mbar_test_wait(full_barriers + (stage + 1) % kNumStages, phase);
+                    buffer_ready = ptx::mbar_test_wait(tmem_empty_barriers + (buf + 1) % kNumTmemBufs, buf_phase ^ 1);
+                    umma_k_block(tmem_base + buf * BLOCK_N, a_low + stage * (L::SMEM_A_SIZE_PER_STAGE >> 4),
+                                 b_low + stage * (L::SMEM_B_SIZE_PER_STAGE >> 4), idesc);
+                    ptx::umma_commit(tmem_full_barriers + buf);  // partial sum of this k-block is complete
+                    ptx::umma_commit(empty_barriers + stage);        // smem stage reusable once these MMAs are done
+                    return true;
+                });
             }
 #ifdef YAN_PHASE_STAMPS
             if (p.clock_probe != nullptr && blockIdx.x == 0) {
@@ -690,7 +699,6 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
         const uint32_t row_in_tile = quarter * 32 + lane_idx;
         const uint32_t col0 = wg * kColsPerWG;
         const uint32_t tmem_lane_base = tmem_base + ((quarter * 32u) << 16) + col0;
-        const uint32_t half = kSplitHalves ? wg : 0;
 
         Sched sched(p.shape_m, p.shape_n, p.grouped_layout, p.num_groups);
         if (p.tile_limit != 0) sched.num_blocks = min(sched.num_blocks, p.tile_limit);
@@ -744,7 +752,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                 auto release_buffer = [&]() {
                     ptx::tcgen05_fence_before_thread_sync();
                     __syncwarp();
-                    if (lane_idx == 0) ptx::mbar_arrive(tmem_empty_barriers + buf * 2 + half);
+                    if (lane_idx == 0) ptx::mbar_arrive(tmem_empty_barriers + buf);
                 };
                 auto group_scale = [&](uint32_t group16) { return (kTwoScales && group16 >= hi_from) ? scale_hi : scale; };
 #pragma unroll
@@ -760,7 +768,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                         if constexpr (kEarlyProbe) {
                             const uint32_t nb = (buf + 1 == kNumTmemBufs) ? 0 : buf + 1;
                             const uint32_t np = (buf + 1 == kNumTmemBufs) ? buf_phase ^ 1 : buf_phase;
-                            next_ready = __all_sync(0xffffffffu, ptx::mbar_test_wait(tmem_full_barriers + nb * 2 + half, np));
+                            next_ready = __all_sync(0xffffffffu, ptx::mbar_test_wait(tmem_full_barriers + nb, np));
                         }
                     }
 #pragma unroll
@@ -801,7 +809,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                     }
                     YAN_STAMP(w0);
                     const bool ok = (kEarlyProbe && next_ready) ||
-                                    detail::bounded_wait(tmem_full_barriers + buf * 2 + half, buf_phase, abort_flag, p, 4);
+                                    detail::bounded_wait(tmem_full_barriers + buf, buf_phase, abort_flag, p, 4);
                     if (!__all_sync(0xffffffffu, ok && scales_ok)) {
                         alive = false;
                         break;
@@ -838,7 +846,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                         }
                         YAN_STAMP(w0);
                         const bool ok = (kEarlyProbe && next_ready) ||
-                                        detail::bounded_wait(tmem_full_barriers + buf * 2 + half, buf_phase, abort_flag, p, 4);
+                                        detail::bounded_wait(tmem_full_barriers + buf, buf_phase, abort_flag, p, 4);
                         if (!__all_sync(0xffffffffu, ok)) {
                             alive = false;
                             continue;

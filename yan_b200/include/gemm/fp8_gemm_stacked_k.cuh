@@ -102,11 +102,20 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
         // the kernel behind this one may start: its own allocation cannot get in front of this grid's any more
         if (order != kConstantWeights) ptx::grid_dependency_launch_dependents();
     }
-    const uint32_t slot = lane_idx / kStack, part = lane_idx % kStack;
-    const uint32_t group_mask = ((1u << kStack) - 1u) << (slot * kStack);  // the producer lanes of a slot
-    uint8_t* w_dst = smem + L.off_w + slot * 16384u + part * (kRows * 128u);
-    uint8_t* x_dst = smem + L.off_x + slot * (kMmaN * 128u) + part * (M_PAD * 128u);
-    const uint32_t kb_lane = (part0 + part) * steps;
+    // the operands of step s, slot by slot: a box per k-part
+    auto load_weights = [&](const uint32_t slot, const uint32_t s) {
+        ptx::mbar_arrive_expect_tx(full_barriers + slot, kStepBytes);
+#pragma unroll
+        for (uint32_t part = 0; part < kStack; ++part)
+            ptx::tma_load_2d(smem + L.off_w + slot * 16384u + part * (kRows * 128u), &tensor_map_w, full_barriers + slot,
+                             static_cast<int32_t>(((part0 + part) * steps + s) * kBlockK), static_cast<int32_t>(n0));
+    };
+    auto load_activations = [&](const uint32_t slot, const uint32_t s) {
+#pragma unroll
+        for (uint32_t part = 0; part < kStack; ++part)
+            ptx::tma_load_2d(smem + L.off_x + slot * (kMmaN * 128u) + part * (M_PAD * 128u), &tensor_map_x, full_barriers + slot,
+                             static_cast<int32_t>(((part0 + part) * steps + s) * kBlockK), 0);
+    };
     if (warp_idx == 4) {
         if (lane_idx == 0) {
             ptx::tma_prefetch_desc(&tensor_map_w);
@@ -126,11 +135,10 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
             ptx::fence_proxy_async_smem();
         }
         __syncwarp();
-        if (slot < kSlots && slot < steps) {
-            if (part == 0) ptx::mbar_arrive_expect_tx(full_barriers + slot, kStepBytes);
-            __syncwarp(group_mask);
-            ptx::tma_load_2d(w_dst, &tensor_map_w, full_barriers + slot, static_cast<int32_t>((kb_lane + slot) * kBlockK),
-                             static_cast<int32_t>(n0));
+        if (ptx::elect_one()) {
+#pragma unroll
+            for (uint32_t slot = 0; slot < kSlots; ++slot)
+                if (slot < steps) load_weights(slot, slot);
         }
         __syncwarp();
     }
@@ -141,40 +149,41 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
 
     if (warp_idx == 4) {
         ptx::grid_dependency_wait();
-        if (slot < kSlots) {
-            if (slot < steps)
-                ptx::tma_load_2d(x_dst, &tensor_map_x, full_barriers + slot, static_cast<int32_t>((kb_lane + slot) * kBlockK), 0);
+        if (ptx::elect_one()) {
+#pragma unroll
+            for (uint32_t slot = 0; slot < kSlots; ++slot)
+                if (slot < steps) load_activations(slot, slot);
             // refills: the slot is free again when the MMAs of the step it held are complete
-            for (uint32_t s = slot + kSlots; s < steps; s += kSlots) {
-                const uint32_t it = s / kSlots;
-                bool ok = detail::bounded_wait(empty_barriers + slot, (it - 1) & 1, abort_flag, p, 7);
-                ok = __all_sync(group_mask, ok);
-                if (!ok) break;
-                if (part == 0) ptx::mbar_arrive_expect_tx(full_barriers + slot, kStepBytes);
-                __syncwarp(group_mask);
-                ptx::tma_load_2d(w_dst, &tensor_map_w, full_barriers + slot, static_cast<int32_t>((kb_lane + s) * kBlockK),
-                                 static_cast<int32_t>(n0));
-                ptx::tma_load_2d(x_dst, &tensor_map_x, full_barriers + slot, static_cast<int32_t>((kb_lane + s) * kBlockK), 0);
-            }
+            uint32_t pos = 0, phase = 0, s = kSlots;
+            if (steps > kSlots)
+                ring_steps<kSlots>(pos, steps - kSlots, [&](const uint32_t slot) {
+                    if (!detail::bounded_wait(empty_barriers + slot, phase, abort_flag, p, 7)) return false;
+                    load_weights(slot, s);
+                    load_activations(slot, s);
+                    ++s;
+                    if (slot + 1 == kSlots) phase ^= 1;
+                    return true;
+                });
         }
         __syncwarp();
     } else if (warp_idx == 5) {
-        if (lane_idx == 0) {
+        if (ptx::elect_one()) {
             constexpr uint32_t idesc = make_instr_desc_e4m3_f32(128, kMmaN);
-            for (uint32_t s = 0; s < steps; ++s) {
-                const uint32_t r = s % kSlots, b = s % kTmemSlots, b_it = s / kTmemSlots;
-                if (!detail::bounded_wait(full_barriers + r, (s / kSlots) & 1, abort_flag, p, 5)) break;
-                if (b_it > 0 && !detail::bounded_wait(tmem_empty_barriers + b, (b_it - 1) & 1, abort_flag, p, 8)) break;
+            const uint32_t w_low = make_smem_desc_low(ptx::smem_u32(smem + L.off_w)), x_low = make_smem_desc_low(ptx::smem_u32(smem + L.off_x));
+            uint32_t pos = 0, phase = 0, buf_phase = 0, left = steps;
+            ring_steps<common_round(kSlots, kTmemSlots)>(pos, steps, [&](const uint32_t u) {
+                const uint32_t r = u % kSlots, b = u % kTmemSlots;
+                if (!detail::bounded_wait(full_barriers + r, phase, abort_flag, p, 5)) return false;
+                if (!detail::bounded_wait(tmem_empty_barriers + b, buf_phase ^ 1, abort_flag, p, 8)) return false;
                 ptx::tcgen05_fence_after_thread_sync();
-                const uint64_t w_desc = make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L.off_w + r * 16384u));
-                const uint64_t x_desc = make_smem_desc_k_major_sw128(ptx::smem_u32(smem + L.off_x + r * (kMmaN * 128u)));
-#pragma unroll
-                for (uint32_t k = 0; k < kBlockK / kUmmaK; ++k)
-                    ptx::umma_f8f6f4_ss(tmem_base + b * kMmaN, w_desc + k * kDescKStep, x_desc + k * kDescKStep, idesc,
-                                        k > 0);
+                umma_k_block(tmem_base + b * kMmaN, w_low + r * (16384u >> 4), x_low + r * (kMmaN * 128u >> 4), idesc);
                 ptx::umma_commit(done_barriers + b);
-                if (!kOneRing && s + kSlots < steps) ptx::umma_commit(empty_barriers + r);
-            }
+                if (!kOneRing && left > kSlots) ptx::umma_commit(empty_barriers + r);
+                --left;
+                if (r + 1 == kSlots) phase ^= 1;
+                if (b + 1 == kTmemSlots) buf_phase ^= 1;
+                return true;
+            });
         }
         __syncwarp();
         // the promotion warps have read the last accumulator, or a role gave up: then loads and products may be in flight

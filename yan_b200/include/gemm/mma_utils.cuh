@@ -7,6 +7,7 @@
 
 #include <cstdint>
 
+#include "ptx.cuh"
 #include "utils.cuh"
 
 namespace yan {
@@ -41,16 +42,16 @@ __host__ __device__ constexpr uint32_t get_num_threads_per_sm(uint32_t block_n) 
 // setmaxnreg.inc draws from is what the CTA was given at launch (registers per thread at launch x threads),
 // NOT the whole register file: an increase that the control warpgroup's decrease does not cover blocks
 // forever.  Launch allocation = floor(65536 / threads / 8) * 8 registers per thread.
-//   2 math warpgroups: launch 168 x 384; 128*40 + 256*232 = 64512 = 168*384
+//   2 math warpgroups: launch 168 x 384; 128*40 + 256*232 = 128*136 + 256*184 = 64512 = 168*384
 //   4 math warpgroups: launch  96 x 640; 128*32 + 512*112 = 61440 =  96*640
 __host__ __device__ constexpr uint32_t get_num_launch_registers(uint32_t block_n) {
     return (65536u / get_num_threads_per_sm<>(block_n)) / 8u * 8u;
 }
 __host__ __device__ constexpr uint32_t get_num_control_registers(uint32_t block_n) {
-    return get_num_math_warpgroups(block_n) == 4 ? 32 : 40;
+    return get_num_math_warpgroups(block_n) == 4 ? 32 : block_n <= 160 ? 136 : 40;
 }
 __host__ __device__ constexpr uint32_t get_num_math_registers(uint32_t block_n) {
-    return get_num_math_warpgroups(block_n) == 4 ? 112 : 232;
+    return get_num_math_warpgroups(block_n) == 4 ? 112 : block_n <= 160 ? 184 : 232;
 }
 
 template <uint32_t BLOCK_N>
@@ -94,5 +95,40 @@ __device__ __forceinline__ uint64_t make_smem_desc_k_major_sw128(uint32_t smem_a
 // 32 >> 4 = 2 to the start-address field.
 constexpr uint32_t kUmmaK = 32;
 constexpr uint32_t kDescKStep = (kUmmaK * 1) >> 4;
+
+// The same descriptor in halves: the high word never changes, the low word is the address.
+constexpr uint32_t kDescHigh = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t make_smem_desc_low(uint32_t smem_addr) { return ((smem_addr & 0x3FFFFu) >> 4) | (1u << 16); }
+
+// The products of one 128-wide k-block, overwriting the accumulator.
+__device__ __forceinline__ void umma_k_block(uint32_t tmem_d, uint32_t desc_a_low, uint32_t desc_b_low, uint32_t idesc) {
+#pragma unroll
+    for (uint32_t k = 0; k < kBlockK / kUmmaK; ++k)
+        ptx::umma_f8f6f4_ss_low<kDescHigh>(tmem_d, desc_a_low + k * kDescKStep, desc_b_low + k * kDescKStep, idesc, k > 0);
+}
+
+// `count` steps of a loop over rings of operand stages and accumulators, continued at position `pos` of a round of kRound steps
+// (a common multiple of the rings).  step(u) gets its position as a constant, so that every descriptor, barrier and tensor
+// memory address is a constant from a base; it returns false to give up.
+// What bounds narrow tiles is the one thread that issues: 512 steps of a 128 x 32 (x 64) tile with one wait and one commit each
+// took 495 (495) cycles per step with a running stage index behind `lane == 0`, 311 (319) behind elect_one, 195 (221) unrolled;
+// the products alone take 161 (193).
+template <uint32_t kRound, typename Step>
+__device__ __forceinline__ bool ring_steps(uint32_t& pos, uint32_t count, Step&& step) {
+    while (count != 0) {
+#pragma unroll
+        for (uint32_t u = 0; u < kRound; ++u) {
+            if (u >= pos && count != 0) {
+                if (!step(u)) return false;
+                --count;
+                pos = u + 1;
+            }
+        }
+        if (pos == kRound) pos = 0;
+    }
+    return true;
+}
+
+constexpr uint32_t common_round(uint32_t a, uint32_t b) { return a / constexpr_gcd(a, b) * b; }
 
 }  // namespace yan

@@ -65,7 +65,7 @@ def get_smem_size(block_n: int, num_stages: int) -> int:
     slots = num_stages + num_tmem_bufs + 1
     if ring + store + slots * 528 + 2048 > 232448:
         slots = 0
-    return ring + store + slots * 528 + (2 * num_stages + 4 * num_tmem_bufs + slots) * 8 + 8 + 1024
+    return ring + store + slots * 528 + (2 * (num_stages + num_tmem_bufs) + slots) * 8 + 8 + 1024
 
 
 # start, time per k-block and epilogue of a wave of tiles, in us (measured; see choose_block_n in csrc/capi.cu)
