@@ -50,6 +50,19 @@ enum StackedOrder : uint32_t {
                               // once, tensor memory is taken after the wait
 };
 
+// Adds kCols floats of shared memory; false where they come from a thread that gave up.
+template <uint32_t kCols>
+__device__ __forceinline__ bool add_row_piece(float (&v)[kCols], uint32_t smem_addr) {
+    bool complete = true;
+#pragma unroll
+    for (uint32_t i = 0; i < kCols; i += 4) {
+        const float4 t = ptx::ld_shared_v4_f32(smem_addr + i * 4u);
+        if (i == 0) complete = detail::is_complete(t.x);
+        v[i] += t.x, v[i + 1] += t.y, v[i + 2] += t.z, v[i + 3] += t.w;
+    }
+    return complete;
+}
+
 template <uint32_t M_PAD, uint32_t kStack, uint32_t kSlots, uint32_t kTmemSlots = stacked_k_tmem_slots(kSlots)>
 __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <= 256 ? 2 : 1)
     fp8_gemm_stacked_k_kernel(const GemmParams p, const __grid_constant__ CUtensorMap tensor_map_w,
@@ -195,19 +208,31 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
 
     // Promotion warps: TMEM lane 32 * warp + lane = (k-part q, weight row n0 + r)
     const uint32_t q = warp_idx / kWarpsPerPart, r_local = (warp_idx % kWarpsPerPart) * 32 + lane_idx;
-    // The final sums: thread (j0, rr) finishes activation rows j0 * kMPerThread + [0, kMPerThread) of weight row n0 + rr.
-    constexpr uint32_t kMPerThread = M_PAD / kStack;
-    const uint32_t rr = threadIdx.x % kRows, m0 = threadIdx.x / kRows * kMPerThread;
-    float v[kMPerThread];
+    // The final sums: an item is kCols neighbouring columns of one activation row, so that a row leaves in whole pieces of 64
+    // or 128 bytes (a thread that finished a column stored 2 bytes of every row: M=64 N=7168 K=2048 1.05 us for 64 x 64 values).
+    constexpr uint32_t kCols = M_PAD == 16 ? 4 : 8, kItems = M_PAD * (kRows / kCols) / 128;
+    const uint32_t m_first = threadIdx.x / (kRows / kCols), col = threadIdx.x % (kRows / kCols) * kCols;
+    constexpr uint32_t kItemRows = 128 / (kRows / kCols);  // item j of a thread: activation row m_first + j * kItemRows
+    float v[kItems][kCols];
     bool alive = true;
     if (warp_idx < 4) {
         // Fold both scale factors of every (k-part, step, row) while the weights stream in.
         const float* sb_ptr = p.scales_b + static_cast<size_t>(n0 / 128u) * num_k_blocks;
         ptx::grid_dependency_wait();
-        for (uint32_t i = threadIdx.x; i < kStack * steps * M_PAD; i += 128) {
-            const uint32_t m = i % M_PAD, kb = part0 * steps + i / M_PAD;
-            const bool ok = m < p.shape_m && kb < num_k_blocks;
-            s_scales[i] = ok ? __ldg(p.scales_a + static_cast<size_t>(kb) * p.sa_ld + m) * __ldg(sb_ptr + kb) : 0.0f;
+        // eight of each in flight: one after the other they took longer than the weights (M=1 N=4096 K=7168: 1.3 us behind them)
+        const uint32_t num_scales = kStack * steps * M_PAD;
+        for (uint32_t first = threadIdx.x; first < num_scales; first += 8 * 128) {
+            float sa[8], sb[8];
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j) {
+                const uint32_t i = first + j * 128, m = i % M_PAD, kb = part0 * steps + i / M_PAD;
+                const bool ok = i < num_scales && m < p.shape_m && kb < num_k_blocks;
+                sa[j] = ok ? __ldg(p.scales_a + static_cast<size_t>(kb) * p.sa_ld + m) : 0.0f;
+                sb[j] = ok ? __ldg(sb_ptr + kb) : 0.0f;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < 8; ++j)
+                if (first + j * 128 < num_scales) s_scales[first + j * 128] = sa[j] * sb[j];
         }
         ptx::named_barrier_sync(1, 128);
         // the useful columns of a step are [slot * kMmaN + q * M_PAD, +M_PAD)
@@ -222,7 +247,7 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
             alive = __all_sync(0xffffffffu, ok);
             if (alive) {
                 ptx::tcgen05_fence_after_thread_sync();
-                const float* sc = s_scales + (q * steps + s) * M_PAD;
+                const uint32_t sc = ptx::smem_u32(s_scales) + (q * steps + s) * (M_PAD * 4u);
 #pragma unroll
                 for (uint32_t c = 0; c < M_PAD / kChunk; ++c) {
                     uint32_t t[kChunk];
@@ -234,8 +259,12 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
                         if (lane_idx == 0) ptx::mbar_arrive(tmem_empty_barriers + b);  // the accumulator slot may be overwritten
                     }
 #pragma unroll
-                    for (uint32_t m = 0; m < kChunk; ++m)
-                        acc[c * kChunk + m] = fmaf(sc[c * kChunk + m], __uint_as_float(t[m]), acc[c * kChunk + m]);
+                    for (uint32_t m = 0; m < kChunk; m += 4) {
+                        const float4 f = ptx::ld_shared_v4_f32(sc + (c * kChunk + m) * 4u);
+                        float* a = acc + c * kChunk + m;
+                        ptx::fma_f32x2(a[0], a[1], t[m], t[m + 1], f.x, f.y);
+                        ptx::fma_f32x2(a[2], a[3], t[m + 2], t[m + 3], f.z, f.w);
+                    }
                 }
             }
         }
@@ -247,41 +276,64 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
 #pragma unroll
         for (uint32_t m = 0; m < M_PAD; ++m) s_reduce[(q * M_PAD + m) * kRows + r_local] = acc[m];
         ptx::named_barrier_sync(1, 128);
-        const uint32_t base = ptx::smem_u32(s_reduce) + rr * 4u;
+        if (rank == 0) {
+            const uint32_t base = ptx::smem_u32(s_reduce) + (m_first * kRows + col) * 4u;
 #pragma unroll
-        for (uint32_t j = 0; j < kMPerThread; ++j) {
-            v[j] = 0.0f;
+            for (uint32_t j = 0; j < kItems; ++j) {
 #pragma unroll
-            for (uint32_t qq = 0; qq < kStack; ++qq) v[j] += ptx::ld_shared_f32(base + ((qq * M_PAD + m0 + j) * kRows) * 4u);
+                for (uint32_t i = 0; i < kCols; ++i) v[j][i] = 0.0f;
+#pragma unroll
+                for (uint32_t qq = 0; qq < kStack; ++qq)
+                    add_row_piece(v[j], base + (qq * M_PAD + j * kItemRows) * (kRows * 4u));
+            }
         }
     }
-    const uint32_t exchange = ptx::smem_u32(smem + L.off_exchange) + rr * 4u;
     if (cluster > 1) {
         __syncwarp();
         ptx::cluster_wait();
         if (warp_idx < 4 && rank != 0) {
-            if (*abort_flag != 0) v[0] = __uint_as_float(detail::kGaveUpSum);
-            const uint32_t remote = ptx::map_to_cta(exchange + (rank - 1) * (M_PAD * kRows * 4u), 0);
+            // a warp sends 128 contiguous bytes at a time (16 per lane were slower: M=32 N=2048 K=7168 7.85 us against 7.3)
+            const bool gave_up = *abort_flag != 0;
+            const uint32_t base = ptx::smem_u32(s_reduce) + threadIdx.x * 4u;
+            const uint32_t remote = ptx::map_to_cta(ptx::smem_u32(smem + L.off_exchange) + (rank - 1) * (M_PAD * kRows * 4u), 0) + threadIdx.x * 4u;
 #pragma unroll
-            for (uint32_t j = 0; j < kMPerThread; ++j) ptx::st_cluster_f32(remote + (m0 + j) * (kRows * 4u), v[j]);
+            for (uint32_t j = 0; j < M_PAD * kRows / 128; ++j) {
+                float sum = 0.0f;
+#pragma unroll
+                for (uint32_t qq = 0; qq < kStack; ++qq) sum += ptx::ld_shared_f32(base + (qq * M_PAD * kRows + j * 128u) * 4u);
+                ptx::st_cluster_f32(remote + j * 512u, gave_up ? __uint_as_float(detail::kGaveUpSum) : sum);
+            }
         }
         ptx::cluster_arrive();
         ptx::cluster_wait();
     }
     if (warp_idx < 4 && rank == 0 && alive && *abort_flag == 0) {
+        const uint32_t exchange = ptx::smem_u32(smem + L.off_exchange) + (m_first * kRows + col) * 4u;
         for (uint32_t c = 0; c + 1 < cluster; ++c) {
 #pragma unroll
-            for (uint32_t j = 0; j < kMPerThread; ++j) {
-                const float sum = ptx::ld_shared_f32(exchange + (c * M_PAD + m0 + j) * (kRows * 4u));
-                if (j == 0) alive = alive && detail::is_complete(sum);
-                v[j] += sum;
-            }
+            for (uint32_t j = 0; j < kItems; ++j)
+                alive = add_row_piece(v[j], exchange + (c * M_PAD + j * kItemRows) * (kRows * 4u)) && alive;
         }
-        if (alive && n0 + rr < p.shape_n) {
-            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + n0 + rr;
+        if (alive && n0 + col < p.shape_n) {  // N % 16 == 0: a piece is inside or outside as a whole
+            __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<size_t>(m_first) * p.ldd + n0 + col;
+            const bool whole = reinterpret_cast<uintptr_t>(p.out) % 16 == 0 && p.ldd % 8 == 0;
 #pragma unroll
-            for (uint32_t j = 0; j < kMPerThread; ++j)
-                if (m0 + j < p.shape_m) out[static_cast<size_t>(m0 + j) * p.ldd] = __float2bfloat16_rn(v[j]);
+            for (uint32_t j = 0; j < kItems; ++j, out += static_cast<size_t>(kItemRows) * p.ldd) {
+                if (m_first + j * kItemRows >= p.shape_m) break;
+                uint32_t w[kCols / 2];
+#pragma unroll
+                for (uint32_t i = 0; i < kCols / 2; ++i) {
+                    const __nv_bfloat162 t = __floats2bfloat162_rn(v[j][2 * i], v[j][2 * i + 1]);
+                    w[i] = *reinterpret_cast<const uint32_t*>(&t);
+                }
+                if (whole) {
+                    if constexpr (kCols == 8) *reinterpret_cast<uint4*>(out) = make_uint4(w[0], w[1], w[2], w[3]);
+                    else *reinterpret_cast<uint2*>(out) = make_uint2(w[0], w[1]);
+                } else {  // an output that is only known to start on an element
+#pragma unroll
+                    for (uint32_t i = 0; i < kCols; ++i) out[i] = __float2bfloat16_rn(v[j][i]);
+                }
+            }
         }
     }
 #endif

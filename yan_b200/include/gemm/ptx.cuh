@@ -359,6 +359,20 @@ __device__ __forceinline__ void fma_f32x2(float& acc0, float& acc1, uint32_t t0,
         : "r"(t0), "r"(t1), "f"(scale));
 }
 
+// acc_i = fma(t_i, scale_i, acc_i)
+__device__ __forceinline__ void fma_f32x2(float& acc0, float& acc1, uint32_t t0, uint32_t t1, float scale0, float scale1) {
+    asm("{\n\t"
+        ".reg .b64 a, t, s;\n\t"
+        "mov.b64 a, {%0, %1};\n\t"
+        "mov.b64 t, {%2, %3};\n\t"
+        "mov.b64 s, {%4, %5};\n\t"
+        "fma.rn.f32x2 a, t, s, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t"
+        "}\n"
+        : "+f"(acc0), "+f"(acc1)
+        : "r"(t0), "r"(t1), "f"(scale0), "f"(scale1));
+}
+
 // bar.sync on a named barrier: the first `count` threads' worth of warps that reach it (count % 32 == 0).
 __device__ __forceinline__ void named_barrier_sync(uint32_t id, uint32_t count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
