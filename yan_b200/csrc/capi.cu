@@ -158,9 +158,7 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        const yan::StackedOrder order = g_programmatic_launch != 0 ? yan::kConstantWeights
-                                        : after_own_quantizer     ? yan::kAfterOwnQuantizer
-                                                                  : yan::kAfterAnyKernel;
+        const yan::StackedOrder order = g_programmatic_launch != 0 ? yan::kConstantWeights : yan::kAfterAnyKernel;
         const bool small_m_ok = yan::small_m_supported(a.m, a.n, a.k, max_smem);
         const bool stacked_ok = yan::stacked_k_supported(a.m, a.n, a.k);
         if (block_n == 2) return stacked_ok ? yan::launch_fp8_gemm_stacked_k(a, s, order) : yan::kBadArgument;
@@ -174,7 +172,7 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
             return yan::launch_fp8_gemm_stacked_k(a, s, order);
         if (block_n == 1 || (want_auto && !general_ok && small_m_ok)) {
             if (!small_m_ok) return yan::kBadArgument;
-            return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || after_own_quantizer);
+            return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || (after_own_quantizer && block_n == 1));
         }
         // what the general kernel is the default for, with an output that it does not take
         if (want_auto && !general_ok && any_output) return yan::launch_fp8_gemm_stacked_k(a, s, order);
@@ -210,9 +208,12 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
 
 bool positive(int a, int b, int c) { return a > 0 && b > 0 && c > 0; }
 
-// The GEMM of a quantize-then-GEMM call.  Its predecessor in the stream is this library's own quantizer, which never
-// writes weights, so the weight-streaming kernel (M <= 64) is always launched with programmatic stream serialization
-// here: its weight loads run while the quantizer does, and it waits for the quantizer before reading the activations.
+// Whether the quantizer of a quantize-then-GEMM call lets the GEMM start before it has waited for the kernel in front.  Every GEMM
+// waits for the quantizer before it reads anything, except the pair kernel (block_n = 1), which loads its weights first: it has to
+// start behind whatever wrote them, unless the caller has promised that nothing did.
+bool release_early(int block_n) { return block_n != 1 || g_programmatic_launch != 0; }
+
+// The GEMM of a quantize-then-GEMM call, behind this library's own quantizer in the stream.
 int gemm_after_quantizer(const void* q, const float* scales, const void* rhs, const void* rhs_scales, void* out, int m,
                          int n, int k, int ldd, void* stream, int num_sms, int block_n) {
     if (ldd <= 0) return yan::kBadArgument;
@@ -406,7 +407,7 @@ YAN_EXPORT void yan_b200_fp8_linear_bf16(const void* a, const void* rhs, const v
     uint8_t* q = static_cast<uint8_t*>(workspace);
     float* scales = reinterpret_cast<float*>(q + yan::align_up(static_cast<size_t>(m) * k, static_cast<size_t>(256)));
     int rc = yan::launch_per_token_cast_to_fp8(a, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
-                                               g_programmatic_launch != 0);
+                                               release_early(block_n));
     if (rc != yan::kOk) return set_rc(return_code, rc);
     set_rc(return_code, gemm_after_quantizer(q, scales, rhs, rhs_scales, out, m, n, k, ldd, stream, num_sms, block_n));
 }
@@ -423,7 +424,7 @@ YAN_EXPORT void yan_b200_fp8_linear_bf16_static(const void* a, const void* rhs, 
     uint8_t* q = scratch;
     float* scales = reinterpret_cast<float*>(scratch + kStaticScratchQBytes);
     const int rc = yan::launch_per_token_cast_to_fp8(a, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
-                                                     g_programmatic_launch != 0);
+                                                     release_early(block_n));
     if (rc != yan::kOk) return set_rc(return_code, rc);
     set_rc(return_code, gemm_after_quantizer(q, scales, rhs, rhs_scales, out, m, n, k, ldd, stream, num_sms, block_n));
 }

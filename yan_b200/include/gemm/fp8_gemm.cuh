@@ -36,6 +36,7 @@ struct GemmParams {
     const float* scales_a;      // [K/128][sa_ld], element (kb, row) at kb * sa_ld + row
     const float* scales_b;      // [groups][ceil(N/128)][K/128]
     const int* grouped_layout;  // Contiguous: [M] group per row (-1 = padding); Masked: [G] valid rows
+    const uint8_t* weights = nullptr;  // the B operand, for prefetches (it is read through its tensor map)
     void* out;                  // [rows][ldd]
     float* out_scales;          // e4m3 output only: [N/128][out_scales_ld], element (nb, row) at nb * out_scales_ld + row
     uint32_t out_scales_ld;
@@ -475,9 +476,6 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
         }
     };
 
-    // A whole-tile launch that is followed by a tail launch lets that one be scheduled at once: its CTAs take the SMs as
-    // this kernel's CTAs leave them (they read operands and write scratch only, nothing this kernel produces).
-    if (!kTail && p.tile_limit != 0) ptx::grid_dependency_launch_dependents();
     if (warp_idx == 0 && lane_idx == 0) {
         ptx::tma_prefetch_desc(&tensor_map_a);
         ptx::tma_prefetch_desc(&tensor_map_b);
@@ -501,14 +499,38 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
     }
-    if (warp_idx == 2) {
-        ptx::tmem_alloc(tmem_slot, L::kTmemCols);
-        ptx::tmem_relinquish_alloc_permit();
+    if constexpr (kGemmType == GemmType::Normal && !kTail && kUnrolledIssue) {
+        // the weights of the first k-blocks on their way to L2 while the kernel in front ends
+        if (warp_idx == 3) {
+            Sched sched(p.shape_m, p.shape_n);
+            uint32_t m_block_idx, n_block_idx;
+            sched.swizzle(kCutK ? p.tail_first_tile + tail_tile : blockIdx.x, sched.num_m_blocks, m_block_idx, n_block_idx);
+            const uint32_t n = n_block_idx * BLOCK_N + lane_idx;
+            const uint8_t* w = p.weights + static_cast<size_t>(n) * p.shape_k + static_cast<size_t>(kb_begin) * kBlockK;
+            for (uint32_t r = 0; r < BLOCK_N && n + r < p.shape_n; r += 32, w += static_cast<size_t>(32) * p.shape_k)
+                for (uint32_t i = 0; i < kNumStages && i < kb_count; ++i) ptx::prefetch_l2(w + i * kBlockK);
+        }
     }
-    ptx::tcgen05_fence_before_thread_sync();
-    __syncthreads();
-    ptx::tcgen05_fence_after_thread_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    __syncthreads();  // the barriers are initialized
+    // Up to here this kernel may run beside the one in front (see GemmLauncher).  (The tail instance reads operands and writes
+    // scratch, nothing that the whole-tile kernel in front of it produces: it waits at its end.)
+    if constexpr (!kTail) ptx::grid_dependency_wait();
+    uint32_t tmem_base = 0;
+    if (warp_idx != 0 && warp_idx != 3) {
+        if (warp_idx == 2) {
+            // After the wait: the kernel in front may still have had tensor memory to take.
+            ptx::tmem_alloc(tmem_slot, L::kTmemCols);
+            ptx::tmem_relinquish_alloc_permit();
+            // Only the kernels that finish this one's last wave (kTail) start before it ends: their CTAs take the SMs as this kernel's
+            // leave them.  Any other would crowd the SMs that are free first (a quantizer, eight CTAs to an SM: M=2048 N=4096
+            // K=1024 with quantizer 15.7 -> 17.1 us); it starts when all CTAs have ended, its launch overlapping their end.
+            if (kTail || p.tile_limit != 0) ptx::grid_dependency_launch_dependents();
+        }
+        ptx::tcgen05_fence_before_thread_sync();
+        ptx::named_barrier_sync(3, kNumMathWarps * 32 + 64);
+        ptx::tcgen05_fence_after_thread_sync();
+        tmem_base = *tmem_slot;
+    }
     if (p.clock_probe != nullptr && blockIdx.x == 0 && threadIdx.x == 0) {
         p.clock_probe[0] = clock64();
         p.clock_probe[1] = static_cast<long long>(ptx::globaltimer_ns());
@@ -960,8 +982,7 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
     // Every role has left its loop (normally or through the bounded-wait path): free tensor memory.
     if constexpr (kTail) {
         // launched programmatically behind the whole-tile kernel: do not complete before that kernel has (the kernel
-        // that sums the partials waits for this one only), and let that kernel be scheduled now
-        ptx::grid_dependency_launch_dependents();
+        // that sums the partials waits for this one only)
         ptx::grid_dependency_wait();
     }
     ptx::tcgen05_fence_before_thread_sync();
@@ -1061,6 +1082,9 @@ __global__ void __launch_bounds__(256) reduce_tail_partials_kernel(const float* 
     *reinterpret_cast<uint4*>(out + static_cast<size_t>(out_row) * ldd + out_col) = v;
 }
 
+// k-blocks per CTA up to which a launch overlaps the end of the kernel in front (see GemmLauncher).
+constexpr uint64_t kOverlapMaxKBlocks = 64;
+
 inline bool is_aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }
 
 // Host-side checks of a launch (smem_size: what its kernel needs) and its device-side parameters.
@@ -1099,6 +1123,7 @@ inline int check_and_fill(const GemmArgs& a, GemmType type, uint32_t out_bytes, 
     p.scales_a = a.lhs_scales;
     p.scales_b = a.rhs_scales;
     p.grouped_layout = a.grouped_layout;
+    p.weights = static_cast<const uint8_t*>(a.rhs);
     p.out = a.out;
     p.out_scales = a.out_scales;
     p.out_scales_ld = a.out_scales_ld;
@@ -1111,6 +1136,35 @@ inline int check_and_fill(const GemmArgs& a, GemmType type, uint32_t out_bytes, 
     p.status = a.status;
     p.timeout_ns = a.timeout_ns;
     p.clock_probe = a.clock_probe;
+    return kOk;
+}
+
+// Launches clusters of `cluster` CTAs; `programmatic`: with programmatic stream serialization (every GEMM kernel waits for the one
+// in front of it by itself).
+template <typename... Params, typename... Args>
+inline int launch_kernel(void (*kernel)(Params...), dim3 grid, uint32_t threads, uint32_t smem_bytes, cudaStream_t stream,
+                         uint32_t cluster, bool programmatic, const Args&... args) {
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem_bytes;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    if (programmatic) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = 1;
+        attr[cfg.numAttrs++].val.clusterDim.z = 1;
+    }
+    if (cudaLaunchKernelEx(&cfg, kernel, args...) != cudaSuccess) {
+        cudaGetLastError();
+        return kLaunchFailed;
+    }
     return kOk;
 }
 
@@ -1141,6 +1195,12 @@ struct GemmLauncher {
             const uint32_t tiles = ceil_div(a.m, kBlockM) * ceil_div(a.n, BLOCK_N);
             grid = tiles < grid ? tiles : grid;
         }
+        // Started while the kernel in front ends, the CTAs go to the SMs in the order in which these become free, and neighbours in
+        // the tile order, which share operands, no longer sit next to each other: a launch of many k-blocks loses more to that
+        // than the two microseconds it saves (M=8192 N=28672 K=8192 behind its quantizer 1912 -> 1997 us; M=4096 N=7168 K=18432
+        // 544 -> 553; M=1111 N=5136 K=3072, 48 k-blocks per CTA, 26.6 -> 25.6; M=256 N=1024 K=1024 with quantizer 8.2 -> 5.8).
+        const uint64_t all_tiles = ceil_div(a_rows, static_cast<uint64_t>(kBlockM)) * ceil_div(a.n, BLOCK_N);
+        const bool overlap = ceil_div(all_tiles, static_cast<uint64_t>(grid)) * (a.k / kBlockK) <= kOverlapMaxKBlocks;
         if constexpr (kGemmType == GemmType::Normal && sizeof(out_t) == 2 && L::kStoreBytes != 0) {
             if (a.scatter_world != 0) {
                 // only the widths whose epilogue goes through the staging boxes know the owners' staging arrays
@@ -1162,8 +1222,7 @@ struct GemmLauncher {
                     cudaGetLastError();
                     return kSmemTooLarge;
                 }
-                scatter_kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), kScatterSmem, stream>>>(p, map_a, map_b);
-                return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+                return launch_kernel(scatter_kernel, grid, get_num_threads_per_sm<>(BLOCK_N), kScatterSmem, stream, 1, overlap, p, map_a, map_b);
             }
         } else {
             if (a.scatter_world != 0) return kBadArgument;
@@ -1181,7 +1240,9 @@ struct GemmLauncher {
                     return kSmemTooLarge;
                 }
                 p.tile_limit = tiles - rest;
-                kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), kSmemSize, stream>>>(p, map_a, map_b);
+                constexpr uint32_t kThreads = get_num_threads_per_sm<>(BLOCK_N);
+                int launched = launch_kernel(kernel, grid, kThreads, kSmemSize, stream, 1, overlap, p, map_a, map_b);
+                if (launched != kOk) return launched;
                 GemmParams tail = p;
                 tail.tile_limit = 0;
                 tail.out = a.tail_workspace;
@@ -1189,34 +1250,15 @@ struct GemmLauncher {
                 tail.tail_tiles = rest;
                 tail.tail_slices = slices;
                 tail.clock_probe = nullptr;
-                // both follow-up kernels are launched with programmatic stream serialization: the launch latencies
-                // hide behind the kernel before; ordering is kept by the waits inside them
-                cudaLaunchAttribute attr[1];
-                attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-                attr[0].val.programmaticStreamSerializationAllowed = 1;
-                cudaLaunchConfig_t cfg = {};
-                cfg.gridDim = dim3(rest * slices);
-                cfg.blockDim = dim3(get_num_threads_per_sm<>(BLOCK_N));
-                cfg.dynamicSmemBytes = kSmemSize;
-                cfg.stream = stream;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                if (cudaLaunchKernelEx(&cfg, tail_kernel, tail, map_a, map_b) != cudaSuccess) {
-                    cudaGetLastError();
-                    return kLaunchFailed;
-                }
-                cfg.gridDim = dim3(rest, kBlockM * (BLOCK_N / 8) / 256);
-                cfg.blockDim = dim3(256);
-                cfg.dynamicSmemBytes = 0;
+                // the launch latencies of the two follow-up kernels hide behind the kernel before; ordering is kept by the waits
+                // inside them
+                launched = launch_kernel(tail_kernel, rest * slices, kThreads, kSmemSize, stream, 1, true, tail, map_a, map_b);
+                if (launched != kOk) return launched;
                 const float* partials = static_cast<const float*>(a.tail_workspace);
                 __nv_bfloat16* out_bf16 = static_cast<__nv_bfloat16*>(a.out);
                 const uint32_t first_tile = tiles - rest;
-                if (cudaLaunchKernelEx(&cfg, reduce_tail_partials_kernel<BLOCK_N>, partials, out_bf16, a.ldd, a.m, a.n,
-                                       first_tile, rest, slices) != cudaSuccess) {
-                    cudaGetLastError();
-                    return kLaunchFailed;
-                }
-                return kOk;
+                return launch_kernel(reduce_tail_partials_kernel<BLOCK_N>, dim3(rest, kBlockM * (BLOCK_N / 8) / 256), 256, 0, stream, 1,
+                                     true, partials, out_bf16, a.ldd, a.m, a.n, first_tile, rest, slices);
             }
         }
         // fp32 output on 256-wide tiles: 128-byte box rows halve the passes of the epilogue but leave no room for the ring of
@@ -1232,13 +1274,12 @@ struct GemmLauncher {
                         cudaGetLastError();
                         return kSmemTooLarge;
                     }
-                    wide_kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), Wide::kSmemSize, stream>>>(p, map_a, map_b);
-                    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+                    return launch_kernel(wide_kernel, grid, get_num_threads_per_sm<>(BLOCK_N), Wide::kSmemSize, stream, 1, overlap, p,
+                                         map_a, map_b);
                 }
             }
         }
-        kernel<<<grid, get_num_threads_per_sm<>(BLOCK_N), kSmemSize, stream>>>(p, map_a, map_b);
-        return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+        return launch_kernel(kernel, grid, get_num_threads_per_sm<>(BLOCK_N), kSmemSize, stream, 1, overlap, p, map_a, map_b);
     }
 };
 
@@ -1271,23 +1312,8 @@ struct GemmClusterKLauncher {
             cudaGetLastError();
             return kSmemTooLarge;
         }
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = slices;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(p.tail_tiles * slices);
-        cfg.blockDim = dim3(get_num_threads_per_sm<>(BLOCK_N));
-        cfg.dynamicSmemBytes = kSmemSize;
-        cfg.stream = stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = slices > 1 ? 1 : 0;
-        if (cudaLaunchKernelEx(&cfg, kernel, p, map_a, map_b) != cudaSuccess) {
-            cudaGetLastError();
-            return kLaunchFailed;
-        }
-        return kOk;
+        return launch_kernel(kernel, p.tail_tiles * slices, get_num_threads_per_sm<>(BLOCK_N), kSmemSize, stream, slices, true, p, map_a,
+                             map_b);
     }
 };
 

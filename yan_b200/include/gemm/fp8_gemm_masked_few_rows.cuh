@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(kFewRowsThreads, 1)
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
     }
+    ptx::grid_dependency_wait();  // up to here this kernel may run beside the one in front
     if (warp_idx == 2) {
         ptx::tmem_alloc(tmem_slot, L::kTmemCols);
         ptx::tmem_relinquish_alloc_permit();
@@ -341,8 +342,7 @@ inline int launch_masked_few_rows(const GemmArgs& a, cudaStream_t stream) {
     // of which 8 have a seventh, and nothing is left over (16 groups, N=7168).
     const uint64_t tiles = static_cast<uint64_t>(a.num_groups) * ceil_div(a.n, 128u), sms = static_cast<uint64_t>(a.num_sms);
     const uint32_t grid = static_cast<uint32_t>(ceil_div(tiles, ceil_div(tiles, sms)));
-    kernel<<<grid, kFewRowsThreads, L::kSmemSize, stream>>>(p, map_w, map_x);
-    return cudaGetLastError() == cudaSuccess ? kOk : kLaunchFailed;
+    return launch_kernel(kernel, grid, kFewRowsThreads, L::kSmemSize, stream, 1, true, p, map_w, map_x);
 }
 
 }  // namespace yan

@@ -27,7 +27,8 @@
 // Tensor memory goes back before a CTA waits for the others of its cluster: two CTAs of different clusters on an SM (another
 // stream's launch, or this launch's next cluster) may need more columns than there are, and one that kept its own while it
 // waited for a CTA that in turn waits for columns elsewhere would close a circle of waits that nothing bounds.
-// Weights are loaded before griddepcontrol.wait (parameters), activations and their scales after it; waits are bounded.
+// In front of griddepcontrol.wait a CTA sets up its barriers and asks L2 for its first weights (a hint); it reads nothing, unless the
+// caller has promised that weights are constant: then they are loaded there.  Waits are bounded.
 
 #include <cstdint>
 #include <cuda.h>
@@ -40,15 +41,17 @@
 namespace yan {
 
 // What may still be running when a CTA of this launch starts (every launch has programmatic stream serialization).
-// Tensor memory is never taken while a kernel that might itself still have to take some could be waiting for this one's:
-// the order of allocation, griddepcontrol.wait and griddepcontrol.launch_dependents follows from that.
+// Tensor memory is taken after the wait for the kernel in front in either case: that kernel, or one that it waits for, may
+// still have to take some, and a CTA that held columns while it waits for it would close a circle.
 enum StackedOrder : uint32_t {
-    kAfterAnyKernel = 0,      // nothing is known: wait for it first, then everything else
-    kAfterOwnQuantizer = 1,   // this library's quantizer, which waits for its own predecessors before it lets this launch
-                              // start: weights and tensor memory are free to use, the activations are not
-    kConstantWeights = 2,     // any kernel, none of which writes weights (the caller's promise): weights are loaded at
-                              // once, tensor memory is taken after the wait
+    kAfterAnyKernel = 0,   // nothing is known: barriers and prefetches, then wait, then everything else
+    kConstantWeights = 1,  // any kernel, none of which writes weights (the caller's promise): they are loaded before the wait
 };
+
+// Steps whose weights every CTA asks L2 for before it waits (0 / 3 / 8 / all, us in a graph: M=1 N=4096 K=7168 7.4 / 7.0 / 7.1 /
+// 7.3, M=16 N=4096 K=4096 5.5 / 5.2 / 5.0 / 5.1, M=4 N=28672 K=8192 40.3 / 39.7 / 42.8 / 45.0: a launch of several waves of CTAs
+// only fetches twice what its loads fetch anyway).
+constexpr uint32_t kPrefetchSteps = 4;
 
 // Adds kCols floats of shared memory; false where they come from a thread that gave up.
 template <uint32_t kCols>
@@ -103,13 +106,19 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     const uint32_t part0 = rank * kStack;
 
     if (cluster > 1) ptx::cluster_arrive();  // waited for in front of the exchange: by then every CTA of it has started
-    if (order == kAfterAnyKernel) ptx::grid_dependency_wait();
     if (order == kConstantWeights) ptx::grid_dependency_launch_dependents();
+    if (warp_idx < 4 && order == kAfterAnyKernel) {
+        // the first weights on their way to L2 while the kernel in front ends: thread = (k-part, row) of a step
+        const uint32_t r = threadIdx.x % kRows, kb = (part0 + threadIdx.x / kRows) * steps;
+        const uint8_t* w = p.weights + static_cast<size_t>(n0 + r) * p.shape_k + kb * kBlockK;
+        if (n0 + r < p.shape_n)
+            for (uint32_t s = 0; s < steps && s < kPrefetchSteps && kb + s < num_k_blocks; ++s) ptx::prefetch_l2(w + s * kBlockK);
+    }
     if (warp_idx == 5) {
         // First thing: an SM does not start its second CTA before the first one has given up the permit to allocate
         // (CTAs 148.. of a 224-CTA grid started 2.0 us late when the allocation followed the activations' loads:
         // M=16 N=7168 K=2048 with its quantizer 8.1 -> 7.0 us).
-        if (order == kConstantWeights) ptx::grid_dependency_wait();
+        ptx::grid_dependency_wait();
         ptx::tmem_alloc(tmem_slot, kTmemCols);
         ptx::tmem_relinquish_alloc_permit();
         // the kernel behind this one may start: its own allocation cannot get in front of this grid's any more
@@ -148,6 +157,7 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
             ptx::fence_proxy_async_smem();
         }
         __syncwarp();
+        if (order == kAfterAnyKernel) ptx::grid_dependency_wait();
         if (ptx::elect_one()) {
 #pragma unroll
             for (uint32_t slot = 0; slot < kSlots; ++slot)
@@ -348,32 +358,8 @@ inline int launch_stacked_k_instance(const GemmParams& p, const CUtensorMap& map
         cudaGetLastError();
         return kSmemTooLarge;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ceil_div(p.shape_n, 128 / kStack) * cluster);
-    cfg.blockDim = dim3(kStackedThreads);
-    cfg.dynamicSmemBytes = smem_bytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    uint32_t num_attrs = 0;
-    if (cluster > 1) {
-        attr[num_attrs].id = cudaLaunchAttributeClusterDimension;
-        attr[num_attrs].val.clusterDim.x = cluster;
-        attr[num_attrs].val.clusterDim.y = 1;
-        attr[num_attrs].val.clusterDim.z = 1;
-        ++num_attrs;
-    }
-    {
-        attr[num_attrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[num_attrs].val.programmaticStreamSerializationAllowed = 1;
-        ++num_attrs;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = num_attrs;
-    if (cudaLaunchKernelEx(&cfg, kernel, p, map_w, map_x, cluster, static_cast<uint32_t>(order)) != cudaSuccess) {
-        cudaGetLastError();
-        return kLaunchFailed;
-    }
-    return kOk;
+    return launch_kernel(kernel, ceil_div(p.shape_n, 128 / kStack) * cluster, kStackedThreads, smem_bytes, stream, cluster, true, p, map_w,
+                         map_x, cluster, static_cast<uint32_t>(order));
 }
 
 // Host launcher.  Arguments as GemmLauncher::launch (Normal GEMM, bf16 output).
@@ -398,6 +384,7 @@ inline int launch_fp8_gemm_stacked_k(const GemmArgs& a, cudaStream_t stream, Sta
     p.scales_a = a.lhs_scales;
     p.scales_b = a.rhs_scales;
     p.grouped_layout = nullptr;
+    p.weights = static_cast<const uint8_t*>(a.rhs);
     p.out = a.out;
     p.out_scales = nullptr;
     p.out_scales_ld = 0;

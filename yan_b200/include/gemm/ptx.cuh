@@ -41,6 +41,10 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// A hint: brings the 128-byte line of `p` into L2, where every reader and writer of it meets.  It gives the program nothing to
+// read, so it needs no order with a kernel that may still write there.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // Programmatic dependent launch: `wait` blocks until the grids this one depends on have completed and
 // their memory is visible (no-op for an ordinary launch); `launch_dependents` lets the next grid of
 // the stream start its own pre-`wait` part early.

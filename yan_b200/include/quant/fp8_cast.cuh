@@ -63,17 +63,18 @@ __global__ void __launch_bounds__(256) per_token_cast_to_fp8_kernel(const __nv_b
                                                                     uint8_t* __restrict__ q,
                                                                     float* __restrict__ scales, uint32_t m, uint32_t k,
                                                                     uint32_t x_ld, uint32_t sa_ld,
-                                                                    bool weights_are_constant) {
+                                                                    bool release_early) {
     constexpr uint32_t kGroups = 4;
     constexpr uint32_t kItems = kRows * kGroups / 32;  // per eight lanes
     __shared__ float s_scales[kGroups][kRows];
     // This kernel is launched with programmatic stream serialization: its CTAs may be resident before the kernel in front
-    // of it has finished, and wait for it (the producer of x, the previous readers of q / scales) here.  A GEMM launched
-    // the same way behind this kernel starts loading its weights when every CTA here has let it: after the wait, so that
-    // whatever the earlier kernels wrote to them is there; before it only if the caller has promised that nothing did.
-    if (weights_are_constant) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // of it has finished, and wait for it (the producer of x, the previous readers of q / scales) here.
+    // release_early: what follows may start at once, because it waits for this kernel before it reads anything (its launch, 0.9 us
+    // behind the release, then overlaps the wait).  Otherwise it starts when every CTA here is past its wait, and may rely on
+    // whatever earlier kernels wrote, weights among it.
+    if (release_early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (!weights_are_constant) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (!release_early) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     const uint32_t octet = threadIdx.x / 8, l = threadIdx.x % 8;
     const uint32_t row0 = blockIdx.y * kRows, kb0 = blockIdx.x * kGroups;
@@ -161,9 +162,8 @@ __global__ void __launch_bounds__(256) per_block_cast_to_fp8_kernel(const __nv_b
 // Host launchers.  Return a ReturnCode.
 // Always launched with programmatic stream serialization, so that the launch latency overlaps the tail of the kernel
 // before it in the stream (the kernel waits for that kernel before it reads or writes anything).
-// weights_are_constant: no kernel in front of this one writes the weights of the GEMM behind it (see the kernel).
 inline int launch_per_token_cast_to_fp8(const void* x, void* q, float* scales, uint32_t m, uint32_t k, uint32_t x_ld,
-                                        uint32_t sa_ld, cudaStream_t stream, bool weights_are_constant = false) {
+                                        uint32_t sa_ld, cudaStream_t stream, bool release_early = true) {
     if (x == nullptr || q == nullptr || scales == nullptr || m == 0 || k == 0 || k % 128 != 0) return kBadArgument;
     if (x_ld < k || x_ld % 8 != 0 || sa_ld < m) return kBadArgument;
     if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(q) % 8 != 0) return kBadArgument;
@@ -184,7 +184,7 @@ inline int launch_per_token_cast_to_fp8(const void* x, void* q, float* scales, u
     if (cfg.gridDim.y > 65535) return kBadArgument;
     auto kernel = rows == 32 ? (wide ? per_token_cast_to_fp8_kernel<32, true> : per_token_cast_to_fp8_kernel<32, false>)
                              : (wide ? per_token_cast_to_fp8_kernel<8, true> : per_token_cast_to_fp8_kernel<8, false>);
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xp, qp, scales, m, k, x_ld, sa_ld, weights_are_constant);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, xp, qp, scales, m, k, x_ld, sa_ld, release_early);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return kLaunchFailed;
