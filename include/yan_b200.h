@@ -250,14 +250,11 @@ void yan_b200_allreduce_bf16_gather_staged(const void* stage, void* const* data,
                                            int num_ctas, void* stream, int* return_code);
 
 /*
- * Programmatic dependent launch for the weight-streaming (M <= 64) kernel.  When enabled, that kernel is
- * launched with cudaLaunchAttributeProgrammaticStreamSerialization: its weight loads (rhs) may start while the
- * previous kernel of the stream is still running; activations, scales of the activations and the output are
- * only touched after the previous kernel has completed.  Enable it only when `rhs` / `rhs_scales` are not
- * written by the kernel that precedes the GEMM in its stream (true for inference weights).  Default: off.
- * The quantizer is always launched that way (its launch overlaps the tail of the previous kernel of the stream, and it
- * waits for that kernel before it reads or writes anything); while this is enabled it also lets the GEMM behind it in
- * yan_b200_fp8_linear_bf16(_static) start loading weights before that wait instead of after it.
+ * Constant weights.  Quantizer and GEMMs are launched with cudaLaunchAttributeProgrammaticStreamSerialization where that
+ * pays: they may start while the previous kernel of the stream is still running, and wait for it before they read or write
+ * anything (they only ask L2 for weights).  When enabled, the weight-streaming (M <= 64) kernels load their weights (rhs)
+ * before that wait.  Enable it only when `rhs` / `rhs_scales` are not written by the kernels that precede the GEMM in its
+ * stream (true for inference weights).  Default: off.
  * No reference counterpart (the reference launches every kernel with plain <<<>>>, e.g.
  * yan/include/gemm/cute_gemm.cuh:373).
  */
