@@ -93,6 +93,8 @@ inline void set_rc(int* rc, int v) {
 // room for the staged epilogue (224, 160, 96) or with a second B scale and a 16-column tail chunk pay for that; but with four
 // accumulators instead of two its epilogue hides better.  Large problems therefore get 256; narrower tiles win when they fill
 // the machine better or K is short.
+// (The issue loop of the narrow tiles has made them up to 0.03 us per k-block faster since; over 57 random shapes of 65 to 4096 rows the
+// choice is within 2 % of the best width.)
 // `time_out`, when given, receives the winner's time.
 int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* time_out = nullptr) {
     static const struct { int bn; double start, per_kb, epilogue; } candidates[8] = {

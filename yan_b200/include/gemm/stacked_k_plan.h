@@ -56,9 +56,9 @@ struct StackedConfig {
 //     M=64 N=7168 K=4096 with 6 operand slots 13.4, with 4 14.8).  More row groups than SMs: 4 slots, two CTAs per SM
 //     (M=16 N=7168 K=2048: 7.0; with 8 slots, one CTA per SM and two waves of them: 8.0).  At most four steps: 4 slots as
 //     well, the others would never hold anything, and their columns are what a second CTA on the SM would wait for.
-//   * a cluster along K where row groups leave SMs idle, as long as it saves every CTA four steps: the exchange costs about
-//     0.45 us and a step 0.15 - 0.3 (M=16 N=2048 K=7168: 9.2 / 8.6 / 9.8 for clusters of 1 / 2 / 4; M=8 N=528 K=13440:
-//     14.2 / 9.6 / 7.4 / 9.2 for 1 / 2 / 4 / 8; M=16 N=1024 K=1024: 4.0 / 4.5 for 1 / 2).
+//   * a cluster along K where row groups leave SMs idle, as long as it saves every CTA four steps (at least two / four / six / nine
+//     saved: M=64 N=1024 K=4096 4.8 / 4.9 / 5.4 / 6.7, M=16 N=1024 K=4096 3.5 / 3.3 / 3.8 / 3.8, M=64 N=2048 K=1024 4.1 / 3.3 / 3.3 /
+//     3.3, M=16 N=1024 K=8192 4.4 / 4.4 / 4.7 / 5.4; clusters of eight: M=8 N=528 K=13440 9.2 against 7.4).
 //   * clusters of four: as many as can be resident at once.  Where a CTA has an SM to itself that is 33 (132 CTAs: the SMs of a
 //     processing cluster are no multiple of four); the others would start when the first have ended (M=64 K=7168: N=2112 8.5,
 //     N=2176 14.1 against 10.6 with clusters of two, N=2368 14.4 against 10.7; M=32 N=2304 K=8192 12.8 against 9.3; M=16
