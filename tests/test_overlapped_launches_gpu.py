@@ -68,3 +68,40 @@ def test_back_to_back_equals_one_at_a_time(cuda_lib, kind, m, n, k):
     for _ in range(3):
         assert all(torch.equal(a, b) for a, b in zip(run(False), want))
     assert yan_b200.read_device_status() == 0
+
+
+# the small-batch kernel and the pair kernel, both of which load weights before their wait under the promise
+@pytest.mark.parametrize("m,block_n", [(16, 0), (64, 0), (16, 1), (64, 1)])
+def test_a_cast_separates_constant_weights_from_their_writer(cuda_lib, m, block_n):
+    """With the promise that the call in front of a GEMM does not write its weights: the weight codes are written by a kernel that
+    lets its successors start early, the activations are quantized by a call between the two, and the GEMM sees the new weights."""
+    import yan_b200
+    n, k = 7168, 2048
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    ws = [torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    codes = (torch.empty(n, k, dtype=torch.float8_e4m3fn, device="cuda"), torch.empty(k // 128, n, device="cuda").t())
+    rhs = (codes[0], torch.full((n // 128, k // 128), 0.01, device="cuda"))
+    lhs = yan_b200.per_token_cast_to_fp8(x)
+    outs = [torch.empty(m, n, dtype=torch.bfloat16, device="cuda") for _ in range(16)]
+
+    def run(sync):
+        for i, out in enumerate(outs):
+            for call in (lambda: yan_b200.per_token_cast_to_fp8(ws[i % 4], out=codes),
+                         lambda: yan_b200.per_token_cast_to_fp8(x, out=lhs),
+                         lambda: yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out, block_n=block_n)):
+                call()
+                if sync:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    yan_b200.set_programmatic_dependent_launch(True)
+    try:
+        want = run(True)
+        assert not torch.equal(want[0], want[1])
+        for _ in range(3):
+            assert all(torch.equal(g, w) for g, w in zip(run(False), want))
+    finally:
+        yan_b200.set_programmatic_dependent_launch(False)
+    assert yan_b200.read_device_status() == 0

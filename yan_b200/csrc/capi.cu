@@ -9,6 +9,7 @@
 
 #include "../../include/yan_b200.h"
 #include "gemm_dispatch.h"
+#include "launch_order.h"
 #include "gemm/fp8_gemm_masked_few_rows.cuh"
 #include "gemm/fp8_gemm_small_m.cuh"
 #include "gemm/fp8_gemm_stacked_k.cuh"
@@ -382,7 +383,8 @@ YAN_EXPORT void yan_b200_per_token_cast_to_fp8(const void* x, void* out, void* o
     if (m <= 0 || k <= 0 || x_ld <= 0 || scales_ld <= 0) return set_rc(return_code, yan::kBadArgument);
     set_rc(return_code,
            yan::launch_per_token_cast_to_fp8(x, out, static_cast<float*>(out_scales), m, k, x_ld, scales_ld,
-                                             static_cast<cudaStream_t>(stream)));
+                                             static_cast<cudaStream_t>(stream),
+                                             yan::cast_releases_early(g_programmatic_launch != 0)));
 }
 
 YAN_EXPORT void yan_b200_per_block_cast_to_fp8(const void* w, void* out, void* out_scales, int n, int k, void* stream,

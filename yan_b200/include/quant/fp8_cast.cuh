@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) per_block_cast_to_fp8_kernel(const __nv_b
 // Always launched with programmatic stream serialization, so that the launch latency overlaps the tail of the kernel
 // before it in the stream (the kernel waits for that kernel before it reads or writes anything).
 inline int launch_per_token_cast_to_fp8(const void* x, void* q, float* scales, uint32_t m, uint32_t k, uint32_t x_ld,
-                                        uint32_t sa_ld, cudaStream_t stream, bool release_early = true) {
+                                        uint32_t sa_ld, cudaStream_t stream, bool release_early) {
     if (x == nullptr || q == nullptr || scales == nullptr || m == 0 || k == 0 || k % 128 != 0) return kBadArgument;
     if (x_ld < k || x_ld % 8 != 0 || sa_ld < m) return kBadArgument;
     if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(q) % 8 != 0) return kBadArgument;

@@ -343,9 +343,11 @@ def fp8_linear_workspace_bytes(m: int, k: int) -> int:
 
 
 def set_programmatic_dependent_launch(enabled: bool) -> None:
-    """Lets the M <= 64 weight-streaming kernel start fetching weights while the previous kernel of the stream is
-    still running (programmatic dependent launch), and lets the quantizer inside fp8_linear be launched over the tail of
-    the kernel before it.  Only valid when the weights are not produced by the kernel that precedes a GEMM."""
+    """A promise of constant weights: lets the M <= 64 weight-streaming kernels load weights while the previous kernel of the stream
+    is still running (programmatic dependent launch).  Only valid when the weights are not written by the call that precedes the
+    GEMM or fp8_linear in its stream; M <= 64 GEMM and fp8_linear calls that follow one another count as one call, whose weights
+    nothing directly in front of it may write.  Any other call in between, per_token_cast_to_fp8 among them, completes what lies
+    in front of it first."""
     _lib.lib().yan_b200_set_programmatic_dependent_launch(int(bool(enabled)))
 
 
