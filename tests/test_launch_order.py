@@ -18,3 +18,37 @@ def _run(tmp_path, body):
 def test_a_cast_completes_what_is_in_front_of_it_under_the_promise(tmp_path):
     out = _run(tmp_path, 'std::printf("%d %d", yan::cast_releases_early(false), yan::cast_releases_early(true));')
     assert out == ["1", "0"]
+
+
+def test_the_first_gemm_of_a_place_waits_after_the_promise_is_made(tmp_path):
+    """A quantizer launched while the promise was off may still let what follows it start early: on every stream, in every capture
+    and after every switch the first GEMM does not rely on the promise, the ones behind it do."""
+    out = _run(tmp_path, """
+    yan::ConstantWeights w;
+    int stream[100];
+    auto at = [&](int device, int s, unsigned long long capture = 0, bool known = true) {
+        return yan::LaunchPlace{w.era(), device, stream + s, capture, known};
+    };
+    auto gemm = [&](const yan::LaunchPlace& p) {
+        std::printf("%d ", w.holds(p));
+        w.settle(p);
+    };
+    gemm(at(0, 0)); gemm(at(0, 0));
+    std::printf("off ");
+    w.set(true);
+    gemm(at(0, 0)); gemm(at(0, 0)); gemm(at(0, 1)); gemm(at(1, 0)); gemm(at(0, 0, 7)); gemm(at(0, 0, 7)); gemm(at(0, 0));
+    gemm(at(0, 2, 0, false)); gemm(at(0, 2, 0, false));
+    w.set(true);
+    gemm(at(0, 0));
+    std::printf("on ");
+    const yan::LaunchPlace before = at(0, 0);
+    w.set(false);
+    gemm(at(0, 0));
+    w.set(true);
+    w.settle(before);
+    gemm(at(0, 0)); gemm(at(0, 0));
+    std::printf("switched ");
+    for (int s = 10; s < 90; ++s) w.settle(at(0, s));
+    gemm(at(0, 89)); gemm(at(0, 10)); gemm(at(0, 10));
+    std::printf("many");""")
+    assert " ".join(out) == "0 0 off 0 1 0 0 0 1 1 0 0 1 on 0 0 1 switched 1 0 1 many"

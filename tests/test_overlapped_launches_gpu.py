@@ -72,9 +72,11 @@ def test_back_to_back_equals_one_at_a_time(cuda_lib, kind, m, n, k):
 
 # the small-batch kernel and the pair kernel, both of which load weights before their wait under the promise
 @pytest.mark.parametrize("m,block_n", [(16, 0), (64, 0), (16, 1), (64, 1)])
-def test_a_cast_separates_constant_weights_from_their_writer(cuda_lib, m, block_n):
+@pytest.mark.parametrize("switched", [False, True])
+def test_a_cast_separates_constant_weights_from_their_writer(cuda_lib, m, block_n, switched):
     """With the promise that the call in front of a GEMM does not write its weights: the weight codes are written by a kernel that
-    lets its successors start early, the activations are quantized by a call between the two, and the GEMM sees the new weights."""
+    lets its successors start early, the activations are quantized by a call between the two, and the GEMM sees the new weights;
+    also where the promise is made for the GEMM's call alone."""
     import yan_b200
     n, k = 7168, 2048
     gen = torch.Generator(device="cuda").manual_seed(m)
@@ -87,16 +89,17 @@ def test_a_cast_separates_constant_weights_from_their_writer(cuda_lib, m, block_
 
     def run(sync):
         for i, out in enumerate(outs):
-            for call in (lambda: yan_b200.per_token_cast_to_fp8(ws[i % 4], out=codes),
-                         lambda: yan_b200.per_token_cast_to_fp8(x, out=lhs),
-                         lambda: yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out, block_n=block_n)):
-                call()
+            for j in range(3):
+                yan_b200.set_programmatic_dependent_launch(j == 2 or not switched)
+                if j < 2:
+                    yan_b200.per_token_cast_to_fp8(*((ws[i % 4], codes) if j == 0 else (x, lhs)))
+                else:
+                    yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out, block_n=block_n)
                 if sync:
                     torch.cuda.synchronize()
         torch.cuda.synchronize()
         return [out.clone() for out in outs]
 
-    yan_b200.set_programmatic_dependent_launch(True)
     try:
         want = run(True)
         assert not torch.equal(want[0], want[1])

@@ -25,7 +25,7 @@ unsigned long long g_timeout_ns = 2000000000ull;
 // The waits between ranks have a bound of their own: ranks of one job drift apart by seconds for ordinary reasons
 // (first-call module loading, a garbage collection, a stalled data loader), which no wait inside one kernel does.
 unsigned long long g_collective_timeout_ns = 10000000000ull;
-int g_programmatic_launch = 0;
+yan::ConstantWeights g_constant_weights;
 long long* g_clock_probe = nullptr;
 
 constexpr int kMaxDevices = 64;
@@ -84,6 +84,20 @@ __global__ void wait_probe_kernel(yan::GemmParams p) {
     __syncthreads();
 }
 
+yan::LaunchPlace launch_place(void* stream) {
+    yan::LaunchPlace place;
+    place.era = g_constant_weights.era();
+    place.stream = stream;
+    if (!yan::ConstantWeights::promised(place.era)) return place;
+    cudaStreamCaptureStatus status;
+    // the handle of the per-thread default stream is the same for every thread
+    place.known = static_cast<cudaStream_t>(stream) != cudaStreamPerThread && cudaGetDevice(&place.device) == cudaSuccess &&
+                  cudaStreamGetCaptureInfo_v2(static_cast<cudaStream_t>(stream), &status, &place.capture) == cudaSuccess;
+    if (!place.known) cudaGetLastError();
+    else if (status == cudaStreamCaptureStatusNone) place.capture = 0;
+    return place;
+}
+
 inline void set_rc(int* rc, int v) {
     if (rc != nullptr) *rc = v;
 }
@@ -139,7 +153,7 @@ int choose_cluster_slices(int m, int n, int k, int num_sms, double whole) {
 }
 
 int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, int block_n, void* stream,
-                  bool after_own_quantizer = false) {
+                  bool constant_weights, bool after_own_quantizer) {
     if (a.m == 0 || a.n == 0 || a.k == 0) return yan::kBadArgument;
     if (a.num_sms <= 0) return yan::kBadArgument;
     const bool want_auto = (block_n == 0);
@@ -161,7 +175,7 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
         cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        const yan::StackedOrder order = g_programmatic_launch != 0 ? yan::kConstantWeights : yan::kAfterAnyKernel;
+        const yan::StackedOrder order = constant_weights ? yan::kConstantWeights : yan::kAfterAnyKernel;
         const bool small_m_ok = yan::small_m_supported(a.m, a.n, a.k, max_smem);
         const bool stacked_ok = yan::stacked_k_supported(a.m, a.n, a.k);
         if (block_n == 2) return stacked_ok ? yan::launch_fp8_gemm_stacked_k(a, s, order) : yan::kBadArgument;
@@ -175,7 +189,7 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
             return yan::launch_fp8_gemm_stacked_k(a, s, order);
         if (block_n == 1 || (want_auto && !general_ok && small_m_ok)) {
             if (!small_m_ok) return yan::kBadArgument;
-            return yan::launch_fp8_gemm_small_m(a, s, g_programmatic_launch != 0 || (after_own_quantizer && block_n == 1));
+            return yan::launch_fp8_gemm_small_m(a, s, constant_weights || (after_own_quantizer && block_n == 1));
         }
         // what the general kernel is the default for, with an output that it does not take
         if (want_auto && !general_ok && any_output) return yan::launch_fp8_gemm_stacked_k(a, s, order);
@@ -209,16 +223,27 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
     }
 }
 
+// A GEMM as a call of its own.
+int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, int block_n, void* stream) {
+    const yan::LaunchPlace place = launch_place(stream);
+    const int rc = dispatch_gemm(type, out_kind, a, block_n, stream, g_constant_weights.holds(place), false);
+    if (rc == yan::kOk) g_constant_weights.settle(place);
+    return rc;
+}
+
 bool positive(int a, int b, int c) { return a > 0 && b > 0 && c > 0; }
 
-// Whether the quantizer of a quantize-then-GEMM call lets the GEMM start before it has waited for the kernel in front.  Every GEMM
-// waits for the quantizer before it reads anything, except the pair kernel (block_n = 1), which loads its weights first: it has to
-// start behind whatever wrote them, unless the caller has promised that nothing did.
-bool release_early(int block_n) { return block_n != 1 || g_programmatic_launch != 0; }
-
-// The GEMM of a quantize-then-GEMM call, behind this library's own quantizer in the stream.
-int gemm_after_quantizer(const void* q, const float* scales, const void* rhs, const void* rhs_scales, void* out, int m,
-                         int n, int k, int ldd, void* stream, int num_sms, int block_n) {
+// Quantizer and GEMM, one behind the other in the stream.
+int quantize_and_gemm(const void* x, uint8_t* q, float* scales, const void* rhs, const void* rhs_scales, void* out, int m, int n,
+                      int k, int ldd, void* stream, int num_sms, int block_n) {
+    const yan::LaunchPlace place = launch_place(stream);
+    const bool constant_weights = g_constant_weights.holds(place);
+    // The quantizer lets the GEMM start before it has waited for the kernel in front: every GEMM waits for the quantizer before it
+    // reads anything, except the pair kernel (block_n = 1), which loads its weights first: it has to start behind whatever wrote
+    // them, unless the caller has promised that nothing did.
+    int rc = yan::launch_per_token_cast_to_fp8(x, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
+                                               block_n != 1 || constant_weights);
+    if (rc != yan::kOk) return rc;
     if (ldd <= 0) return yan::kBadArgument;
     yan::GemmArgs a;
     a.lhs = q;
@@ -230,7 +255,9 @@ int gemm_after_quantizer(const void* q, const float* scales, const void* rhs, co
     a.ldd = static_cast<uint32_t>(ldd);
     a.m = m, a.n = n, a.k = k;
     a.num_sms = num_sms;
-    return dispatch_gemm(yan::GemmType::Normal, yan::OutKind::BF16, a, block_n, stream, true);
+    rc = dispatch_gemm(yan::GemmType::Normal, yan::OutKind::BF16, a, block_n, stream, constant_weights, true);
+    if (rc == yan::kOk) g_constant_weights.settle(place);
+    return rc;
 }
 
 }  // namespace
@@ -384,7 +411,7 @@ YAN_EXPORT void yan_b200_per_token_cast_to_fp8(const void* x, void* out, void* o
     set_rc(return_code,
            yan::launch_per_token_cast_to_fp8(x, out, static_cast<float*>(out_scales), m, k, x_ld, scales_ld,
                                              static_cast<cudaStream_t>(stream),
-                                             yan::cast_releases_early(g_programmatic_launch != 0)));
+                                             yan::cast_releases_early(yan::ConstantWeights::promised(g_constant_weights.era()))));
 }
 
 YAN_EXPORT void yan_b200_per_block_cast_to_fp8(const void* w, void* out, void* out_scales, int n, int k, void* stream,
@@ -410,10 +437,7 @@ YAN_EXPORT void yan_b200_fp8_linear_bf16(const void* a, const void* rhs, const v
         return set_rc(return_code, yan::kWorkspaceTooSmall);
     uint8_t* q = static_cast<uint8_t*>(workspace);
     float* scales = reinterpret_cast<float*>(q + yan::align_up(static_cast<size_t>(m) * k, static_cast<size_t>(256)));
-    int rc = yan::launch_per_token_cast_to_fp8(a, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
-                                               release_early(block_n));
-    if (rc != yan::kOk) return set_rc(return_code, rc);
-    set_rc(return_code, gemm_after_quantizer(q, scales, rhs, rhs_scales, out, m, n, k, ldd, stream, num_sms, block_n));
+    set_rc(return_code, quantize_and_gemm(a, q, scales, rhs, rhs_scales, out, m, n, k, ldd, stream, num_sms, block_n));
 }
 
 YAN_EXPORT void yan_b200_fp8_linear_bf16_static(const void* a, const void* rhs, const void* rhs_scales, void* out,
@@ -427,10 +451,7 @@ YAN_EXPORT void yan_b200_fp8_linear_bf16_static(const void* a, const void* rhs, 
     if (scratch == nullptr) return set_rc(return_code, yan::kLaunchFailed);
     uint8_t* q = scratch;
     float* scales = reinterpret_cast<float*>(scratch + kStaticScratchQBytes);
-    const int rc = yan::launch_per_token_cast_to_fp8(a, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
-                                                     release_early(block_n));
-    if (rc != yan::kOk) return set_rc(return_code, rc);
-    set_rc(return_code, gemm_after_quantizer(q, scales, rhs, rhs_scales, out, m, n, k, ldd, stream, num_sms, block_n));
+    set_rc(return_code, quantize_and_gemm(a, q, scales, rhs, rhs_scales, out, m, n, k, ldd, stream, num_sms, block_n));
 }
 
 YAN_EXPORT void yan_b200_read_device_status(int* status, int reset, int* return_code) {
@@ -610,7 +631,7 @@ YAN_EXPORT void yan_b200_allreduce_bf16_gather_staged(const void* stage, void* c
     set_rc(return_code, yan::launch_gather_staged_allreduce_bf16(a, static_cast<cudaStream_t>(stream)));
 }
 
-YAN_EXPORT void yan_b200_set_programmatic_dependent_launch(int enabled) { g_programmatic_launch = enabled; }
+YAN_EXPORT void yan_b200_set_programmatic_dependent_launch(int enabled) { g_constant_weights.set(enabled != 0); }
 
 YAN_EXPORT void yan_b200_set_clock_probe(void* device_buffer) { g_clock_probe = static_cast<long long*>(device_buffer); }
 
