@@ -9,15 +9,17 @@ from conftest import ROOT
 def _run(tmp_path, body):
     cxx = os.environ.get("CXX") or shutil.which("g++")
     assert cxx, "g++ not found: set CXX"
-    (tmp_path / "rules.cpp").write_text('#include <cstdio>\n#include "launch_order.h"\nint main() {\n' + body + "\n}\n")
+    (tmp_path / "rules.cpp").write_text('#include <cstdio>\n#include <initializer_list>\n#include "launch_order.h"\nint main() {\n' + body + "\n}\n")
     subprocess.run([cxx, "-std=c++17", "-pthread", f"-I{ROOT}/yan_b200/csrc", str(tmp_path / "rules.cpp"), "-o", str(tmp_path / "rules")],
                    check=True)
     return subprocess.run([str(tmp_path / "rules")], check=True, capture_output=True, text=True).stdout.split()
 
 
-def test_a_cast_completes_what_is_in_front_of_it_under_the_promise(tmp_path):
-    out = _run(tmp_path, 'std::printf("%d %d", yan::cast_releases_early(false), yan::cast_releases_early(true));')
-    assert out == ["1", "0"]
+def test_which_casts_let_their_successor_start_early(tmp_path):
+    """None under the promise that the call in front of a GEMM does not write its weights; otherwise those of the small batches."""
+    out = _run(tmp_path, """for (unsigned m : {1u, 64u, 65u, 8192u})
+        std::printf("%d%d ", yan::cast_releases_early(m, false), yan::cast_releases_early(m, true));""")
+    assert out == ["10", "10", "00", "00"]
 
 
 def test_the_first_gemm_of_a_place_waits_after_the_promise_is_made(tmp_path):

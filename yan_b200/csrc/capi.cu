@@ -411,7 +411,7 @@ YAN_EXPORT void yan_b200_per_token_cast_to_fp8(const void* x, void* out, void* o
     set_rc(return_code,
            yan::launch_per_token_cast_to_fp8(x, out, static_cast<float*>(out_scales), m, k, x_ld, scales_ld,
                                              static_cast<cudaStream_t>(stream),
-                                             yan::cast_releases_early(yan::ConstantWeights::promised(g_constant_weights.era()))));
+                                             yan::cast_releases_early(m, yan::ConstantWeights::promised(g_constant_weights.era()))));
 }
 
 YAN_EXPORT void yan_b200_per_block_cast_to_fp8(const void* w, void* out, void* out_scales, int n, int k, void* stream,
