@@ -1,5 +1,7 @@
 """The host-side rules of which kernel lets its successor start when (csrc/launch_order.h), without a GPU."""
+import glob
 import os
+import re
 import shutil
 import subprocess
 
@@ -54,3 +56,14 @@ def test_the_first_gemm_of_a_place_waits_after_the_promise_is_made(tmp_path):
     gemm(at(0, 89)); gemm(at(0, 10)); gemm(at(0, 10));
     std::printf("many");""")
     assert " ".join(out) == "0 0 off 0 1 0 0 0 1 1 0 0 1 on 0 0 1 switched 1 0 1 many"
+
+
+def test_kernels_that_start_beside_the_one_in_front_use_coherent_loads():
+    """The non-coherent path is defined for data that nobody writes while the kernel is resident: only a kernel that is launched
+    plainly, after everything in front of it, may use it."""
+    for path in glob.glob(f"{ROOT}/yan_b200/include/**/*.cuh", recursive=True):
+        with open(path) as f:
+            code = re.sub(r"//.*", "", f.read())
+        plain = re.search(r"__global__[^;{]*per_block_cast_to_fp8_kernel.*?\n}\n", code, re.S)
+        code = code.replace(plain.group(0), "") if plain else code
+        assert not re.search(r"__ldg\b|ld\.global\S*\.nc\b", code), path

@@ -754,9 +754,9 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
             float sa_ring[kScaleDepth], sb_ring[kScaleDepth], sb_hi_ring[kTwoScales ? kScaleDepth : 1];
 #pragma unroll
             for (uint32_t i = 0; i < kScaleDepth && !L::kScaleRing; ++i) {
-                sa_ring[i] = (row_ok && i < kb_count) ? __ldg(sa_ptr + static_cast<size_t>(i) * p.sa_ld) : 0.0f;
-                sb_ring[i] = (i < kb_count) ? __ldg(sb_ptr + i) : 0.0f;
-                if constexpr (kTwoScales) sb_hi_ring[i] = (i < kb_count) ? __ldg(sb_hi_ptr + i) : 0.0f;
+                sa_ring[i] = (row_ok && i < kb_count) ? ptx::ld_global(sa_ptr + static_cast<size_t>(i) * p.sa_ld) : 0.0f;
+                sb_ring[i] = (i < kb_count) ? ptx::ld_global(sb_ptr + i) : 0.0f;
+                if constexpr (kTwoScales) sb_hi_ring[i] = (i < kb_count) ? ptx::ld_global(sb_hi_ptr + i) : 0.0f;
             }
 #pragma unroll
             for (uint32_t j = 0; j < kColsPerWG; ++j) acc[j] = 0.0f;
@@ -861,10 +861,10 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
                             }
                         }
                         if (kb + kScaleDepth < kb_count) {
-                            sa_ring[fill] = row_ok ? __ldg(sa_next) : 0.0f;
+                            sa_ring[fill] = row_ok ? ptx::ld_global(sa_next) : 0.0f;
                             sa_next += p.sa_ld;
-                            sb_ring[fill] = __ldg(sb_ptr + kb + kScaleDepth);
-                            if constexpr (kTwoScales) sb_hi_ring[fill] = __ldg(sb_hi_ptr + kb + kScaleDepth);
+                            sb_ring[fill] = ptx::ld_global(sb_ptr + kb + kScaleDepth);
+                            if constexpr (kTwoScales) sb_hi_ring[fill] = ptx::ld_global(sb_hi_ptr + kb + kScaleDepth);
                         }
                         YAN_STAMP(w0);
                         const bool ok = (kEarlyProbe && next_ready) ||

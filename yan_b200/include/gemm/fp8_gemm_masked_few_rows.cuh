@@ -81,7 +81,7 @@ struct FewRowsWalk {
     __device__ __forceinline__ bool advance() {
         for (; group < num_groups; ++group) {
             // the count lives in device memory where the host cannot check it: clamped to [0, m_max]
-            rows = static_cast<uint32_t>(min(max(__ldg(masked_m + group), 0), static_cast<int>(m_max)));
+            rows = static_cast<uint32_t>(min(max(ptx::ld_global(masked_m + group), 0), static_cast<int>(m_max)));
             const uint32_t tiles = rows == 0 ? 0 : tiles_per_group;
             if (next < first + tiles) {
                 n_block = next - first;

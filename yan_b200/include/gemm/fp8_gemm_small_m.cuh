@@ -126,8 +126,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kSmallMThreads, 1)
         ptx::grid_dependency_wait();
         for (uint32_t i = threadIdx.x; i < kbh * M_PAD; i += 128) {
             const uint32_t kb = i / M_PAD, m = i % M_PAD;
-            const float sa = (m < p.shape_m) ? __ldg(p.scales_a + static_cast<size_t>(kb_first + kb) * p.sa_ld + m) : 0.0f;
-            s_scales[i] = sa * __ldg(sb_ptr + kb);
+            const float sa = (m < p.shape_m) ? ptx::ld_global(p.scales_a + static_cast<size_t>(kb_first + kb) * p.sa_ld + m) : 0.0f;
+            s_scales[i] = sa * ptx::ld_global(sb_ptr + kb);
         }
     }
     ptx::tcgen05_fence_before_thread_sync();

@@ -237,8 +237,8 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
             for (uint32_t j = 0; j < 8; ++j) {
                 const uint32_t i = first + j * 128, m = i % M_PAD, kb = part0 * steps + i / M_PAD;
                 const bool ok = i < num_scales && m < p.shape_m && kb < num_k_blocks;
-                sa[j] = ok ? __ldg(p.scales_a + static_cast<size_t>(kb) * p.sa_ld + m) : 0.0f;
-                sb[j] = ok ? __ldg(sb_ptr + kb) : 0.0f;
+                sa[j] = ok ? ptx::ld_global(p.scales_a + static_cast<size_t>(kb) * p.sa_ld + m) : 0.0f;
+                sb[j] = ok ? ptx::ld_global(sb_ptr + kb) : 0.0f;
             }
 #pragma unroll
             for (uint32_t j = 0; j < 8; ++j)

@@ -45,6 +45,31 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // read, so it needs no order with a kernel that may still write there.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// Loads of what the kernel in front may still have been writing when this one started (scales, group indices and counts, the
+// quantizer's input): coherent ones, kept behind the wait for that kernel.  The non-coherent path (__ldg) is defined only for data
+// that nobody writes while the kernel is resident.
+__device__ __forceinline__ float ld_global(const float* p) {
+    float v;
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int ld_global(const int* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_global(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+// 32 bytes, from a 32-byte boundary
+__device__ __forceinline__ void ld_global_32(uint4 (&v)[2], const void* p) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0].x), "=r"(v[0].y), "=r"(v[0].z), "=r"(v[0].w), "=r"(v[1].x), "=r"(v[1].y), "=r"(v[1].z), "=r"(v[1].w)
+                 : "l"(p));
+}
+
 // Programmatic dependent launch: `wait` blocks until the grids this one depends on have completed and
 // their memory is visible (no-op for an ordinary launch); `launch_dependents` lets the next grid of
 // the stream start its own pre-`wait` part early.

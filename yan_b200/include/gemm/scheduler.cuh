@@ -6,6 +6,7 @@
 
 #include <cstdint>
 
+#include "ptx.cuh"
 #include "utils.cuh"
 
 namespace yan {
@@ -77,7 +78,7 @@ struct Scheduler {
     // Group that owns the current tile (Normal: 0).  Contiguous: read from the layout at the tile's
     // first row; negative = padding tile with nothing to compute.
     __device__ __forceinline__ int get_group(uint32_t m_block_idx) const {
-        if constexpr (kGemmType == GemmType::GroupedContiguous) return __ldg(grouped_layout + m_block_idx * BLOCK_M);
+        if constexpr (kGemmType == GemmType::GroupedContiguous) return ptx::ld_global(grouped_layout + m_block_idx * BLOCK_M);
         if constexpr (kGemmType == GemmType::GroupedMasked) return static_cast<int>(curr_group_idx);
         return 0;
     }
@@ -98,7 +99,7 @@ struct Scheduler {
     // Valid rows of a masked group, clamped to [0, M_max]: the count lives in device memory where the host cannot
     // check it, and an oversized or negative value must not make a tile store into the next group or past the output.
     __device__ __forceinline__ uint32_t get_masked_rows(uint32_t group) const {
-        const int rows = __ldg(grouped_layout + group);
+        const int rows = ptx::ld_global(grouped_layout + group);
         return static_cast<uint32_t>(min(max(rows, 0), static_cast<int>(shape_m)));
     }
 };

@@ -19,6 +19,7 @@
 #include <cuda_fp8.h>
 #include <cuda_runtime.h>
 
+#include "../gemm/ptx.cuh"
 #include "../gemm/utils.cuh"
 
 namespace yan {
@@ -89,13 +90,10 @@ __global__ void __launch_bounds__(256) per_token_cast_to_fp8_kernel(const __nv_b
         if (row < m && kb < num_kb) {
             const __nv_bfloat16* src = x + static_cast<size_t>(row) * x_ld + kb * 128 + l * 16;
             if constexpr (kWide) {
-                asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                             : "=r"(v[j][0].x), "=r"(v[j][0].y), "=r"(v[j][0].z), "=r"(v[j][0].w), "=r"(v[j][1].x),
-                               "=r"(v[j][1].y), "=r"(v[j][1].z), "=r"(v[j][1].w)
-                             : "l"(src));
+                ptx::ld_global_32(v[j], src);
             } else {
-                v[j][0] = __ldg(reinterpret_cast<const uint4*>(src));
-                v[j][1] = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+                v[j][0] = ptx::ld_global(reinterpret_cast<const uint4*>(src));
+                v[j][1] = ptx::ld_global(reinterpret_cast<const uint4*>(src) + 1);
             }
         }
     }
