@@ -134,3 +134,37 @@ def test_a_cast_separates_constant_weights_from_their_writer(cuda_lib, m, block_
     finally:
         yan_b200.set_programmatic_dependent_launch(False)
     assert yan_b200.read_device_status() == 0
+
+
+# an output that only the weight-streaming kernels take, where the pair kernel is the one of them; the same kernel by name
+@pytest.mark.parametrize("block_n,pad", [(0, 1), (1, 1), (1, 0)])
+def test_fp8_linear_of_the_pair_kernel_sees_weights_written_directly_in_front(cuda_lib, block_n, pad):
+    """The pair kernel loads weights before it waits for the quantizer of its call, which lets it start behind whatever wrote them."""
+    import yan_b200
+    m, n, k = 64, 14336, 1024
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    ws = [torch.randn(n, k, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    codes = yan_b200.per_token_cast_to_fp8(ws[0])
+    rhs = (codes[0], torch.full((n // 128, k // 128), 0.01, device="cuda"))
+    outs = [torch.zeros(m, n + pad, dtype=torch.bfloat16, device="cuda") for _ in range(8)]
+
+    def run(sync):
+        for i, out in enumerate(outs):
+            yan_b200.per_token_cast_to_fp8(ws[i % 4], out=codes)
+            if sync:
+                torch.cuda.synchronize()
+            yan_b200.fp8_linear(x, rhs, out[:, :n], block_n=block_n)
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return [out.clone() for out in outs]
+
+    want = run(True)
+    assert not torch.equal(want[0], want[1])
+    general = yan_b200.fp8_linear(x, rhs, block_n=64)
+    # other order of the fp32 sums: bf16 results differ by one rounding of few values
+    assert float((want[3][:, :n].float() - general.float()).norm() / general.float().norm()) <= 1e-3
+    for _ in range(3):
+        assert all(torch.equal(g, w) for g, w in zip(run(False), want))
+    assert yan_b200.read_device_status() == 0

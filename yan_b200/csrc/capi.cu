@@ -152,7 +152,37 @@ int choose_cluster_slices(int m, int n, int k, int num_sms, double whole) {
     return best;
 }
 
-int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, int block_n, void* stream,
+// Which kernel serves a bf16 product of ordinary operands.  M <= 64: the weight-streaming kernels.  block_n 1 asks for the
+// pair-cluster kernel, 2 for the stacked-K kernel (M <= 32), 0 picks the stacked one where it is the fastest.
+enum class BatchRoute { General, Stacked, Pair, Refused };
+
+BatchRoute batch_route(const yan::GemmArgs& a, int block_n) {
+    const bool want_auto = block_n == 0;
+    if (!want_auto && block_n != 1 && block_n != 2) return BatchRoute::General;
+    int dev = 0, max_smem = 0, sm_count = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    const bool small_m_ok = yan::small_m_supported(a.m, a.n, a.k, max_smem);
+    const bool stacked_ok = yan::stacked_k_supported(a.m, a.n, a.k);
+    if (block_n == 2) return stacked_ok ? BatchRoute::Stacked : BatchRoute::Refused;
+    if (block_n == 1) return small_m_ok ? BatchRoute::Pair : BatchRoute::Refused;
+    // The general kernel stores 16 bytes at a time and checks num_sms; the weight-streaming kernels do neither.  A shape
+    // that one of them serves whatever the output is keeps that; the others are held to the general kernel's terms.
+    const bool general_ok = yan::is_aligned(a.out, 16) && a.ldd % 8 == 0 && a.num_sms <= sm_count;
+    const bool any_output = small_m_ok || (stacked_ok && (a.m <= 16 || a.n / 32 <= static_cast<uint32_t>(sm_count)));
+    if ((general_ok || any_output) &&
+        yan::stacked_k_preferred(a.m, a.n, a.k, static_cast<uint32_t>(a.num_sms), static_cast<uint32_t>(sm_count),
+                                 static_cast<uint32_t>(max_smem)))
+        return BatchRoute::Stacked;
+    // what the general kernel is the default for, with an output that it does not take
+    if (!general_ok && any_output) return small_m_ok ? BatchRoute::Pair : BatchRoute::Stacked;
+    return BatchRoute::General;
+}
+
+// after_own_quantizer: the kernel in front is this library's quantizer, which has let the pair kernel start only when whatever wrote
+// its weights had completed.
+int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, int block_n, void* stream, BatchRoute route,
                   bool constant_weights, bool after_own_quantizer) {
     if (a.m == 0 || a.n == 0 || a.k == 0) return yan::kBadArgument;
     if (a.num_sms <= 0) return yan::kBadArgument;
@@ -168,31 +198,11 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
     a.timeout_ns = g_timeout_ns;
     a.clock_probe = g_clock_probe;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // M <= 64: the weight-streaming kernels.  block_n 1 asks for the pair-cluster kernel, 2 for the stacked-K kernel
-    // (M <= 32), 0 picks the stacked one where it is the fastest.
-    if (type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16 && (want_auto || block_n == 1 || block_n == 2)) {
-        int dev = 0, max_smem = 0, sm_count = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-        cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-        const yan::StackedOrder order = constant_weights ? yan::kConstantWeights : yan::kAfterAnyKernel;
-        const bool small_m_ok = yan::small_m_supported(a.m, a.n, a.k, max_smem);
-        const bool stacked_ok = yan::stacked_k_supported(a.m, a.n, a.k);
-        if (block_n == 2) return stacked_ok ? yan::launch_fp8_gemm_stacked_k(a, s, order) : yan::kBadArgument;
-        // The general kernel stores 16 bytes at a time and checks num_sms; the weight-streaming kernels do neither.  A shape
-        // that one of them serves whatever the output is keeps that; the others are held to the general kernel's terms.
-        const bool general_ok = yan::is_aligned(a.out, 16) && a.ldd % 8 == 0 && a.num_sms <= sm_count;
-        const bool any_output = small_m_ok || (stacked_ok && (a.m <= 16 || a.n / 32 <= static_cast<uint32_t>(sm_count)));
-        if (want_auto && (general_ok || any_output) &&
-            yan::stacked_k_preferred(a.m, a.n, a.k, static_cast<uint32_t>(a.num_sms), static_cast<uint32_t>(sm_count),
-                                     static_cast<uint32_t>(max_smem)))
-            return yan::launch_fp8_gemm_stacked_k(a, s, order);
-        if (block_n == 1 || (want_auto && !general_ok && small_m_ok)) {
-            if (!small_m_ok) return yan::kBadArgument;
-            return yan::launch_fp8_gemm_small_m(a, s, constant_weights || (after_own_quantizer && block_n == 1));
-        }
-        // what the general kernel is the default for, with an output that it does not take
-        if (want_auto && !general_ok && any_output) return yan::launch_fp8_gemm_stacked_k(a, s, order);
+    if (type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16) {
+        if (route == BatchRoute::Refused) return yan::kBadArgument;
+        if (route == BatchRoute::Stacked)
+            return yan::launch_fp8_gemm_stacked_k(a, s, constant_weights ? yan::kConstantWeights : yan::kAfterAnyKernel);
+        if (route == BatchRoute::Pair) return yan::launch_fp8_gemm_small_m(a, s, constant_weights || after_own_quantizer);
     }
     if (type == yan::GemmType::Normal && want_auto && out_kind != yan::OutKind::E4M3 && a.scatter_world == 0) {
         const int slices = choose_cluster_slices(static_cast<int>(a.m), static_cast<int>(a.n), static_cast<int>(a.k), a.num_sms,
@@ -226,7 +236,9 @@ int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, i
 // A GEMM as a call of its own.
 int dispatch_gemm(yan::GemmType type, yan::OutKind out_kind, yan::GemmArgs& a, int block_n, void* stream) {
     const yan::LaunchPlace place = launch_place(stream);
-    const int rc = dispatch_gemm(type, out_kind, a, block_n, stream, g_constant_weights.holds(place), false);
+    const bool batch = type == yan::GemmType::Normal && out_kind == yan::OutKind::BF16 && a.num_sms > 0;
+    const BatchRoute route = batch ? batch_route(a, block_n) : BatchRoute::General;
+    const int rc = dispatch_gemm(type, out_kind, a, block_n, stream, route, g_constant_weights.holds(place), false);
     if (rc == yan::kOk) g_constant_weights.settle(place);
     return rc;
 }
@@ -238,13 +250,6 @@ int quantize_and_gemm(const void* x, uint8_t* q, float* scales, const void* rhs,
                       int k, int ldd, void* stream, int num_sms, int block_n) {
     const yan::LaunchPlace place = launch_place(stream);
     const bool constant_weights = g_constant_weights.holds(place);
-    // The quantizer lets the GEMM start before it has waited for the kernel in front: every GEMM waits for the quantizer before it
-    // reads anything, except the pair kernel (block_n = 1), which loads its weights first: it has to start behind whatever wrote
-    // them, unless the caller has promised that nothing did.
-    int rc = yan::launch_per_token_cast_to_fp8(x, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
-                                               block_n != 1 || constant_weights);
-    if (rc != yan::kOk) return rc;
-    if (ldd <= 0) return yan::kBadArgument;
     yan::GemmArgs a;
     a.lhs = q;
     a.lhs_scales = scales;
@@ -255,7 +260,16 @@ int quantize_and_gemm(const void* x, uint8_t* q, float* scales, const void* rhs,
     a.ldd = static_cast<uint32_t>(ldd);
     a.m = m, a.n = n, a.k = k;
     a.num_sms = num_sms;
-    rc = dispatch_gemm(yan::GemmType::Normal, yan::OutKind::BF16, a, block_n, stream, constant_weights, true);
+    if (ldd <= 0 || num_sms <= 0) return yan::kBadArgument;
+    const BatchRoute route = batch_route(a, block_n);
+    // The quantizer lets the GEMM start before it has waited for the kernel in front: every GEMM waits for the quantizer before it
+    // reads anything, except the pair kernel, which loads its weights first: it has to start behind whatever wrote them, unless the
+    // caller has promised that nothing did.  (Into an output that only that kernel takes, us in a graph, launched like this / when the
+    // quantizer has ended: M=64 N=14336 K=1024 16.7 / 17.1, M=64 N=16384 K=2048 21.7 / 22.4, M=32 N=20480 K=1024 13.0 / 13.7.)
+    int rc = yan::launch_per_token_cast_to_fp8(x, q, scales, m, k, k, m, static_cast<cudaStream_t>(stream),
+                                               route != BatchRoute::Pair || constant_weights);
+    if (rc != yan::kOk) return rc;
+    rc = dispatch_gemm(yan::GemmType::Normal, yan::OutKind::BF16, a, block_n, stream, route, constant_weights, true);
     if (rc == yan::kOk) g_constant_weights.settle(place);
     return rc;
 }
