@@ -252,8 +252,8 @@ void yan_b200_allreduce_bf16_gather_staged(const void* stage, void* const* data,
 /*
  * Constant weights.  Quantizer and GEMMs are launched with cudaLaunchAttributeProgrammaticStreamSerialization where that
  * pays: they may start while the previous kernel of the stream is still running, and wait for it before they read or write
- * anything (they only ask L2 for weights).  When enabled, the weight-streaming (M <= 64) kernels load their weights (rhs)
- * before that wait.  Enable it only when `rhs` / `rhs_scales` are not written by the call that precedes the GEMM or
+ * anything (the small-batch kernel only asks L2 for weights).  When enabled, the weight-streaming (M <= 64) kernels load
+ * their weights (rhs) before that wait.  Enable it only when `rhs` / `rhs_scales` are not written by the call that precedes the GEMM or
  * yan_b200_fp8_linear call in its stream (true for inference weights).  M <= 64 GEMM and yan_b200_fp8_linear calls let their
  * successor start before they have waited themselves, so a run of them counts as one: nothing directly in front of the run may
  * write the weights of any of its calls.  Any other call in between, yan_b200_per_token_cast_to_fp8 among them, completes what

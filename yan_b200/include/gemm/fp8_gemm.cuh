@@ -36,7 +36,7 @@ struct GemmParams {
     const float* scales_a;      // [K/128][sa_ld], element (kb, row) at kb * sa_ld + row
     const float* scales_b;      // [groups][ceil(N/128)][K/128]
     const int* grouped_layout;  // Contiguous: [M] group per row (-1 = padding); Masked: [G] valid rows
-    const uint8_t* weights = nullptr;  // the B operand, for prefetches (it is read through its tensor map)
+    const uint8_t* weights = nullptr;  // the B operand, for the small-batch kernel's prefetches (it is read through its tensor map)
     void* out;                  // [rows][ldd]
     float* out_scales;          // e4m3 output only: [N/128][out_scales_ld], element (nb, row) at nb * out_scales_ld + row
     uint32_t out_scales_ld;
@@ -499,20 +499,10 @@ __global__ void __launch_bounds__(get_num_threads_per_sm<>(BLOCK_N), 1)
         ptx::fence_barrier_init();
         ptx::fence_proxy_async_smem();
     }
-    if constexpr (kGemmType == GemmType::Normal && !kTail && kUnrolledIssue) {
-        // the weights of the first k-blocks on their way to L2 while the kernel in front ends
-        if (warp_idx == 3) {
-            Sched sched(p.shape_m, p.shape_n);
-            uint32_t m_block_idx, n_block_idx;
-            sched.swizzle(kCutK ? p.tail_first_tile + tail_tile : blockIdx.x, sched.num_m_blocks, m_block_idx, n_block_idx);
-            const uint32_t n = n_block_idx * BLOCK_N + lane_idx;
-            const uint8_t* w = p.weights + static_cast<size_t>(n) * p.shape_k + static_cast<size_t>(kb_begin) * kBlockK;
-            for (uint32_t r = 0; r < BLOCK_N && n + r < p.shape_n; r += 32, w += static_cast<size_t>(32) * p.shape_k)
-                for (uint32_t i = 0; i < kNumStages && i < kb_count; ++i) ptx::prefetch_l2(w + i * kBlockK);
-        }
-    }
     __syncthreads();  // the barriers are initialized
-    // Up to here this kernel may run beside the one in front (see GemmLauncher).  (The tail instance reads operands and writes
+    // Up to here this kernel may run beside the one in front (see GemmLauncher).  It does not ask L2 for weights meanwhile: the requests,
+    // a line per row and stage, held the barrier above back by half a microsecond (M=512 N=2048 K=2048 6.6 us with them, 6.1 without,
+    // behind a kernel of 1 us 8.2 and 7.8; M=205 N=6512 K=768 fp32 6.3 and 5.8; with quantizer M=512 N=2048 K=2048 7.9 and 7.6).  (The tail instance reads operands and writes
     // scratch, nothing that the whole-tile kernel in front of it produces: it waits at its end.)
     if constexpr (!kTail) ptx::grid_dependency_wait();
     uint32_t tmem_base = 0;
