@@ -56,7 +56,9 @@ const char* yan_b200_return_code_string(int code);
  * for M <= 64 (split-K over a pair of CTAs), 2 = the weight-streaming kernel of 0 for small batches, asked for by
  * name for M <= 32, N % 32 = 0, K % 512 = 0, K <= 16384 (YAN_B200_BAD_ARGUMENT when the problem does not fit the kernel asked for).
  * num_sms: the most CTAs a launch may have (<= device SMs).  The weight-streaming kernels asked for by name size their own grid,
- * and so does block_n = 0 for an output that only they take (a row stride that is no multiple of 8).
+ * and so does block_n = 0 for an output that only they take (a row stride that is no multiple of 8).  It bounds one launch: a GEMM
+ * that starts while the kernel in front still runs (behind a quantizer or an M <= 64 GEMM) holds SMs of its own meanwhile, so that a
+ * kernel of another stream that counts on the SMs beyond num_sms may start when the GEMM has ended.
  * With block_n = 0 the K of a tile may be shared by the CTAs of a cluster (M <= 64, or few tiles and long K; also fp32 output):
  * deterministic, but the last bit can differ from a call with an explicit tile width.
  */

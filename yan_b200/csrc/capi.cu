@@ -108,8 +108,8 @@ inline void set_rc(int* rc, int v) {
 // room for the staged epilogue (224, 160, 96) or with a second B scale and a 16-column tail chunk pay for that; but with four
 // accumulators instead of two its epilogue hides better.  Large problems therefore get 256; narrower tiles win when they fill
 // the machine better or K is short.
-// (The issue loop of the narrow tiles has made them up to 0.03 us per k-block faster since; over 57 random shapes of 65 to 4096 rows the
-// choice is within 2 % of the best width.)
+// (The issue loop of the narrow tiles and the overlapped launches have since taken up to 0.03 us per k-block and a microsecond of the
+// start off; over 57 random shapes of 65 to 4096 rows the choice is within 2 % of the best width.)
 // `time_out`, when given, receives the winner's time.
 int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* time_out = nullptr) {
     static const struct { int bn; double start, per_kb, epilogue; } candidates[8] = {
@@ -136,9 +136,11 @@ int choose_block_n(int m, int n, int k, int num_sms, bool can_cut_tail, double* 
 }
 
 // CTAs per tile when K is cut over clusters (64-wide tiles), or 0 to leave tiles whole.  `whole` is the time of whole tiles by
-// the model above; a clustered launch takes about 6.0 us + 0.215 per k-block of a slice (M=209 N=480 K=12928, four slices: 11.7
-// against 24.5; M=128 N=2048 K=7168 9.8 against 15.8; M=600 N=512 K=4096, two slices: 8.6 against 10.0).  Clusters of four stop
-// fitting the GPU at once between 132 and 136 CTAs (M=128 K=7168: N=2112 10.1, N=2176 17.6), clusters of two at 148.
+// the model above, and 6.0 us + 0.215 per k-block of a slice that of a clustered launch: both were fitted before the issue loop and the
+// overlapped launches of today, which took 0.7 us off a clustered launch and 2 to 3 off whole tiles.  Today, clustered against the best whole tiles: M=209
+// N=480 K=12928, four slices, 11.0 us against 21.8; M=128 N=2048 K=7168 9.0 against 12.9; M=256 N=1024 K=8192, two slices, 9.6
+// against 14.2; M=600 N=512 K=4096 7.9 against 8.5; left whole: M=128 N=1024 K=2048 5.6.  Clusters of four stop fitting the GPU at once
+// between 132 and 136 CTAs, clusters of two at 148.
 int choose_cluster_slices(int m, int n, int k, int num_sms, double whole) {
     const long tiles = static_cast<long>((m + 127) / 128) * ((n + 63) / 64);
     const int kb = k / 128;

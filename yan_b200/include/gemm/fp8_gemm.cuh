@@ -1189,8 +1189,16 @@ struct GemmLauncher {
         }
         // Started while the kernel in front ends, the CTAs go to the SMs in the order in which these become free, and neighbours in
         // the tile order, which share operands, no longer sit next to each other: a launch of many k-blocks loses more to that
-        // than the two microseconds it saves (M=8192 N=28672 K=8192 behind its quantizer 1912 -> 1997 us; M=4096 N=7168 K=18432
-        // 544 -> 553; M=1111 N=5136 K=3072, 48 k-blocks per CTA, 26.6 -> 25.6; M=256 N=1024 K=1024 with quantizer 8.2 -> 5.8).
+        // than the microsecond it saves.  Without / with overlap, us in a graph, back to back | behind a quantizer | behind a 2 us
+        // kernel of another library:
+        //     8 k-blocks per CTA  M=512 N=2048 K=1024 fp32         5.6 /   5.0                   7.6 /   7.5
+        //    48                   M=1111 N=5136 K=3072            22.2 /  21.6                  24.2 /  24.4
+        //    80                   M=2048 N=4096 K=5120            39.4 /  38.8   44.2 /  43.7   40.8 /  40.9
+        //   112                   M=2048 N=4096 K=7168            53.3 /  52.8   61.9 /  60.1   55.0 /  55.0
+        //   152                   M=4096 N=4096 K=4864            73.6 /  72.9   83.3 /  92.1   75.6 /  83.4
+        //   200                   M=4096 N=4096 K=6400            95.2 /  98.6  106.6 / 116.8   96.7 / 102.5
+        //   301                   M=4096 N=8192 K=5504           153.1 / 153.4  164.7 / 168.8  155.2 / 157.4
+        // (M=256 N=1024 K=1024 with its quantizer 6.4 / 5.3.)
         const uint64_t all_tiles = ceil_div(a_rows, static_cast<uint64_t>(kBlockM)) * ceil_div(a.n, BLOCK_N);
         const bool overlap = ceil_div(all_tiles, static_cast<uint64_t>(grid)) * (a.k / kBlockK) <= kOverlapMaxKBlocks;
         if constexpr (kGemmType == GemmType::Normal && sizeof(out_t) == 2 && L::kStoreBytes != 0) {

@@ -15,7 +15,7 @@
 //     loads in flight share a few scoreboards, and waiting for the oldest waits for the newest.)
 //   * warps 4-11: two promotion warpgroups that share a tile's 16-column chunks alternately; thread = weight row;
 //   * output straight from registers: 32 lanes hold 32 consecutive columns of a row, 64 bytes per store instruction.
-// What bounds it: HBM (M_max=128, 16 groups of 24 rows, N=7168 K=2048: 57.3 -> 47.1 us, 5.1 TB/s of weights; 24 groups of 8
+// What bounds it: HBM (M_max=128, 16 groups of 24 rows, N=7168 K=2048: 57.3 -> 45.0 us, 5.3 TB/s of weights; 24 groups of 8
 // rows, N=2048 K=4096: 48.5 -> 38.7), a CTA alone streams at about 500 cycles per k-block of 16 KB.
 
 #include <cstdint>

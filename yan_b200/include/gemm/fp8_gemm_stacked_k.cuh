@@ -19,8 +19,8 @@
 // and read zeros).  A cluster of 2 or 4 CTAs shares the R weight rows when N / R CTAs alone would leave SMs idle; its
 // CTAs send their M_PAD x R sums to the first one through distributed shared memory.
 //
-//   warps 0-3: promotion (thread = TMEM lane = (k-part, weight row)); warp 4: producer, lane = (slot, k-part);
-//   warp 5: tensor memory and MMA.
+//   warps 0-3: promotion (thread = TMEM lane = (k-part, weight row)); warp 4: producer; warp 5: tensor memory and MMA.  One elected
+//   lane issues all loads, another one all products.
 // kSlots step slots of shared memory and kTmemSlots of tensor memory rotate: the loads of step s + kSlots go out as soon as
 // the MMAs of step s are complete, the MMAs of step s + kTmemSlots wait until the promotion warps have read the accumulator
 // of step s.
@@ -48,9 +48,11 @@ enum StackedOrder : uint32_t {
     kConstantWeights = 1,  // any kernel, none of which writes weights (the caller's promise): they are loaded before the wait
 };
 
-// Steps whose weights every CTA asks L2 for before it waits (0 / 3 / 8 / all, us in a graph: M=1 N=4096 K=7168 7.4 / 7.0 / 7.1 /
-// 7.3, M=16 N=4096 K=4096 5.5 / 5.2 / 5.0 / 5.1, M=4 N=28672 K=8192 40.3 / 39.7 / 42.8 / 45.0: a launch of several waves of CTAs
-// only fetches twice what its loads fetch anyway).
+// Steps whose weights every CTA asks L2 for before it waits (0 / 4, us in a graph over weights from HBM: M=1 N=4096 K=7168 7.6 / 7.0,
+// M=16 N=7168 K=2048 5.0 / 4.6, M=64 N=7168 K=2048 6.1 / 5.8, behind a quantizer 6.2 / 5.8 and 7.3 / 6.9; several waves of CTAs:
+// M=3 N=16384 K=2048 11.0 / 10.2, M=4 N=28672 K=8192 40.1 / 40.1; fp8_linear M=16 N=2048 K=7168 7.2 / 6.8).  More only fetch twice
+// what the loads of a launch of several waves fetch anyway (8 / all: M=4 N=28672 K=8192 42.8 / 45.0).  Leaving it to the CTAs that
+// start first gives nothing (fp8_linear M=4 N=28672 K=2048 16.3 against 15.9).
 constexpr uint32_t kPrefetchSteps = 4;
 
 // Adds kCols floats of shared memory; false where they come from a thread that gave up.
@@ -79,7 +81,7 @@ __global__ void __launch_bounds__(kStackedThreads, kTmemSlots * kStack * M_PAD <
     constexpr uint32_t kTmemCols = stacked_k_tmem_cols(M_PAD, kStack, kSlots);
     static_assert(M_PAD == 16 || M_PAD == 32 || M_PAD == 64, "activation rows are padded to 16, 32 or 64");
     static_assert(kStack == 1 || kStack == 2 || kStack == 4, "whole lane quarters of the 128-row operand");
-    static_assert(kSlots <= 8 && kTmemSlots <= 8 && kSlots * kStack <= 32, "one producer lane per (slot, k-part)");
+    static_assert(kSlots <= 8 && kTmemSlots <= 8, "the issue loops are unrolled over both rings");
     static_assert(kTmemCols == kTmemSlots * kMmaN && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "a power of two of at most 512 columns");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
