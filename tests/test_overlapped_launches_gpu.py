@@ -168,3 +168,31 @@ def test_fp8_linear_of_the_pair_kernel_sees_weights_written_directly_in_front(cu
     for _ in range(3):
         assert all(torch.equal(g, w) for g, w in zip(run(False), want))
     assert yan_b200.read_device_status() == 0
+
+
+# e4m3 output on tiles of one wave, on both sides of the line up to which the launch overlaps the kernel in front
+@pytest.mark.parametrize("k", [12288, 12416])
+def test_e4m3_output_of_long_k_behind_its_quantizer(cuda_lib, k):
+    import yan_b200
+    m, n = 200, 384
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    xs = [torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(4)]
+    rhs = yan_b200.per_block_cast_to_fp8((torch.randn(n, k, generator=gen, device="cuda") * 0.02).to(torch.bfloat16))
+    want = []
+    for x in xs:
+        out = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        lhs = yan_b200.per_token_cast_to_fp8(x)
+        torch.cuda.synchronize()
+        yan_b200.gemm_fp8_fp8_bf16_nt(lhs, rhs, out, block_n=256)
+        torch.cuda.synchronize()
+        want.append(yan_b200.per_token_cast_to_fp8(out))
+        torch.cuda.synchronize()
+    lhs = yan_b200.per_token_cast_to_fp8(xs[0])
+    got = []
+    for i in range(12):
+        yan_b200.per_token_cast_to_fp8(xs[i % 4], out=lhs)
+        got.append(yan_b200.gemm_fp8_fp8_e4m3_nt(lhs, rhs))
+    torch.cuda.synchronize()
+    for i, (q, s) in enumerate(got):
+        assert torch.equal(q.view(torch.uint8), want[i % 4][0].view(torch.uint8)) and torch.equal(s, want[i % 4][1])
+    assert yan_b200.read_device_status() == 0
