@@ -123,6 +123,9 @@ void yan_b200_m_grouped_gemm_fp8_fp8_bf16_nt_masked(const void* lhs, const void*
  * Activation quantizer: bf16 [M, x_ld] -> e4m3 [M, K] + fp32 scales (k-block-major, leading dimension
  * scales_ld >= M), 1 x 128 groups, scale = amax/448.  The reference names this component but holds no
  * code for it; the output feeds `lhs` / `lhs_scales` of the GEMM (yan/jit_kernels/gemm.py:23-25).
+ * It waits for the kernel in front before it touches anything.  Up to 64 rows (and with the promise of constant weights off, below) a
+ * kernel launched behind it with programmatic stream serialization may start before that wait: what such a kernel reads in front
+ * of its own griddepcontrol.wait must not be written by the kernel in front of the quantizer either.
  */
 void yan_b200_per_token_cast_to_fp8(const void* x, void* out, void* out_scales, int m, int k, int x_ld, int scales_ld,
                                     void* stream, int* return_code);
@@ -135,8 +138,7 @@ void yan_b200_per_block_cast_to_fp8(const void* w, void* out, void* out_scales, 
 /*
  * Quantize-then-GEMM in one call: out = bf16( quant_1x128(a) . rhs^T ).  `workspace` is caller-owned
  * scratch of at least yan_b200_fp8_linear_workspace_bytes(m, k) bytes (256-byte aligned) that holds the
- * quantized activations and their scales between the two kernels.  This is the path the north-star
- * names end to end (bf16 A in, bf16 D out); the reference has no such function.
+ * quantized activations and their scales between the two kernels: bf16 A in, bf16 D out.  The reference has no such function.
  */
 size_t yan_b200_fp8_linear_workspace_bytes(int m, int k);
 void yan_b200_fp8_linear_bf16(const void* a, const void* rhs, const void* rhs_scales, void* out, void* workspace,
